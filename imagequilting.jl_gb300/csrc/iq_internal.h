@@ -621,8 +621,10 @@ __device__ __forceinline__ uint32_t iq_quad_ssd(const uint8_t* base, const uint4
                                                 const Bound& bound) {
   const int lane = threadIdx.x & 31;
   uint32_t acc = 0;
+  // Batches of 8 x 32 quads while all lanes have one, so that the trip count and the exit (the
+  // bound as lane 0 read it) are the warp's: the loop holds full-warp shuffles.
   int i = lane;
-  for (; i + 7 * 32 < nq; i += 8 * 32) {
+  for (; i - lane + 8 * 32 <= nq; i += 8 * 32) {
     uint32_t v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) v[u] = iq_ld4(base + (int32_t)q[i + 32 * u].x);
@@ -635,7 +637,7 @@ __device__ __forceinline__ uint32_t iq_quad_ssd(const uint8_t* base, const uint4
     uint32_t part = acc;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if ((float)part > bound()) return 0xFFFFFFFFu;
+    if ((float)part > __shfl_sync(0xffffffffu, bound(), 0)) return 0xFFFFFFFFu;
   }
   for (; i < nq; i += 32) {
     const uint4 e = q[i];
@@ -709,8 +711,9 @@ __device__ __forceinline__ uint32_t iq_plane_ssd(const LpImg& im, int64_t x0, in
   const uint32_t base = (uint32_t)z0 * zs + ((uint32_t)x0 >> 5) * 16u;
   const uint32_t y0u = (uint32_t)y0;
   int acc = 0;
+  // batches of 4 x 32 rows while all lanes have one (see iq_quad_ssd)
   int r = lane;
-  for (; r + 3 * 32 < R; r += 4 * 32) {
+  for (; r - lane + 4 * 32 <= R; r += 4 * 32) {
     unsigned long long wa[4], wb[4];
     uint4 t[4];
 #pragma unroll
@@ -730,7 +733,7 @@ __device__ __forceinline__ uint32_t iq_plane_ssd(const LpImg& im, int64_t x0, in
     int part = acc;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if ((float)part > bound()) return 0xFFFFFFFFu;
+    if ((float)part > __shfl_sync(0xffffffffu, bound(), 0)) return 0xFFFFFFFFu;
   }
   for (; r < R; r += 32) {
     const uint4 t = rows[r];
