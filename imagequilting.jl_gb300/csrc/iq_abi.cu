@@ -9,7 +9,7 @@
 #include <cmath>
 #include <vector>
 
-#include "iq_internal.h"
+#include "iq_tz_plan.h"
 
 static thread_local char g_err[1024] = "";
 
@@ -456,44 +456,70 @@ extern "C" int iq_fastdistance(iq_ctx* ctx, const int64_t* tilesize, int32_t ntm
     if ((rc = iq_value_stats(ctx, d_tmpl, T * ntmpl, tstats))) return rc;
     TcBox box0;
     for (int d = 0; d < 3; ++d) { box0.lo[d] = (int32_t)blo[d]; box0.hi[d] = (int32_t)bhi[d]; }
-    TcStages stg;
-    iq_tc_stages(t, &box0, 1, stg);
-    const size_t ns = stg.word.size(), n16 = stg.w16a.size();
-    stw.resize(2 * ns + 3 * n16);
-    for (size_t e = 0; e < ns; ++e) { stw[e] = stg.word[e]; stw[ns + e] = stg.prefix[e]; }
-    for (size_t e = 0; e < n16; ++e) {
-      stw[2 * ns + e] = stg.w16a[e];
-      stw[2 * ns + n16 + e] = stg.w16b[e];
-      stw[2 * ns + 2 * n16 + e] = stg.pre16[e];
-    }
-    for (int32_t c0 = 0; c0 < ntmpl; c0 += IQ_TC_MAXN) {
-      const int nb = std::min<int32_t>(IQ_TC_MAXN, ntmpl - c0);
-      const int Np = (nb + 15) / 16 * 16;
-      for (int i = 0; i < Np; ++i)
-        cols.push_back(i < nb ? TcCol{(int64_t)(c0 + i) * T, d_out + (size_t)(c0 + i) * P, d_b2 + c0 + i, nullptr, 0, 0}
-                              : TcCol{-1, nullptr, nullptr, nullptr, 0, 0});
-    }
-    uint32_t* d_st = (uint32_t*)iq_scratch(ctx, S_TCSTAGE, sizeof(uint32_t) * std::max<size_t>(stw.size(), 1));
-    TcCol* d_cols = (TcCol*)iq_scratch(ctx, S_TCCOLS, sizeof(TcCol) * cols.size());
-    void* d_B = iq_scratch(ctx, S_TCB, (size_t)std::max<int64_t>(std::max(stg.nsteps, stg.nsteps16), 1) *
-                                          64 * IQ_TC_MAXN);
-    if (!d_st || !d_cols || !d_B) return IQ_ERR_ALLOC;
-    IQ_CUDA_OK(cudaMemcpyAsync(d_st, stw.data(), sizeof(uint32_t) * stw.size(), cudaMemcpyHostToDevice, ctx->stream));
-    IQ_CUDA_OK(cudaMemcpyAsync(d_cols, cols.data(), sizeof(TcCol) * cols.size(), cudaMemcpyHostToDevice, ctx->stream));
-    size_t col0 = 0;
-    for (int32_t c0 = 0; c0 < ntmpl; c0 += IQ_TC_MAXN) {
-      const int nb = std::min<int32_t>(IQ_TC_MAXN, ntmpl - c0);
-      TcCorrLaunch L;
-      L.img = ctx->d_ti; L.img_dims = ctx->ti; L.out_dims = od; L.tile = t; L.ii = ctx->d_ti2ii;
-      L.nbox = 1; L.box[0] = box0;
-      L.disabled = d_dis;
-      L.stage_word = d_st; L.stage_prefix = d_st + ns; L.nstage = (int)ns; L.nsteps = stg.nsteps;
-      L.stage16 = d_st + 2 * ns; L.nstage16 = (int)n16; L.nsteps16 = stg.nsteps16;
-      L.grid = d_tmpl; L.grid_dims = t; L.cols = d_cols + col0; L.N = (nb + 15) / 16 * 16;
-      L.B = d_B; L.img_stats = ctx->ti_stats; L.tmpl_stats = tstats;
-      L.flops = 2.0 * (double)P * (double)K * nb;
-      if ((rc = iq_launch_corr_tc(ctx, L))) return rc;
-      col0 += L.N;
+    // Values whose FP16 products and FP32 sums are exact: the Toeplitz form. Other data keep the
+    // summation of iq_corr_tc.cu, whose maps this entry point returns as they are (in iq_simulate
+    // the pick's exact re-rank makes the form immaterial).
+    if (ctx->corr_engine == 2 && ctx->ti_stats.fp16_range() && tstats.fp16_range() &&
+        iq_map_kappa(ctx->ti_stats, tstats, K, 1) == 0.0 && ctx->ti_stats.narrow && tstats.narrow &&
+        iq_tz_fits(ctx->ti, t, od)) {
+      TzPlan pl;
+      pl.img = ctx->ti; pl.tile = t; pl.boxes.push_back(box0);
+      // at most 16 groups per launch: their packed templates share one buffer
+      for (int32_t c0 = 0; c0 < ntmpl; c0 += 16 * IQ_TZ_COLS) {
+        std::vector<TcCol> cc;
+        for (int32_t i = c0; i < std::min<int32_t>(ntmpl, c0 + 16 * IQ_TZ_COLS); ++i)
+          cc.push_back(TcCol{(int64_t)i * T, d_out + (size_t)i * P, d_b2 + i, nullptr, 0, 0});
+        pl.add_launch(cc, 2.0 * (double)P * (double)K * (double)cc.size());
+      }
+      void* img = iq_scratch(ctx, S_TZ_IMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * 2);
+      float* a2 = (float*)iq_scratch(ctx, S_TZ_A2, sizeof(float) * P);
+      void* B = iq_scratch(ctx, S_TZ_B, (size_t)pl.max_bytes());
+      if (!img || !a2 || !B) return IQ_ERR_ALLOC;
+      if ((rc = pl.upload(ctx, S_TZ_PLAN, ctx->stream))) return rc;
+      if ((rc = iq_tz_image(ctx, ctx->d_ti, ctx->ti, ctx->ti_stats, false, img))) return rc;
+      if ((rc = iq_tz_a2_maps(ctx, ctx->d_ti2ii, ctx->ti, od, t, pl.d_boxes, 1, d_dis, a2))) return rc;
+      for (const TzPlan::Launch& l : pl.launches)
+        if ((rc = pl.launch(ctx, l, img, od, a2, d_tmpl, t, B, ctx->ti_stats, tstats))) return rc;
+    } else {
+      TcStages stg;
+      iq_tc_stages(t, &box0, 1, stg);
+      const size_t ns = stg.word.size(), n16 = stg.w16a.size();
+      stw.resize(2 * ns + 3 * n16);
+      for (size_t e = 0; e < ns; ++e) { stw[e] = stg.word[e]; stw[ns + e] = stg.prefix[e]; }
+      for (size_t e = 0; e < n16; ++e) {
+        stw[2 * ns + e] = stg.w16a[e];
+        stw[2 * ns + n16 + e] = stg.w16b[e];
+        stw[2 * ns + 2 * n16 + e] = stg.pre16[e];
+      }
+      for (int32_t c0 = 0; c0 < ntmpl; c0 += IQ_TC_MAXN) {
+        const int nb = std::min<int32_t>(IQ_TC_MAXN, ntmpl - c0);
+        const int Np = (nb + 15) / 16 * 16;
+        for (int i = 0; i < Np; ++i)
+          cols.push_back(i < nb ? TcCol{(int64_t)(c0 + i) * T, d_out + (size_t)(c0 + i) * P, d_b2 + c0 + i, nullptr, 0, 0}
+                                : TcCol{-1, nullptr, nullptr, nullptr, 0, 0});
+      }
+      uint32_t* d_st = (uint32_t*)iq_scratch(ctx, S_TCSTAGE, sizeof(uint32_t) * std::max<size_t>(stw.size(), 1));
+      TcCol* d_cols = (TcCol*)iq_scratch(ctx, S_TCCOLS, sizeof(TcCol) * cols.size());
+      void* d_B = iq_scratch(ctx, S_TCB, (size_t)std::max<int64_t>(std::max(stg.nsteps, stg.nsteps16), 1) *
+                                            64 * IQ_TC_MAXN);
+      if (!d_st || !d_cols || !d_B) return IQ_ERR_ALLOC;
+      IQ_CUDA_OK(cudaMemcpyAsync(d_st, stw.data(), sizeof(uint32_t) * stw.size(), cudaMemcpyHostToDevice, ctx->stream));
+      IQ_CUDA_OK(cudaMemcpyAsync(d_cols, cols.data(), sizeof(TcCol) * cols.size(), cudaMemcpyHostToDevice, ctx->stream));
+      size_t col0 = 0;
+      for (int32_t c0 = 0; c0 < ntmpl; c0 += IQ_TC_MAXN) {
+        const int nb = std::min<int32_t>(IQ_TC_MAXN, ntmpl - c0);
+        TcCorrLaunch L;
+        L.img = ctx->d_ti; L.img_dims = ctx->ti; L.out_dims = od; L.tile = t; L.ii = ctx->d_ti2ii;
+        L.nbox = 1; L.box[0] = box0;
+        L.disabled = d_dis;
+        L.stage_word = d_st; L.stage_prefix = d_st + ns; L.nstage = (int)ns; L.nsteps = stg.nsteps;
+        L.stage16 = d_st + 2 * ns; L.nstage16 = (int)n16; L.nsteps16 = stg.nsteps16;
+        L.grid = d_tmpl; L.grid_dims = t; L.cols = d_cols + col0; L.N = (nb + 15) / 16 * 16;
+        L.B = d_B; L.img_stats = ctx->ti_stats; L.tmpl_stats = tstats;
+        L.flops = 2.0 * (double)P * (double)K * nb;
+        if ((rc = iq_launch_corr_tc(ctx, L))) return rc;
+        col0 += L.N;
+      }
     }
   } else {
     CorrLaunch C;

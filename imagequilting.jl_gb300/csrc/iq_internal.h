@@ -128,6 +128,7 @@ enum IqSlot {
   S_PBH_OUT, S_PBH_POOL, S_PBH_SRC,
   S_LP_T, S_LP_NT, S_LP_TAU, S_LP_LIST, S_LP_CNT, S_LP_DL, S_LP_COLS, S_LP_TSRC, S_LP_TBOX,
   S_LP_RIND, S_LP_NCAND, S_LP_D, S_LP_BITS, S_LP_ITEMS, S_LP_X, S_LP_E, S_LP_GE, S_LP_FEAT, S_LP_BH1, S_LP_BGZ1, S_LP_BH2, S_LP_DENSE, S_LP_QUAD,
+  S_TZ_IMG, S_TZ_A2, S_TZ_PLAN, S_TZ_B, S_TZ_SIMG, S_TZ_SA2, S_PREDRAW,
   S_COUNT
 };
 
@@ -283,6 +284,58 @@ int iq_launch_corr_tc(iq_ctx* ctx, const TcCorrLaunch& L);
 // statistics of a device array of floats
 int iq_value_stats(iq_ctx* ctx, const float* d, int64_t n, IqValueStats& out);
 
+// ---- tensor-core correlation, Toeplitz templates (iq_corr_tz.cu) ----
+constexpr int IQ_TZ_COLS = 32;   // columns (templates) per group: N = 8 x columns <= 256
+constexpr int IQ_TZ_ROWS = 5;    // image rows staged together
+constexpr int IQ_TZ_STEPS = 5;   // K-steps (two 8-offset chunks each) staged together
+
+// One stage's step table: w[0] = row entries | K-steps << 8, w[1] = K-steps before it,
+// w[2..6] = image offset of each entry / 8, w[7] = chunks each entry spans plus one (4 bits each),
+// w[8..12] = per K-step its two chunks, (entry | chunk << 4) each 8 bits.
+struct TzStage {
+  uint32_t w[16];
+};
+// The K-steps of the union of some masks, as stages, and per chunk ky | kz << 10 | chunk << 20
+// (all ones: padding); touched[b]: K-steps that hold an offset of mask b.
+struct TzList {
+  std::vector<TzStage> stage;
+  std::vector<uint32_t> chunk;
+  std::vector<int64_t> touched;
+  int64_t nstep = 0;
+};
+// Columns [col0, col0 + ncol) computed together (ncol even; padding columns have src < 0): one
+// stage list, templates packed from byte boff (nstep * 32 * N bytes, twice when split).
+struct TzGroup {
+  int32_t col0, ncol, N, nstage, stage0, nstep, chunk0, pad_;
+  int64_t boff;
+};
+struct TzLaunch {
+  const void* img = nullptr;            // FP16 image made by iq_tz_image
+  Dim3 img_dims{1, 1, 1}, out_dims{1, 1, 1}, tile{1, 1, 1};
+  const TzGroup* groups = nullptr;      // device array
+  int ngroup = 0, Nmax = 0;
+  const TzStage* stages = nullptr;      // device arrays the groups index
+  const uint32_t* chunks = nullptr;
+  const TcBox* boxes = nullptr;         // device array the columns' box indexes
+  const float* a2 = nullptr;            // A2 maps (iq_tz_a2_maps), one per box
+  const float* grid = nullptr; Dim3 grid_dims{1, 1, 1};  // template source
+  const TcCol* cols = nullptr;
+  void* B = nullptr;                    // packed templates
+  int64_t max_units = 0;                // most 16-byte units (nstep * 2 * N) of a group
+  IqValueStats img_stats, tmpl_stats;
+  double flops = 0, mma_flops = 0;      // algorithmic; issued per 1024 positions (profiling)
+  int ncols = 0;
+};
+bool iq_tz_fits(Dim3 img, Dim3 tile, Dim3 out);
+void iq_tz_list(Dim3 img, Dim3 tile, const TcBox* boxes, int nbox, TzList& out);
+// error coefficient of a map of this form: nsteps K-steps hold offsets of its mask
+double iq_map_kappa_tz(const IqValueStats& A, const IqValueStats& B, int64_t K, int64_t nsteps);
+int64_t iq_tz_image_halves(Dim3 img);   // halves of one FP16 image (hi, or lo when split)
+int iq_tz_image(iq_ctx* ctx, const float* img, Dim3 d, const IqValueStats& st, bool split, void* dst);
+int iq_tz_a2_maps(iq_ctx* ctx, const double* ii, Dim3 img, Dim3 out, Dim3 tile, const TcBox* boxes,
+                  int nbox, const uint8_t* disabled, float* maps);
+int iq_launch_corr_tz(iq_ctx* ctx, const TzLaunch& L);
+
 // integral images and disabled windows
 int iq_build_integrals(iq_ctx* ctx, const float* d_img, Dim3 dims, double* d_sqii,
                        int32_t* d_nanii, const uint8_t* d_nan);
@@ -341,6 +394,8 @@ struct PickTask {
   const int32_t* x0_pool;                   // its band list
   const int32_t* pb_pool;                   // their band lists
   int nkeys;
+  const int64_t* pre;                       // draws made on the host, per realization (nullable:
+                                            // the pick makes them)
   int64_t tile;                             // Philox counter of the draw
   // direct re-evaluation of D0 and of each auxiliary map (kappa == 0, or img == nullptr:
   // the map's values are taken as exact)

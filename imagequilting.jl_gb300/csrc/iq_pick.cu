@@ -1412,6 +1412,13 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
   const int r = b % a.nreal;
   const PickTask& tk = a.tasks ? a.tasks[b / a.nreal] : a.t0;
   const int64_t P = a.P;
+  if (tk.pre) {  // every position is a candidate of one rank: drawn already
+    if (threadIdx.x == 0) {
+      a.rind[b] = tk.pre[r];
+      if (a.ncand) a.ncand[b] = P;
+    }
+    return;
+  }
   const float* D = tk.D0 + r * tk.D0_rs;
   const unsigned* mm = tk.mm0 + r * tk.mm0_rs;
   const int naux = tk.naux < NAUX ? tk.naux : NAUX;

@@ -17,7 +17,7 @@
 #include <unordered_map>
 #include <vector>
 
-#include "iq_internal.h"
+#include "iq_tz_plan.h"
 
 // ---------------------------------------------------------------------------------------
 // host helpers
@@ -463,6 +463,12 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
     cfg_kappa[c] = iq_map_kappa(ctx->ti_stats, sim_stats, cfgs[c].K, ovl_form);
     need_ref = need_ref || cfg_kappa[c] > 0.0;
   }
+  // Without data and without inactive windows a tile with no pasted neighbour has distance 0
+  // everywhere: every position is a candidate of rank 1, and its draw depends on the position
+  // count alone. Such draws are made here (below), and the tile's maps and pick are left out.
+  auto predrawn = [&](const Step& s) {
+    return cfgs[s.cfg].K == 0 && !s.hardtile && nsoft == 0 && ctx->ti_nan == 0;
+  };
   const double ovl_eabs = iq_map_eabs(ctx->ti_stats, tivol_all);
   // hard lists of data tiles
   std::vector<int64_t> hoff(g.ntot + 1, 0);
@@ -495,6 +501,12 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
                            T * (rpad + 1) * 4 + (int64_t)R * 6 * (slabmax + cutscr_per) + 4096;
   size_t freeb = 0, totalb = 0;
   cudaMemGetInfo(&freeb, &totalb);
+  // The Toeplitz form of the correlation (iq_corr_tz.cu) for data FP16 halves represent, unless
+  // its A2 maps (one per mask) would take more than an eighth of the free memory: then, and for
+  // data of wider range, the form of iq_corr_tc.cu.
+  const bool tz = ovl_form == 1 && T > 0 && iq_tz_fits(ctx->ti, tileD, distD) &&
+                  (double)(ncfg + 1) * (double)P * 4.0 <= (double)freeb / 8.0;
+  const bool tz_split = !(ctx->ti_stats.narrow && sim_stats.narrow);
   // hard-data distance maps depend on the data only: one map per data tile, all held at once
   int64_t nhs = 0;
   for (const Step& s : steps) nhs += s.hardtile ? 1 : 0;
@@ -613,6 +625,9 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   struct TcRun {
     int64_t chunk; size_t col0; int N; std::vector<int> cfgset; TcStageRef st; double flops;
   };
+  TzPlan tzp;                 // launch of (chunk c, group g): c * ngrp + g
+  tzp.img = ctx->ti; tzp.tile = tileD; tzp.split = tz_split;
+  for (int c = 0; c <= ncfg; ++c) tzp.boxes.push_back(cfg_box(c));
   std::vector<TcRun> tcruns;
   std::vector<TcCol> tccols;
   std::vector<int64_t> tcbeg(nchunk * ngrp + 1, 0);  // launches of (chunk c, group g): c * ngrp + g
@@ -629,9 +644,27 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
     chunk_tc[c] = ok;
     if (ok) {
       std::vector<std::pair<int, int64_t>> order;  // (cfg, step index in chunk) sorted by cfg
-      for (int64_t k = cbeg[c]; k < cbeg[c + 1]; ++k) order.push_back({steps[k].cfg, k - cbeg[c]});
+      for (int64_t k = cbeg[c]; k < cbeg[c + 1]; ++k)
+        if (!predrawn(steps[k])) order.push_back({steps[k].cfg, k - cbeg[c]});
       std::stable_sort(order.begin(), order.end(),
                        [](const std::pair<int, int64_t>& x, const std::pair<int, int64_t>& y) { return x.first < y.first; });
+      if (tz) {
+        std::vector<TcCol> cc;
+        double fl = 0;
+        for (const auto& o : order)
+          for (int r = gb[grp]; r < gb[grp + 1]; ++r) {
+            cc.push_back(TcCol{r * padvol + steps[cbeg[c] + o.second].startlin,
+                               d_D + ((size_t)o.second * R + r) * P, d_b2 + (size_t)o.second * rpad + r,
+                               d_mm + (size_t)o.second * R * 2 + 2 * r, o.first, 0});
+            fl += 2.0 * (double)P * (double)cfgs[o.first].K;
+          }
+        tzp.add_launch(cc, fl);
+        continue;
+      }
+      if (order.empty()) {
+        tcbeg[cg + 1] = (int64_t)tcruns.size();
+        continue;
+      }
       const int64_t ncols = (int64_t)order.size() * Rg;
       const int64_t nl = (ncols + IQ_TC_MAXN - 1) / IQ_TC_MAXN;
       const int64_t per = std::min<int64_t>(IQ_TC_MAXN, ((ncols + nl - 1) / nl + 15) / 16 * 16);
@@ -667,6 +700,25 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
       }
     }
     tcbeg[cg + 1] = (int64_t)tcruns.size();
+  }
+  // Toeplitz form: the FP16 image, the A2 maps of every mask and the plan, once per call
+  void *d_tzimg = nullptr, *d_tzB = nullptr;
+  float* d_tza2 = nullptr;
+  size_t tzb_bytes = 0;
+  if (tz) {
+    for (int c = 0; c < ncfg; ++c)
+      if (cfg_kappa[c] > 0.0) {
+        tzp.touched.resize(tzp.boxes.size(), 0);
+        cfg_kappa[c] = iq_map_kappa_tz(ctx->ti_stats, sim_stats, cfgs[c].K, tzp.touched[c]);
+      }
+    tzb_bytes = (size_t)tzp.max_bytes();
+    d_tzimg = iq_scratch(ctx, S_TZ_IMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * (tz_split ? 4 : 2));
+    d_tza2 = (float*)iq_scratch(ctx, S_TZ_A2, sizeof(float) * P * (ncfg + 1));
+    d_tzB = iq_scratch(ctx, S_TZ_B, tzb_bytes * ngrp);
+    if (!d_tzimg || !d_tza2 || !d_tzB) return IQ_ERR_ALLOC;
+    RET_IF(tzp.upload(ctx, S_TZ_PLAN, st));
+    RET_IF(iq_tz_image(ctx, ctx->d_ti, ctx->ti, ctx->ti_stats, tz_split, d_tzimg));
+    RET_IF(iq_tz_a2_maps(ctx, ctx->d_ti2ii, ctx->ti, distD, tileD, tzp.d_boxes, ncfg, d_dis, d_tza2));
   }
   const TcStageRef soft_st = (tc && nsoft > 0 && T > 0) ? stages_for(std::vector<int>{ncfg})
                                                          : TcStageRef{0, 0, 0, 0, 0, 0};
@@ -781,15 +833,57 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
       IQ_CUDA_OK(cudaMemcpyAsync(d_starts, starts.data(), sizeof(int64_t) * starts.size(),
                                  cudaMemcpyHostToDevice, st));
       IqValueStats aux_stats, auxti_stats;
+      TzPlan sp;
+      bool stz = false;
       RET_IF(iq_value_stats(ctx, d_aux[s], psz.vol(), aux_stats));
       RET_IF(iq_value_stats(ctx, d_auxti[s], tivol, auxti_stats));
       {
         const int form = !(tc && T > 0) ? 0 : (ctx->corr_engine == 2 && auxti_stats.fp16_range() &&
                                                 aux_stats.fp16_range()) ? 1 : 2;
+        stz = form == 1 && iq_tz_fits(ctx->ti, tileD, distD);
+        if (stz) {
+          sp.img = ctx->ti; sp.tile = tileD; sp.boxes.push_back(TcBox{});
+          sp.split = !(auxti_stats.narrow && aux_stats.narrow);
+          // at most 16 groups per launch: their packed templates share one buffer
+          const int64_t most = 16 * (sp.split ? IQ_TZ_COLS / 2 : IQ_TZ_COLS);
+          for (int64_t b0 = 0; b0 < (int64_t)tl.size(); b0 += most) {
+            std::vector<TcCol> cc;
+            for (int64_t i = b0; i < std::min<int64_t>(b0 + most, (int64_t)tl.size()); ++i) {
+              const int64_t slot = (int64_t)s * nslot + slot_of[tl[i]];
+              cc.push_back(TcCol{starts[i], d_soft + slot * P, d_softb2 + slot, d_softmm + 2 * slot, 0, 0});
+            }
+            sp.add_launch(cc, 2.0 * (double)P * (double)T * (double)cc.size());
+          }
+          soft_kappa[s] = iq_map_kappa_tz(auxti_stats, aux_stats, T, sp.touched[0]);
+        } else
         soft_kappa[s] = iq_map_kappa(auxti_stats, aux_stats, T, form);
         soft_eabs[s] = iq_map_eabs(auxti_stats, tivol);
       }
-      if (tc && T > 0) {
+      if (stz) {
+        // per-tile soft distance maps, Toeplitz form
+        void* img = iq_scratch(ctx, S_TZ_SIMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * (sp.split ? 4 : 2));
+        float* a2 = (float*)iq_scratch(ctx, S_TZ_SA2, sizeof(float) * P);
+        void* B = iq_scratch(ctx, S_TZ_B, std::max((size_t)sp.max_bytes(), tzb_bytes * ngrp));
+        if (!img || !a2 || !B) return IQ_ERR_ALLOC;
+        d_tzB = B;  // the slot may have moved
+        RET_IF(sp.upload(ctx, S_TCSOFT, st));
+        RET_IF(iq_tz_image(ctx, d_auxti[s], ctx->ti, auxti_stats, sp.split, img));
+        RET_IF(iq_tz_a2_maps(ctx, d_auxii[s], ctx->ti, distD, tileD, sp.d_boxes, 1, d_dis, a2));
+        // B2 of every template, and its map's [min, max] reset
+        GatherLaunch G;
+        G.grid = d_aux[s]; G.grid_dims = psz; G.grid_stride = 0; G.starts = d_starts;
+        const int64_t slot0 = (int64_t)s * nslot;
+        for (size_t b0 = 0; b0 < tl.size(); b0 += IQ_TC_MAXN) {
+          const int nb = (int)std::min<size_t>(IQ_TC_MAXN, tl.size() - b0);
+          G.starts = d_starts + b0;
+          G.ntmpl = nb; G.rpad = nb;
+          G.t0 = GatherTask{d_kl + (size_t)ncfg * T, (int)T, 0, nullptr, nullptr,
+                            d_softb2 + slot0 + b0, d_softmm + 2 * (slot0 + b0)};
+          RET_IF(iq_launch_gather(ctx, G));
+        }
+        for (const TzPlan::Launch& l : sp.launches)
+          RET_IF(sp.launch(ctx, l, img, distD, a2, d_aux[s], psz, B, auxti_stats, aux_stats));
+      } else if (tc && T > 0) {
         // per-tile soft distance maps on the tensor cores, up to 256 tiles per launch
         std::vector<TcCol> cols;
         std::vector<std::pair<size_t, int>> launches;  // (first column, N)
@@ -912,6 +1006,52 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
     if (!d_pbh || !d_pbhpool) return IQ_ERR_ALLOC;
     hard_x.resize(nhs);
   }
+  // ---- draws of the tiles whose distance is 0 everywhere (predrawn above) ----
+  // All P candidates have rank 1, so one weight w and one sum per chunk of IQ_DRAW_CHUNK serve
+  // every draw: the arithmetic and its order are the pick kernel's (Float64, round to nearest).
+  std::vector<int64_t> pre_of(steps.size(), -1), pre;
+  for (size_t k = 0; k < steps.size(); ++k)
+    if (predrawn(steps[k])) { pre_of[k] = (int64_t)(pre.size() / R); pre.resize(pre.size() + R); }
+  const int64_t* d_pre = nullptr;
+  if (!pre.empty()) {
+    const int64_t nch = (P + IQ_DRAW_CHUNK - 1) / IQ_DRAW_CHUNK;
+    double w = 1.0;
+    if (P > 1) {
+      const double dn = (double)P, inv_n = 1.0 / dn, x0 = (1.0 - inv_n) / inv_n;
+      const double Pi = dn / (double)((unsigned long long)P * (unsigned long long)P);
+      const double X = (1.0 - Pi) / Pi;
+      const double prod = 1.0 * (X / x0);
+      const double x = x0 * prod;
+      w = 1.0 / (1.0 + x);
+    }
+    std::vector<double> cum(nch);
+    double full = 0.0, last = 0.0, run = 0.0;
+    for (int64_t i = 0; i < IQ_DRAW_CHUNK; ++i) full = full + w;
+    for (int64_t i = (nch - 1) * IQ_DRAW_CHUNK; i < P; ++i) last = last + w;
+    for (int64_t c = 0; c < nch; ++c) { run = run + (c < nch - 1 ? full : last); cum[c] = run; }
+    for (size_t k = 0; k < steps.size(); ++k) {
+      if (pre_of[k] < 0) continue;
+      for (int r = 0; r < R; ++r) {
+        const double t = iq_draw_uniform(p->seed, steps[k].tile, p->real0 + r) * run;
+        // the first chunk whose running total reaches t (the totals never decrease), the last one
+        // otherwise
+        const int64_t c = std::min<int64_t>(std::lower_bound(cum.begin(), cum.end(), t) - cum.begin(), nch - 1);
+        const double base = c == 0 ? 0.0 : cum[c - 1];
+        const int64_t lo = c * IQ_DRAW_CHUNK, hi2 = std::min<int64_t>(P, lo + IQ_DRAW_CHUNK);
+        double part = 0.0;
+        int64_t pick = hi2 - 1;
+        for (int64_t i = lo; i < hi2; ++i) {
+          part = part + w;
+          if (base + part >= t) { pick = i; break; }
+        }
+        pre[pre_of[k] * R + r] = P > 1 ? pick : 0;
+      }
+    }
+    int64_t* dp = (int64_t*)iq_scratch(ctx, S_PREDRAW, sizeof(int64_t) * pre.size());
+    if (!dp) return IQ_ERR_ALLOC;
+    IQ_CUDA_OK(cudaMemcpyAsync(dp, pre.data(), sizeof(int64_t) * pre.size(), cudaMemcpyHostToDevice, st));
+    d_pre = dp;
+  }
   // ---- task descriptors of every step, uploaded once ----
   // Gather and pick tasks point at per-realization slots: each group has its own copy, whose
   // pointers start at the group's first realization. Cut and paste tasks are shared.
@@ -956,6 +1096,7 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
         PickTask& q = pt[grp * nsteps + k];
         memset(&q, 0, sizeof(q));
         q.tile = s.tile;
+        if (predrawn(s)) q.pre = d_pre + pre_of[k] * R + r0;
         // direct re-evaluation of the overlap map of realization r: the TI against the group's
         // simulation grid at the tile, over the mask's offsets
         ExactSrc xo{};
@@ -1143,7 +1284,10 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
         G.rpad = ngrp == 1 ? rpad : Rg;
         G.ntask = m; G.tasks = d_gt + grp * nsteps + k0;
         RET_IF(iq_launch_gather(ctx, G));
-        if (chunk_tc[c]) {
+        if (tz) {
+          RET_IF(tzp.launch(ctx, tzp.launches[c * ngrp + grp], d_tzimg, distD, d_tza2, d_sim, padD,
+                            (char*)d_tzB + grp * tzb_bytes, ctx->ti_stats, sim_stats));
+        } else if (chunk_tc[c]) {
           for (int64_t l = tcbeg[c * ngrp + grp]; l < tcbeg[c * ngrp + grp + 1]; ++l) {
             const TcRun& u = tcruns[l];
             RET_IF(tc_launch(u.cfgset, u.st, ctx->d_ti, ctx->d_ti2ii, d_sim, padD, d_tccols + u.col0,
