@@ -11,8 +11,8 @@ ROOT = os.path.dirname(HERE)
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libiqgpu.so")
 SOURCES = ["iq_abi.cu", "iq_sim.cu", "iq_distance.cu", "iq_pick.cu", "iq_graphcut.cu",
-           "iq_paste.cu", "iq_noalloc.cu", "iq_corr_tc.cu", "iq_corr_tz.cu", "iq_proposal.cu", "iq_proposal_pick.cu",
-           "iq_proposal_host.cu"]
+           "iq_paste.cu", "iq_noalloc.cu", "iq_corr_tc.cu", "iq_corr_tz.cu", "iq_proposal.cu",
+           "iq_proposal_net.cu", "iq_proposal_pick.cu", "iq_proposal_host.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -49,7 +49,7 @@ def build(verbose=False, force=False, extra=()):
         if force or _stale(o, [s] + headers):
             jobs.append([cc] + _flags(extra) + ["-c", s, "-o", o])
     if jobs:
-        with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
+        with concurrent.futures.ThreadPoolExecutor(max_workers=min(16, len(jobs))) as ex:
             res = list(ex.map(lambda c: subprocess.run(c, capture_output=True, text=True), jobs))
         for cmd, r in zip(jobs, res):
             if verbose or r.returncode:

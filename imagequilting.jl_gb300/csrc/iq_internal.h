@@ -128,7 +128,7 @@ enum IqSlot {
   S_PBH_OUT, S_PBH_POOL, S_PBH_SRC,
   S_LP_T, S_LP_NT, S_LP_TAU, S_LP_LIST, S_LP_CNT, S_LP_DL, S_LP_COLS, S_LP_TSRC, S_LP_TBOX,
   S_LP_RIND, S_LP_NCAND, S_LP_D, S_LP_BITS, S_LP_ITEMS, S_LP_X, S_LP_E, S_LP_GE, S_LP_FEAT, S_LP_BH1, S_LP_BGZ1, S_LP_BH2, S_LP_DENSE, S_LP_QUAD,
-  S_TZ_IMG, S_TZ_A2, S_TZ_PLAN, S_TZ_B, S_TZ_SIMG, S_TZ_SA2, S_PREDRAW,
+  S_TZ_IMG, S_TZ_A2, S_TZ_PLAN, S_TZ_B, S_TZ_SIMG, S_TZ_SA2, S_PREDRAW, S_LP_W,
   S_COUNT
 };
 
@@ -551,9 +551,20 @@ struct LpGeo {
 };
 LpGeo iq_lp_geo(Dim3 tile);
 
+// The training image as the encoder's windows read it: Float64 integral images of the values and
+// squares, and for integer data (iq_lp_int_cells) the same modulo 2^32 (else nullptr).
+struct LpWindows {
+  const double *ii1, *ii2;
+  const int *iq1, *iq2;
+  Dim3 img, dist;
+};
+// Whether cell sums of such values over a tile are exact in 32-bit integers and FP32.
+bool iq_lp_int_cells(const IqValueStats& s, Dim3 tile);
+int iq_lp_int_integral(iq_ctx* ctx, const double* ii, int64_t n, int* out);
+
 // One training step's data (device pointers): nA anchors with features feats[feat row], their
 // positives and nneg negatives per anchor as windows of the image (integral images ii1, ii2);
-// items: anchors, then positives, then negatives (iq_proposal.cu TrainItem layout, 16 bytes).
+// items: anchors, then positives, then negatives (iq_proposal_net.cu TrainItem layout, 16 bytes).
 struct LpTrainBatch {
   const float* w;          // FP32 parameters
   const void* items;
@@ -561,9 +572,7 @@ struct LpTrainBatch {
   float temp;
   const float* feats;      // [rows][3 * ng]
   const int32_t* boxes;    // [rows][6]
-  const double* ii1;
-  const double* ii2;
-  Dim3 img, dist;
+  LpWindows win;
   float* X;                // scratch [items][3 * ng]
   float* E;                // scratch [items][64]
   float* gE;               // scratch [items][64]
@@ -574,10 +583,9 @@ int iq_lp_train_batch(iq_ctx* ctx, const LpGeo& g, const LpTrainBatch& B, double
 int iq_lp_adam(iq_ctx* ctx, float* p, const float* g, float* m, float* v, int n, float lr, int step);
 struct __nv_bfloat16;
 // Window embeddings of every distance-map position (pos == nullptr) or of pos[0, npos).
-int iq_lp_encode_windows(iq_ctx* ctx, const LpGeo& g, const float* w, const double* ii1,
-                         const double* ii2, Dim3 img, Dim3 dist, const int* lo, const int* hi,
-                         __nv_bfloat16* out, float* norm, const int64_t* pos = nullptr,
-                         int64_t npos = 0);
+int iq_lp_encode_windows(iq_ctx* ctx, const LpGeo& g, const float* w, const LpWindows& W,
+                         const int* lo, const int* hi, __nv_bfloat16* out, float* norm,
+                         const int64_t* pos = nullptr, int64_t npos = 0);
 // One column of the proposal's pick: tile `tile` of global realization `real`, with the mask's
 // offsets and the simulation grid at the tile.
 // Quads of a mask: four consecutive x offsets of one (y, z) row starting at a multiple of 4,
@@ -879,7 +887,7 @@ void iq_lp_begin_call(iq_ctx* ctx);
 void iq_lp_count_full(iq_ctx* ctx, int64_t ncol);
 int iq_lp_capture_reserve(iq_ctx* ctx, int64_t n);
 int iq_lp_encode_templates(iq_ctx* ctx, const LpGeo& g, const float* w, const float* grid,
-                           Dim3 gdims, const int64_t* tsrc, const int* tbox, int64_t n,
+                           Dim3 gdims, const int64_t* tsrc, const int* tbox, int64_t n, bool ints,
                            __nv_bfloat16* out, float* norm);
 
 // relaxation sizes of src/relaxation.jl:11-36 for a given npatterns (iq_sim.cu)

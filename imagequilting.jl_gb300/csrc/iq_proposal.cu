@@ -29,672 +29,15 @@
 #include <cmath>
 #include <cstring>
 
-#include "iq_internal.h"
+#include "iq_proposal_cells.cuh"
 
 namespace {
 
-constexpr int CH = IQ_LP_CH;
 constexpr int EMB = IQ_LP_EMB;
 constexpr int NIN = 3;
-constexpr int LT = 256;  // threads of the encoder kernels
-
-// ---- geometry -------------------------------------------------------------------------------
-__device__ __forceinline__ void cell_of(const LpGeo& g, int cell, int& i, int& j, int& k) {
-  i = cell % g.g[0];
-  j = (cell / g.g[0]) % g.g[1];
-  k = cell / (g.g[0] * g.g[1]);
-}
-
-// Features of cell `cell` of a training-image window at image origin (x0, y0, z0) under the mask
-// "tile minus box [lo, hi)": Float64 integral images ii1 (values) and ii2 (squares).
-__device__ void window_cell(const LpGeo& g, const double* __restrict__ ii1,
-                            const double* __restrict__ ii2, int64_t sx, int64_t sxy, int64_t x0,
-                            int64_t y0, int64_t z0, const int* lo, const int* hi, int cell,
-                            float* out) {
-  int c3[3];
-  cell_of(g, cell, c3[0], c3[1], c3[2]);
-  int a[3], b[3], ia[3], ib[3];
-  bool inner = true;
-  for (int d = 0; d < 3; ++d) {
-    a[d] = c3[d] * g.c[d];
-    b[d] = min(a[d] + g.c[d], g.t[d]);
-    ia[d] = max(a[d], lo[d]);
-    ib[d] = min(b[d], hi[d]);
-    inner = inner && ia[d] < ib[d];
-  }
-  double s1 = 0.0, s2 = 0.0, cnt = 0.0;
-  if (b[0] > a[0] && b[1] > a[1] && b[2] > a[2]) {
-    s1 = iq_box_sum(ii1, sx, sxy, x0 + a[0], y0 + a[1], z0 + a[2], b[0] - a[0], b[1] - a[1],
-                    b[2] - a[2]);
-    s2 = iq_box_sum(ii2, sx, sxy, x0 + a[0], y0 + a[1], z0 + a[2], b[0] - a[0], b[1] - a[1],
-                    b[2] - a[2]);
-    cnt = (double)(b[0] - a[0]) * (b[1] - a[1]) * (b[2] - a[2]);
-    if (inner) {
-      s1 -= iq_box_sum(ii1, sx, sxy, x0 + ia[0], y0 + ia[1], z0 + ia[2], ib[0] - ia[0],
-                       ib[1] - ia[1], ib[2] - ia[2]);
-      s2 -= iq_box_sum(ii2, sx, sxy, x0 + ia[0], y0 + ia[1], z0 + ia[2], ib[0] - ia[0],
-                       ib[1] - ia[1], ib[2] - ia[2]);
-      cnt -= (double)(ib[0] - ia[0]) * (ib[1] - ia[1]) * (ib[2] - ia[2]);
-    }
-  }
-  const double vol = (double)g.c[0] * g.c[1] * g.c[2];
-  out[0] = (float)(cnt / vol);
-  out[1] = (float)(s1 / vol);
-  out[2] = (float)(s2 / vol);
-}
-
-// Features of cell `cell` of a template: the simulation grid at `src` (grid strides gx, gxy),
-// summed directly over the cell's voxels outside the box.
-__device__ void template_cell(const LpGeo& g, const float* __restrict__ src, int64_t gx,
-                              int64_t gxy, const int* lo, const int* hi, int cell, float* out) {
-  int c3[3];
-  cell_of(g, cell, c3[0], c3[1], c3[2]);
-  // rows summed in FP32, rows added in Float64 (exact for integer codes, the proposal's data;
-  // GB300's FP64 pipe is narrow, so FP64 work per row rather than per voxel)
-  double s1 = 0.0, s2 = 0.0;
-  int cnt = 0;
-  const int a0 = c3[0] * g.c[0], a1 = c3[1] * g.c[1], a2 = c3[2] * g.c[2];
-  const int b0 = min(a0 + g.c[0], g.t[0]), b1 = min(a1 + g.c[1], g.t[1]), b2 = min(a2 + g.c[2], g.t[2]);
-  for (int z = a2; z < b2; ++z)
-    for (int y = a1; y < b1; ++y) {
-      const bool rin = y >= lo[1] && y < hi[1] && z >= lo[2] && z < hi[2];
-      float r1 = 0.f, r2 = 0.f;
-      for (int x = a0; x < b0; ++x) {
-        if (rin && x >= lo[0] && x < hi[0]) continue;
-        const float v = src[x + gx * y + gxy * z];
-        r1 += v;
-        r2 = fmaf(v, v, r2);
-        ++cnt;
-      }
-      s1 += (double)r1;
-      s2 += (double)r2;
-    }
-  const double vol = (double)g.c[0] * g.c[1] * g.c[2];
-  out[0] = (float)((double)cnt / vol);
-  out[1] = (float)(s1 / vol);
-  out[2] = (float)(s2 / vol);
-}
-
-// ---- one encoder pass in shared memory ------------------------------------------------------
-// Weights are read through W(i) (BF16 or FP32 storage); X: [NIN][G], h1: [CH][G],
-// h2: [CH][G2], h3: [CH][G3] (pre-activations z kept when zbuf is set, for the backward pass).
-template <typename WT>
-__device__ __forceinline__ float wget(const WT* w, int i) { return (float)w[i]; }
-template <>
-__device__ __forceinline__ float wget<__nv_bfloat16>(const __nv_bfloat16* w, int i) {
-  return __bfloat162float(w[i]);
-}
-
-__device__ __forceinline__ int tap_cell(const int* G, int ox, int oy, int oz, int t) {
-  const int x = 2 * ox + (t % 3) - 1, y = 2 * oy + ((t / 3) % 3) - 1, z = 2 * oz + (t / 9) - 1;
-  if (x < 0 || y < 0 || z < 0 || x >= G[0] || y >= G[1] || z >= G[2]) return -1;
-  return x + G[0] * (y + G[1] * z);
-}
-
-template <typename WT>
-__device__ void enc_forward(const LpGeo& g, const WT* __restrict__ w, const float* X, float* h1,
-                            float* z1, float* h2, float* z2, float* h3, float* z3, float* e) {
-  const int G = g.ng, G2 = g.ng2, G3 = g.ng3;
-  for (int o = threadIdx.x; o < CH * G; o += blockDim.x) {
-    const int c = o / G, cell = o - c * G;
-    float acc = wget(w, LP_OFF_B1 + c);
-#pragma unroll
-    for (int ci = 0; ci < NIN; ++ci) acc = fmaf(wget(w, LP_OFF_W1 + c * NIN + ci), X[ci * G + cell], acc);
-    if (z1) z1[o] = acc;
-    h1[o] = fmaxf(acc, 0.f);
-  }
-  __syncthreads();
-  for (int o = threadIdx.x; o < CH * G2; o += blockDim.x) {
-    const int c = o / G2, m = o - c * G2;
-    const int ox = m % g.g2[0], oy = (m / g.g2[0]) % g.g2[1], oz = m / (g.g2[0] * g.g2[1]);
-    float acc = wget(w, LP_OFF_B2 + c);
-    for (int t = 0; t < 27; ++t) {
-      const int src = tap_cell(g.g, ox, oy, oz, t);
-      if (src < 0) continue;
-      const int wb = LP_OFF_W2 + c * CH * 27 + t;
-      for (int ci = 0; ci < CH; ++ci) acc = fmaf(wget(w, wb + ci * 27), h1[ci * G + src], acc);
-    }
-    if (z2) z2[o] = acc;
-    h2[o] = fmaxf(acc, 0.f);
-  }
-  __syncthreads();
-  for (int o = threadIdx.x; o < CH * G3; o += blockDim.x) {
-    const int c = o / G3, m = o - c * G3;
-    const int ox = m % g.g3[0], oy = (m / g.g3[0]) % g.g3[1], oz = m / (g.g3[0] * g.g3[1]);
-    float acc = wget(w, LP_OFF_B3 + c);
-    for (int t = 0; t < 27; ++t) {
-      const int src = tap_cell(g.g2, ox, oy, oz, t);
-      if (src < 0) continue;
-      const int wb = LP_OFF_W3 + c * CH * 27 + t;
-      for (int ci = 0; ci < CH; ++ci) acc = fmaf(wget(w, wb + ci * 27), h2[ci * G2 + src], acc);
-    }
-    if (z3) z3[o] = acc;
-    h3[o] = fmaxf(acc, 0.f);
-  }
-  __syncthreads();
-  const int nf = CH * G3;
-  for (int o = threadIdx.x; o < EMB; o += blockDim.x) {
-    float acc = wget(w, g.off_b4 + o);
-    for (int f = 0; f < nf; ++f) {
-      const int c = f % CH, m = f / CH;  // flat feature: channel fastest, then cell
-      acc = fmaf(wget(w, LP_OFF_W4 + o * nf + f), h3[c * G3 + m], acc);
-    }
-    e[o] = acc;
-  }
-  __syncthreads();
-}
-
-// Shared-memory layout of the encoder kernels (floats): X, h1, h2, h3, e
-constexpr int SM_X = 0;
-constexpr int SM_H1 = SM_X + NIN * IQ_LP_MAXG;
-constexpr int SM_H2 = SM_H1 + CH * IQ_LP_MAXG;
-constexpr int SM_H3 = SM_H2 + CH * IQ_LP_MAXG2;
-constexpr int SM_E = SM_H3 + CH * IQ_LP_MAXG3;
-constexpr int SM_END = SM_E + EMB;
-
-// ---- inference: embeddings of windows or templates ------------------------------------------
-struct EncArgs {
-  LpGeo g;
-  const float* w;        // FP32 parameters (converted to BF16 in shared memory)
-  int npar;
-  int64_t n;             // items
-  // windows: positions 0..n-1 of the distance map (strides dx, dxy) on the image
-  const double* ii1;
-  const double* ii2;
-  int64_t isx, isxy;     // integral-image strides (x + 1, (x + 1)(y + 1))
-  int64_t dx, dxy;
-  int lo[3], hi[3];      // mask box
-  // templates (when tsrc is set): item i reads grid + tsrc[i]
-  const float* grid;
-  const int64_t* tsrc;
-  int64_t gx, gxy;
-  const int* tbox;       // per item: lo[3], hi[3] (nullable: lo/hi above)
-  const int64_t* pos;    // windows: per item the position (nullable: item i is position i)
-  __nv_bfloat16* out;    // n x EMB
-  float* norm;           // n: |e|^2 of the BF16 embedding
-};
-
-__global__ void __launch_bounds__(LT) lp_encode_kernel(const EncArgs a) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  float* sm = reinterpret_cast<float*>(smraw);
-  __nv_bfloat16* wb = reinterpret_cast<__nv_bfloat16*>(sm + SM_END);
-  for (int i = threadIdx.x; i < a.npar; i += blockDim.x) wb[i] = __float2bfloat16_rn(a.w[i]);
-  __syncthreads();
-  float* X = sm + SM_X;
-  for (int64_t item = blockIdx.x; item < a.n; item += gridDim.x) {
-    int lo[3], hi[3];
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = a.tbox ? a.tbox[6 * item + d] : a.lo[d];
-      hi[d] = a.tbox ? a.tbox[6 * item + 3 + d] : a.hi[d];
-    }
-    for (int cell = threadIdx.x; cell < a.g.ng; cell += blockDim.x) {
-      float f[3];
-      if (a.tsrc) {
-        template_cell(a.g, a.grid + a.tsrc[item], a.gx, a.gxy, lo, hi, cell, f);
-      } else {
-        const int64_t q = a.pos ? a.pos[item] : item;
-        const int64_t z = q / a.dxy, r = q - z * a.dxy, y = r / a.dx, x = r - y * a.dx;
-        window_cell(a.g, a.ii1, a.ii2, a.isx, a.isxy, x, y, z, lo, hi, cell, f);
-      }
-      for (int c = 0; c < NIN; ++c) X[c * a.g.ng + cell] = f[c];
-    }
-    __syncthreads();
-    enc_forward<__nv_bfloat16>(a.g, wb, X, sm + SM_H1, nullptr, sm + SM_H2, nullptr, sm + SM_H3,
-                               nullptr, sm + SM_E);
-    if (threadIdx.x < 32) {
-      float s = 0.f;
-      for (int o = threadIdx.x; o < EMB; o += 32) {
-        const __nv_bfloat16 v = __float2bfloat16_rn(sm[SM_E + o]);
-        a.out[item * EMB + o] = v;
-        const float fv = __bfloat162float(v);
-        s = fmaf(fv, fv, s);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (threadIdx.x == 0) a.norm[item] = s;
-    }
-    __syncthreads();
-  }
-}
+constexpr int LT = 256;  // threads of the template feature kernel
 
 }  // namespace
-
-// ---------------------------------------------------------------------------------------------
-LpGeo iq_lp_geo(Dim3 tile) {
-  LpGeo g{};
-  const int64_t t[3] = {tile.x, tile.y, tile.z};
-  const int gm[3] = {8, 8, 4};
-  for (int d = 0; d < 3; ++d) {
-    g.t[d] = (int)t[d];
-    g.g[d] = (int)std::min<int64_t>(t[d], gm[d]);
-    g.c[d] = (int)((t[d] + g.g[d] - 1) / g.g[d]);
-    g.g2[d] = (g.g[d] + 1) / 2;
-    g.g3[d] = (g.g2[d] + 1) / 2;
-  }
-  g.ng = g.g[0] * g.g[1] * g.g[2];
-  g.ng2 = g.g2[0] * g.g2[1] * g.g2[2];
-  g.ng3 = g.g3[0] * g.g3[1] * g.g3[2];
-  g.nf = CH * g.ng3;
-  g.off_b4 = LP_OFF_W4 + EMB * g.nf;
-  g.npar = g.off_b4 + EMB;
-  return g;
-}
-
-static size_t enc_smem(const LpGeo& g) {
-  return sizeof(float) * SM_END + sizeof(__nv_bfloat16) * (size_t)g.npar + 16;
-}
-
-int iq_lp_encode_windows(iq_ctx* ctx, const LpGeo& g, const float* w, const double* ii1,
-                         const double* ii2, Dim3 img, Dim3 dist, const int* lo, const int* hi,
-                         __nv_bfloat16* out, float* norm, const int64_t* pos, int64_t npos) {
-  EncArgs a{};
-  a.g = g; a.w = w; a.npar = g.npar; a.n = pos ? npos : dist.vol();
-  a.pos = pos;
-  a.ii1 = ii1; a.ii2 = ii2; a.isx = img.x + 1; a.isxy = (img.x + 1) * (img.y + 1);
-  a.dx = dist.x; a.dxy = dist.x * dist.y;
-  for (int d = 0; d < 3; ++d) { a.lo[d] = lo[d]; a.hi[d] = hi[d]; }
-  a.out = out; a.norm = norm;
-  const size_t sm = enc_smem(g);
-  IQ_CUDA_OK(cudaFuncSetAttribute(lp_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t blocks = std::min<int64_t>(a.n, (int64_t)nsm * 4);
-  iq_timer_start(ctx, "lp.encode");
-  lp_encode_kernel<<<(unsigned)blocks, LT, sm, ctx->stream>>>(a);
-  iq_timer_stop(ctx, "lp.encode");
-  iq_count(ctx);
-  IQ_CUDA_OK(cudaGetLastError());
-  return IQ_OK;
-}
-
-int iq_lp_encode_templates(iq_ctx* ctx, const LpGeo& g, const float* w, const float* grid,
-                           Dim3 gdims, const int64_t* tsrc, const int* tbox, int64_t n,
-                           __nv_bfloat16* out, float* norm) {
-  if (n <= 0) return IQ_OK;
-  EncArgs a{};
-  a.g = g; a.w = w; a.npar = g.npar; a.n = n;
-  a.grid = grid; a.tsrc = tsrc; a.gx = gdims.x; a.gxy = gdims.x * gdims.y; a.tbox = tbox;
-  a.out = out; a.norm = norm;
-  const size_t sm = enc_smem(g);
-  IQ_CUDA_OK(cudaFuncSetAttribute(lp_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  iq_timer_start(ctx, "lp.encode");
-  lp_encode_kernel<<<(unsigned)std::min<int64_t>(n, 4096), LT, sm, ctx->stream>>>(a);
-  iq_timer_stop(ctx, "lp.encode");
-  iq_count(ctx);
-  IQ_CUDA_OK(cudaGetLastError());
-  return IQ_OK;
-}
-
-// =============================================================================================
-// Training: FP32 forward, InfoNCE loss, backward with parameter gradients, Adam
-// =============================================================================================
-namespace {
-
-// One training item: the features of a template (feat >= 0: row of `feats`) or a window of the
-// image at distance-map position `pos` under the mask box of anchor `box`.
-struct TrainItem {
-  int32_t feat;   // row of the anchor feature table, or -1
-  int32_t pos;    // window position when feat < 0
-  int32_t box;    // row of the box table
-  int32_t pad_;
-};
-
-struct TrainArgs {
-  LpGeo g;
-  const float* w;              // FP32 parameters
-  const TrainItem* items;
-  int64_t nitems;
-  const float* feats;          // [rows][NIN * ng]
-  const int32_t* boxes;        // [rows][6]
-  const double* ii1;
-  const double* ii2;
-  int64_t isx, isxy, dx, dxy;
-  float* X;                    // [nitems][NIN * ng] features (written by the forward pass)
-  float* E;                    // [nitems][EMB]
-  const float* gE;             // [nitems][EMB] d loss / d embedding (backward)
-  float* grad;                 // parameter gradients (accumulated)
-};
-
-__device__ void item_features(const TrainArgs& a, const TrainItem& it, float* X) {
-  const int G = a.g.ng;
-  if (it.feat >= 0) {
-    for (int i = threadIdx.x; i < NIN * G; i += blockDim.x) X[i] = a.feats[(int64_t)it.feat * NIN * G + i];
-  } else {
-    int lo[3], hi[3];
-    for (int d = 0; d < 3; ++d) { lo[d] = a.boxes[6 * it.box + d]; hi[d] = a.boxes[6 * it.box + 3 + d]; }
-    const int64_t p = it.pos;
-    const int64_t z = p / a.dxy, r = p - z * a.dxy, y = r / a.dx, x = r - y * a.dx;
-    for (int cell = threadIdx.x; cell < G; cell += blockDim.x) {
-      float f[3];
-      window_cell(a.g, a.ii1, a.ii2, a.isx, a.isxy, x, y, z, lo, hi, cell, f);
-      for (int c = 0; c < NIN; ++c) X[c * G + cell] = f[c];
-    }
-  }
-  __syncthreads();
-}
-
-__global__ void __launch_bounds__(LT) lp_train_fwd_kernel(const TrainArgs a) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  float* sm = reinterpret_cast<float*>(smraw);
-  const int G = a.g.ng;
-  for (int64_t item = blockIdx.x; item < a.nitems; item += gridDim.x) {
-    float* X = sm + SM_X;
-    item_features(a, a.items[item], X);
-    for (int i = threadIdx.x; i < NIN * G; i += blockDim.x) a.X[item * NIN * G + i] = X[i];
-    enc_forward<float>(a.g, a.w, X, sm + SM_H1, nullptr, sm + SM_H2, nullptr, sm + SM_H3, nullptr,
-                       sm + SM_E);
-    for (int o = threadIdx.x; o < EMB; o += blockDim.x) a.E[item * EMB + o] = sm[SM_E + o];
-    __syncthreads();
-  }
-}
-
-// Backward of one item. Shared memory (floats): X, h1, h2, h3, e (as the forward), then gh1
-// [CH][G], gh2 [CH][G2], gz3 [CH][G3], gf [nf], ge [EMB].
-constexpr int SB_GH1 = SM_END;
-constexpr int SB_GH2 = SB_GH1 + CH * IQ_LP_MAXG;
-constexpr int SB_GZ3 = SB_GH2 + CH * IQ_LP_MAXG2;
-constexpr int SB_GF = SB_GZ3 + CH * IQ_LP_MAXG3;
-constexpr int SB_GE = SB_GF + CH * IQ_LP_MAXG3;
-constexpr int SB_END = SB_GE + EMB;
-
-// Cell of the layer below that output cell m reads through tap t (-1: padding), as tap_cell;
-// the inverse: output cell of grid Go reading input cell j through tap t (-1: none).
-__device__ __forceinline__ int tap_out(const int* Gi, const int* Go, int j, int t) {
-  const int jx = j % Gi[0], jy = (j / Gi[0]) % Gi[1], jz = j / (Gi[0] * Gi[1]);
-  const int dx = t % 3, dy = (t / 3) % 3, dz = t / 9;
-  const int ax = jx + 1 - dx, ay = jy + 1 - dy, az = jz + 1 - dz;
-  if ((ax | ay | az) & 1) return -1;
-  if (ax < 0 || ay < 0 || az < 0) return -1;
-  const int mx = ax >> 1, my = ay >> 1, mz = az >> 1;
-  if (mx >= Go[0] || my >= Go[1] || mz >= Go[2]) return -1;
-  return mx + Go[0] * (my + Go[1] * mz);
-}
-
-// Backward, phase 1 (one CTA per item): recompute the forward pass, then the gradients of the
-// pre-activations of every layer (zero where the ReLU was off): gz3, gz2, gz1. They and the
-// activations go to per-item buffers; phase 2 reduces them over the batch into the weight
-// gradients (no atomics).
-struct BwdBufs {
-  float* h1; float* gz1;   // [items][CH * G]
-  float* h2; float* gz2;   // [items][CH * G2]
-  float* h3; float* gz3;   // [items][CH * G3]
-};
-
-__global__ void __launch_bounds__(LT) lp_train_bwd_kernel(const TrainArgs a, const BwdBufs o) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  float* sm = reinterpret_cast<float*>(smraw);
-  const LpGeo& g = a.g;
-  const int G = g.ng, G2 = g.ng2, G3 = g.ng3, nf = g.nf;
-  const float* w = a.w;
-  for (int64_t item = blockIdx.x; item < a.nitems; item += gridDim.x) {
-    float* X = sm + SM_X;
-    float* h1 = sm + SM_H1;
-    float* h2 = sm + SM_H2;
-    float* h3 = sm + SM_H3;
-    for (int i = threadIdx.x; i < NIN * G; i += blockDim.x) X[i] = a.X[item * NIN * G + i];
-    __syncthreads();
-    enc_forward<float>(g, w, X, h1, nullptr, h2, nullptr, h3, nullptr, sm + SM_E);
-    float* ge = sm + SB_GE;
-    float* gf = sm + SB_GF;
-    float* gz3 = sm + SB_GZ3;
-    float* gh2 = sm + SB_GH2;
-    for (int i = threadIdx.x; i < EMB; i += blockDim.x) ge[i] = a.gE[item * EMB + i];
-    __syncthreads();
-    for (int f = threadIdx.x; f < nf; f += blockDim.x) {
-      float acc = 0.f;
-      for (int oo = 0; oo < EMB; ++oo) acc = fmaf(w[LP_OFF_W4 + oo * nf + f], ge[oo], acc);
-      gf[f] = acc;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < CH * G3; i += blockDim.x) {
-      const int c = i / G3, m = i - c * G3;
-      gz3[i] = h3[i] > 0.f ? gf[c + CH * m] : 0.f;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < CH * G2; i += blockDim.x) {
-      const int ci = i / G2, j = i - ci * G2;
-      float acc = 0.f;
-      if (h2[i] > 0.f) {
-        for (int t = 0; t < 27; ++t) {
-          const int m = tap_out(g.g2, g.g3, j, t);
-          if (m < 0) continue;
-          for (int c = 0; c < CH; ++c) acc = fmaf(w[LP_OFF_W3 + (c * CH + ci) * 27 + t], gz3[c * G3 + m], acc);
-        }
-      }
-      gh2[i] = acc;  // d/dz2
-    }
-    __syncthreads();
-    float* gz1 = o.gz1 + item * CH * G;
-    for (int i = threadIdx.x; i < CH * G; i += blockDim.x) {
-      const int ci = i / G, j = i - ci * G;
-      float acc = 0.f;
-      if (h1[i] > 0.f) {
-        for (int t = 0; t < 27; ++t) {
-          const int m = tap_out(g.g, g.g2, j, t);
-          if (m < 0) continue;
-          for (int c = 0; c < CH; ++c) acc = fmaf(w[LP_OFF_W2 + (c * CH + ci) * 27 + t], gh2[c * G2 + m], acc);
-        }
-      }
-      gz1[i] = acc;  // d/dz1
-      o.h1[item * CH * G + i] = h1[i];
-    }
-    for (int i = threadIdx.x; i < CH * G2; i += blockDim.x) {
-      o.h2[item * CH * G2 + i] = h2[i];
-      o.gz2[item * CH * G2 + i] = gh2[i];
-    }
-    for (int i = threadIdx.x; i < CH * G3; i += blockDim.x) {
-      o.h3[item * CH * G3 + i] = h3[i];
-      o.gz3[item * CH * G3 + i] = gz3[i];
-    }
-    __syncthreads();
-  }
-}
-
-// Phase 2, convolution layers: CTA (tap t, output channel c); thread (input channel ci, part):
-// grad W[c][ci][t] = sum over items and output cells m of gz[c][m] * h_in[ci][tap(m, t)];
-// the bias gradient of c with tap 0.
-__global__ void lp_grad_conv_kernel(LpGeo g, int layer, const float* __restrict__ gz,
-                                    const float* __restrict__ hin, int64_t nitems, float* grad) {
-  __shared__ float red[8][CH];
-  __shared__ float bred[8];
-  const int t = blockIdx.x, c = blockIdx.y;
-  const int ci = threadIdx.x & 31, part = threadIdx.x >> 5;
-  const int* Gin = layer == 2 ? g.g : g.g2;
-  const int* Go = layer == 2 ? g.g2 : g.g3;
-  const int nin = layer == 2 ? g.ng : g.ng2;
-  const int nout = layer == 2 ? g.ng2 : g.ng3;
-  float acc = 0.f, bacc = 0.f;
-  for (int64_t item = part; item < nitems; item += 8) {
-    const float* gzi = gz + item * CH * nout + c * nout;
-    const float* hi = hin + item * CH * nin + ci * nin;
-    for (int m = 0; m < nout; ++m) {
-      const float gv = gzi[m];
-      if (t == 0 && ci == 0) bacc += gv;
-      if (gv == 0.f) continue;
-      const int ox = m % Go[0], oy = (m / Go[0]) % Go[1], oz = m / (Go[0] * Go[1]);
-      const int src = tap_cell(Gin, ox, oy, oz, t);
-      if (src >= 0) acc = fmaf(gv, hi[src], acc);
-    }
-  }
-  red[part][ci] = acc;
-  if (ci == 0) bred[part] = bacc;
-  __syncthreads();
-  if (part == 0) {
-    float s = 0.f;
-    for (int q = 0; q < 8; ++q) s += red[q][ci];
-    const int woff = layer == 2 ? LP_OFF_W2 : LP_OFF_W3;
-    grad[woff + (c * CH + ci) * 27 + t] = s;
-    if (t == 0 && ci == 0) {
-      float bs = 0.f;
-      for (int q = 0; q < 8; ++q) bs += bred[q];
-      grad[(layer == 2 ? LP_OFF_B2 : LP_OFF_B3) + c] = bs;
-    }
-  }
-}
-
-// Phase 2, first layer: CTA per channel c: grad W1[c][ci] = sum gz1[c][cell] X[ci][cell], bias.
-__global__ void lp_grad_w1_kernel(LpGeo g, const float* __restrict__ gz1, const float* __restrict__ X,
-                                  int64_t nitems, float* grad) {
-  __shared__ float red[4][LT];
-  const int c = blockIdx.x, G = g.ng;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int64_t i = threadIdx.x; i < nitems * G; i += blockDim.x) {
-    const int64_t item = i / G;
-    const int cell = (int)(i - item * G);
-    const float gv = gz1[item * CH * G + c * G + cell];
-    for (int q = 0; q < NIN; ++q) acc[q] = fmaf(gv, X[item * NIN * G + q * G + cell], acc[q]);
-    acc[3] += gv;
-  }
-  for (int q = 0; q < 4; ++q) red[q][threadIdx.x] = acc[q];
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    float s = 0.f;
-    for (int i = 0; i < LT; ++i) s += red[threadIdx.x][i];
-    if (threadIdx.x < NIN) grad[LP_OFF_W1 + c * NIN + threadIdx.x] = s;
-    else grad[LP_OFF_B1 + c] = s;
-  }
-}
-
-// Phase 2, output layer: one thread per weight (and per bias): sums over the items.
-__global__ void lp_grad_w4_kernel(LpGeo g, const float* __restrict__ gE, const float* __restrict__ h3,
-                                  int64_t nitems, float* grad) {
-  const int nf = g.nf, G3 = g.ng3;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < EMB * nf) {
-    const int oo = i / nf, f = i - oo * nf;
-    const int c = f % CH, m = f / CH;
-    float acc = 0.f;
-    for (int64_t item = 0; item < nitems; ++item)
-      acc = fmaf(gE[item * EMB + oo], h3[item * CH * G3 + c * G3 + m], acc);
-    grad[LP_OFF_W4 + i] = acc;
-  } else if (i < EMB * nf + EMB) {
-    const int oo = i - EMB * nf;
-    float acc = 0.f;
-    for (int64_t item = 0; item < nitems; ++item) acc += gE[item * EMB + oo];
-    grad[g.off_b4 + oo] = acc;
-  }
-}
-
-// InfoNCE of anchor b (one warp): items b (anchor), nA + b (positive), 2 nA + b * nneg + n
-// (negatives). Writes d loss / d embedding of those items (scaled by 1 / nA) and adds the loss.
-__global__ void lp_loss_kernel(const float* __restrict__ E, int nA, int nneg, float temp,
-                               float* gE, double* loss) {
-  const int lane = threadIdx.x & 31;
-  const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (b >= nA) return;
-  const int nj = 1 + nneg;
-  auto item_of = [&](int j) -> int64_t {
-    return j == 0 ? (int64_t)nA + b : 2 * (int64_t)nA + (int64_t)b * nneg + (j - 1);
-  };
-  const float a0 = E[(int64_t)b * EMB + lane], a1 = E[(int64_t)b * EMB + 32 + lane];
-  // logits
-  float zmax = -1e30f;
-  for (int j = 0; j < nj; ++j) {
-    const int64_t it = item_of(j);
-    const float d0 = a0 - E[it * EMB + lane], d1 = a1 - E[it * EMB + 32 + lane];
-    float s = d0 * d0 + d1 * d1;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    zmax = fmaxf(zmax, -s / temp);
-  }
-  float den = 0.f, z0 = 0.f;
-  for (int j = 0; j < nj; ++j) {
-    const int64_t it = item_of(j);
-    const float d0 = a0 - E[it * EMB + lane], d1 = a1 - E[it * EMB + 32 + lane];
-    float s = d0 * d0 + d1 * d1;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const float z = -s / temp;
-    if (j == 0) z0 = z;
-    den += expf(z - zmax);
-  }
-  if (lane == 0) atomicAdd(loss, (double)(-z0 + zmax + logf(den)) / nA);
-  float ga0 = 0.f, ga1 = 0.f;
-  const float sc = 1.f / (float)nA;
-  for (int j = 0; j < nj; ++j) {
-    const int64_t it = item_of(j);
-    const float d0 = a0 - E[it * EMB + lane], d1 = a1 - E[it * EMB + 32 + lane];
-    float s = d0 * d0 + d1 * d1;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    float gz = expf(-s / temp - zmax) / den - (j == 0 ? 1.f : 0.f);
-    gz *= sc;
-    // z_j = -|ea - ej|^2 / T: dz/dea = -2 d / T, dz/dej = 2 d / T
-    ga0 += gz * (-2.f * d0 / temp);
-    ga1 += gz * (-2.f * d1 / temp);
-    gE[it * EMB + lane] = gz * (2.f * d0 / temp);
-    gE[it * EMB + 32 + lane] = gz * (2.f * d1 / temp);
-  }
-  gE[(int64_t)b * EMB + lane] = ga0;
-  gE[(int64_t)b * EMB + 32 + lane] = ga1;
-}
-
-__global__ void lp_adam_kernel(float* p, const float* g, float* m, float* v, int n, float lr,
-                               float b1, float b2, float eps, float c1, float c2) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-}
-
-}  // namespace
-
-int iq_lp_train_batch(iq_ctx* ctx, const LpGeo& g, const LpTrainBatch& B, double* loss_out) {
-  const int64_t nitems = (int64_t)B.nA * (2 + B.nneg);
-  TrainArgs a{};
-  a.g = g; a.w = B.w; a.items = static_cast<const TrainItem*>(B.items); a.nitems = nitems;
-  a.feats = B.feats; a.boxes = B.boxes; a.ii1 = B.ii1; a.ii2 = B.ii2;
-  a.isx = B.img.x + 1; a.isxy = (B.img.x + 1) * (B.img.y + 1);
-  a.dx = B.dist.x; a.dxy = B.dist.x * B.dist.y;
-  a.X = B.X; a.E = B.E; a.gE = B.gE; a.grad = B.grad;
-  const size_t smf = sizeof(float) * SM_END + 16;
-  const size_t smb = sizeof(float) * SB_END + 16;
-  IQ_CUDA_OK(cudaFuncSetAttribute(lp_train_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smf));
-  IQ_CUDA_OK(cudaFuncSetAttribute(lp_train_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb));
-  cudaStream_t st = ctx->stream;
-  const unsigned blocks = (unsigned)std::min<int64_t>(nitems, 2048);
-  lp_train_fwd_kernel<<<blocks, LT, smf, st>>>(a);
-  IQ_CUDA_OK(cudaGetLastError());
-  IQ_CUDA_OK(cudaMemsetAsync(B.loss, 0, sizeof(double), st));
-  lp_loss_kernel<<<(unsigned)((B.nA + 7) / 8), 256, 0, st>>>(B.E, B.nA, B.nneg, B.temp, B.gE, B.loss);
-  IQ_CUDA_OK(cudaGetLastError());
-  BwdBufs o;
-  const int64_t G = g.ng, G2 = g.ng2, G3 = g.ng3;
-  o.h1 = (float*)iq_scratch(ctx, S_LP_BH1, sizeof(float) * nitems * CH * G);
-  o.gz1 = (float*)iq_scratch(ctx, S_LP_BGZ1, sizeof(float) * nitems * CH * G);
-  o.h2 = (float*)iq_scratch(ctx, S_LP_BH2, sizeof(float) * nitems * CH * (G2 + G3) * 2);
-  if (!o.h1 || !o.gz1 || !o.h2) return IQ_ERR_ALLOC;
-  o.gz2 = o.h2 + nitems * CH * G2;
-  o.h3 = o.gz2 + nitems * CH * G2;
-  o.gz3 = o.h3 + nitems * CH * G3;
-  lp_train_bwd_kernel<<<blocks, LT, smb, st>>>(a, o);
-  IQ_CUDA_OK(cudaGetLastError());
-  lp_grad_conv_kernel<<<dim3(27, CH), LT, 0, st>>>(g, 2, o.gz2, o.h1, nitems, B.grad);
-  lp_grad_conv_kernel<<<dim3(27, CH), LT, 0, st>>>(g, 3, o.gz3, o.h2, nitems, B.grad);
-  lp_grad_w1_kernel<<<CH, LT, 0, st>>>(g, o.gz1, B.X, nitems, B.grad);
-  lp_grad_w4_kernel<<<(EMB * g.nf + EMB + 255) / 256, 256, 0, st>>>(g, B.gE, o.h3, nitems, B.grad);
-  IQ_CUDA_OK(cudaGetLastError());
-  iq_count(ctx, 7);
-  if (loss_out) {
-    IQ_CUDA_OK(cudaMemcpyAsync(loss_out, B.loss, sizeof(double), cudaMemcpyDeviceToHost, st));
-    IQ_CUDA_OK(cudaStreamSynchronize(st));
-  }
-  return IQ_OK;
-}
-
-int iq_lp_adam(iq_ctx* ctx, float* p, const float* g, float* m, float* v, int n, float lr, int step) {
-  const float b1 = 0.9f, b2 = 0.999f;
-  const float c1 = 1.f - std::pow(b1, (float)step), c2 = 1.f - std::pow(b2, (float)step);
-  lp_adam_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(p, g, m, v, n, lr, b1, b2, 1e-8f, c1, c2);
-  iq_count(ctx);
-  IQ_CUDA_OK(cudaGetLastError());
-  return IQ_OK;
-}
 
 // =============================================================================================
 // Shortlist: sampled per-column threshold, then a tensor-core scan of every position
@@ -852,7 +195,7 @@ __global__ void lp_template_features_kernel(LpGeo g, const float* grid, const in
     for (int d = 0; d < 3; ++d) { lo[d] = tbox[6 * item + d]; hi[d] = tbox[6 * item + 3 + d]; }
     for (int cell = threadIdx.x; cell < g.ng; cell += blockDim.x) {
       float f[3];
-      template_cell(g, grid + tsrc[item], gx, gxy, lo, hi, cell, f);
+      template_cell<false>(g, grid + tsrc[item], gx, gxy, lo, hi, cell, f);
       for (int c = 0; c < NIN; ++c) out[item * NIN * g.ng + c * g.ng + cell] = f[c];
     }
   }

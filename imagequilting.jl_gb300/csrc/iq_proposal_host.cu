@@ -41,6 +41,9 @@ struct IqLp {
   double* ii1 = nullptr;  // Float64 integral image of the values
   size_t ii1_bytes = 0;
   int64_t ii1_ti = -1;
+  int* iq = nullptr;      // 32-bit integral images of the values and squares (integer data)
+  size_t iq_bytes = 0;
+  int64_t iq_ti = -1;
   uint8_t* ti8 = nullptr;  // the image as bytes (the exact sums of the shortlist pick)
   size_t ti8_bytes = 0;
   int64_t ti8_ti = -1;
@@ -148,6 +151,38 @@ int ensure_ii1(iq_ctx* ctx, IqLp* lp) {
   return IQ_OK;
 }
 
+// The training image as the encoder reads its windows (the integral images made when missing).
+int windows_of(iq_ctx* ctx, IqLp* lp, LpWindows* W) {
+  int rc = ensure_ii1(ctx, lp);
+  if (rc) return rc;
+  W->ii1 = lp->ii1;
+  W->ii2 = ctx->d_ti2ii;
+  W->iq1 = W->iq2 = nullptr;
+  W->img = ctx->ti;
+  W->dist = Dim3{ctx->ti.x - lp->tile.x + 1, ctx->ti.y - lp->tile.y + 1, ctx->ti.z - lp->tile.z + 1};
+  if (!iq_lp_int_cells(ctx->ti_stats, lp->tile)) return IQ_OK;
+  const int64_t n = (ctx->ti.x + 1) * (ctx->ti.y + 1) * (ctx->ti.z + 1);
+  if (!lp->iq || lp->iq_ti != ctx->ti_version) {
+    const size_t bytes = 2 * sizeof(int) * (size_t)n;
+    if (lp->iq_bytes < bytes) {
+      cudaFree(lp->iq);
+      lp->iq = nullptr;
+      lp->iq_bytes = 0;
+      if (cudaMalloc(&lp->iq, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return iq_set_error(IQ_ERR_ALLOC, "proposal: integral image allocation failed");
+      }
+      lp->iq_bytes = bytes;
+    }
+    if ((rc = iq_lp_int_integral(ctx, lp->ii1, n, lp->iq))) return rc;
+    if ((rc = iq_lp_int_integral(ctx, ctx->d_ti2ii, n, lp->iq + n))) return rc;
+    lp->iq_ti = ctx->ti_version;
+  }
+  W->iq1 = lp->iq;
+  W->iq2 = lp->iq + n;
+  return IQ_OK;
+}
+
 // The image as bytes, when every value is an integer in [0, 255] (categorical codes).
 int ensure_ti8(iq_ctx* ctx, IqLp* lp) {
   if (lp->ti8_ti == ctx->ti_version) return IQ_OK;
@@ -236,10 +271,6 @@ void make_quads(Dim3 tile, const int32_t* lohi, int64_t isx, int64_t isxy, int64
       }
 }
 
-Dim3 dist_of(iq_ctx* ctx, Dim3 tile) {
-  return Dim3{ctx->ti.x - tile.x + 1, ctx->ti.y - tile.y + 1, ctx->ti.z - tile.z + 1};
-}
-
 // Window embeddings of every position under the mask box lohi (cached per training image and
 // parameters).
 int window_embeddings(iq_ctx* ctx, IqLp* lp, const int32_t* lohi, const LpCache** out) {
@@ -250,10 +281,10 @@ int window_embeddings(iq_ctx* ctx, IqLp* lp, const int32_t* lohi, const LpCache*
   }
   for (const LpCache& c : lp->cache)
     if (!memcmp(c.lohi, lohi, sizeof(c.lohi))) { *out = &c; return IQ_OK; }
-  int rc = ensure_ii1(ctx, lp);
+  LpWindows win;
+  int rc = windows_of(ctx, lp, &win);
   if (rc) return rc;
-  const Dim3 dist = dist_of(ctx, lp->tile);
-  const int64_t P = dist.vol();
+  const int64_t P = win.dist.vol();
   LpCache c;
   memcpy(c.lohi, lohi, sizeof(c.lohi));
   if (cudaMalloc(&c.W, sizeof(__nv_bfloat16) * P * IQ_LP_EMB) != cudaSuccess ||
@@ -266,8 +297,7 @@ int window_embeddings(iq_ctx* ctx, IqLp* lp, const int32_t* lohi, const LpCache*
     cudaFree(c.Ws);
     return iq_set_error(IQ_ERR_ALLOC, "proposal: window embeddings of %lld positions", (long long)P);
   }
-  rc = iq_lp_encode_windows(ctx, lp->g, lp->w, lp->ii1, ctx->d_ti2ii, ctx->ti, dist, lohi,
-                            lohi + 3, c.W, c.nW);
+  rc = iq_lp_encode_windows(ctx, lp->g, lp->w, win, lohi, lohi + 3, c.W, c.nW);
   if (!rc) rc = iq_lp_sample_rows(ctx, c.W, c.nW, P, c.Ws, c.nWs);
   if (rc) {
     cudaFree(c.W); cudaFree(c.nW); cudaFree(c.Ws); cudaFree(c.nWs);
@@ -287,6 +317,7 @@ void iq_lp_free(iq_ctx* ctx) {
   cudaFree(lp->ti8); cudaFree(lp->ti2); cudaFree(lp->d_bad);
   cudaFree(lp->w); cudaFree(lp->m); cudaFree(lp->v); cudaFree(lp->grad); cudaFree(lp->loss);
   cudaFree(lp->ii1);
+  cudaFree(lp->iq);
   cudaFree(lp->cap_feat); cudaFree(lp->cap_box); cudaFree(lp->cap_pos);
   cudaFree(lp->d_counters); cudaFree(lp->d_dmin);
   delete lp;
@@ -392,7 +423,8 @@ int iq_lp_run_chunk(iq_ctx* ctx, const LpChunk& c, int64_t chunk_index, int* don
   IQ_CUDA_OK(cudaMemcpyAsync(dtsrc, tsrc.data(), sizeof(int64_t) * N, cudaMemcpyHostToDevice, st));
   IQ_CUDA_OK(cudaMemcpyAsync(dtbox, tbox.data(), sizeof(int32_t) * 6 * N, cudaMemcpyHostToDevice, st));
   IQ_CUDA_OK(cudaMemcpyAsync(dcols, cols.data(), sizeof(LpColumn) * N, cudaMemcpyHostToDevice, st));
-  int rc = iq_lp_encode_templates(ctx, lp->g, lp->w, c.sim, c.sim_dims, dtsrc, dtbox, N, dT, dnT);
+  int rc = iq_lp_encode_templates(ctx, lp->g, lp->w, c.sim, c.sim_dims, dtsrc, dtbox, N,
+                                  iq_lp_int_cells(ctx->ti_stats, c.tile_dims), dT, dnT);
   if (rc) return rc;
   // shortlists, one scan per mask configuration
   for (int q0 = 0; q0 < N;) {
@@ -599,9 +631,10 @@ extern "C" int iq_lp_embed(iq_ctx* ctx, int64_t n, const int64_t* positions, con
   IqLp* lp = ctx->lp;
   if (!lp || !lp->w) return iq_set_error(IQ_ERR_STATE, "no proposal parameters (iq_lp_init)");
   IQ_CUDA_OK(cudaSetDevice(ctx->device));
-  int rc = ensure_ii1(ctx, lp);
+  LpWindows win;
+  int rc = windows_of(ctx, lp, &win);
   if (rc) return rc;
-  const Dim3 dist = dist_of(ctx, lp->tile);
+  const Dim3 dist = win.dist;
   int64_t* dpos = (int64_t*)iq_scratch(ctx, S_LP_TSRC, sizeof(int64_t) * n);
   __nv_bfloat16* dW = (__nv_bfloat16*)iq_scratch(ctx, S_LP_T, sizeof(__nv_bfloat16) * n * IQ_LP_EMB);
   float* dn = (float*)iq_scratch(ctx, S_LP_NT, sizeof(float) * n);
@@ -609,8 +642,7 @@ extern "C" int iq_lp_embed(iq_ctx* ctx, int64_t n, const int64_t* positions, con
   for (int64_t i = 0; i < n; ++i)
     if (positions[i] < 0 || positions[i] >= dist.vol()) return iq_set_error(IQ_ERR_ARG, "position out of range");
   IQ_CUDA_OK(cudaMemcpyAsync(dpos, positions, sizeof(int64_t) * n, cudaMemcpyHostToDevice, ctx->stream));
-  rc = iq_lp_encode_windows(ctx, lp->g, lp->w, lp->ii1, ctx->d_ti2ii, ctx->ti, dist, box, box + 3,
-                            dW, dn, dpos, n);
+  rc = iq_lp_encode_windows(ctx, lp->g, lp->w, win, box, box + 3, dW, dn, dpos, n);
   if (rc) return rc;
   std::vector<__nv_bfloat16> h((size_t)n * IQ_LP_EMB);
   IQ_CUDA_OK(cudaMemcpyAsync(h.data(), dW, sizeof(__nv_bfloat16) * h.size(), cudaMemcpyDeviceToHost,
@@ -635,12 +667,11 @@ int train_step(iq_ctx* ctx, IqLp* lp, const float* feats, const int32_t* boxes,
   if (!ditems || !dX || !dE || !dgE) return IQ_ERR_ALLOC;
   IQ_CUDA_OK(cudaMemcpyAsync(ditems, items.data(), sizeof(int32_t) * 4 * nitems,
                              cudaMemcpyHostToDevice, ctx->stream));
-  int rc = ensure_ii1(ctx, lp);
-  if (rc) return rc;
   LpTrainBatch B;
+  int rc = windows_of(ctx, lp, &B.win);
+  if (rc) return rc;
   B.w = lp->w; B.items = ditems; B.nA = nA; B.nneg = nneg; B.temp = (float)temp;
-  B.feats = feats; B.boxes = boxes; B.ii1 = lp->ii1; B.ii2 = ctx->d_ti2ii;
-  B.img = ctx->ti; B.dist = dist_of(ctx, lp->tile);
+  B.feats = feats; B.boxes = boxes;
   B.X = dX; B.E = dE; B.gE = dgE; B.grad = lp->grad; B.loss = lp->loss;
   return iq_lp_train_batch(ctx, lp->g, B, loss);  // synchronizes (host `items`)
 }
