@@ -128,7 +128,7 @@ enum IqSlot {
   S_PBH_OUT, S_PBH_POOL, S_PBH_SRC,
   S_LP_T, S_LP_NT, S_LP_TAU, S_LP_LIST, S_LP_CNT, S_LP_DL, S_LP_COLS, S_LP_TSRC, S_LP_TBOX,
   S_LP_RIND, S_LP_NCAND, S_LP_D, S_LP_BITS, S_LP_ITEMS, S_LP_X, S_LP_E, S_LP_GE, S_LP_FEAT, S_LP_BH1, S_LP_BGZ1, S_LP_BH2, S_LP_DENSE, S_LP_QUAD,
-  S_TZ_IMG, S_TZ_A2, S_TZ_PLAN, S_TZ_B, S_TZ_SIMG, S_TZ_SA2, S_PREDRAW, S_LP_W,
+  S_TZ_IMG, S_TZ_A2, S_TZ_PLAN, S_TZ_B, S_TZ_SIMG, S_TZ_SA2, S_PREDRAW, S_LP_W, S_LVL1, S_PB_MEMB,
   S_COUNT
 };
 
@@ -367,11 +367,13 @@ struct ExactSrc {
 // Refined top-k selection of a map shared by all realizations of a tile (a soft-data map),
 // computed once per (map, relaxation step): positions with D < lo are in, D > hi out, and the
 // positions in between are listed at pool + off (ascending, bit 31 set when in).
+constexpr int IQ_MEMB_CAP = 8192;  // largest refined selection listed whole
 struct PreBand {
   double lo, hi;
   int64_t off, n;
   unsigned long long key;   // the FP32 (value, index) key of the selection
   long long ties;           // near-ties at its boundary (the boundary position excluded)
+  int64_t nm;               // entries of the set's own list (-1: not listed)
   int32_t ok;               // 0: not precomputed (the pick selects itself); 1: band; 2: the
                             // map is exact and the key alone decides
   int32_t pad_;
@@ -392,7 +394,9 @@ struct PickTask {
   const PreBand* aux_pb[IQ_MAX_AUX];        // refined selections of shared maps (nullable)
   const PreBand* x0_pb;                     // D's dbsize selection, shared (nullable)
   const int32_t* x0_pool;                   // its band list
-  const int32_t* pb_pool;                   // their band lists
+  const int32_t* pb_pool;                   // their band lists, pb_cap entries per selection
+  const int32_t* memb;                      // their sets, IQ_MEMB_CAP per selection (nullable)
+  int64_t pb_cap;
   int nkeys;
   const int64_t* pre;                       // draws made on the host, per realization (nullable:
                                             // the pick makes them)
@@ -403,6 +407,7 @@ struct PickTask {
   ExactSrc xa[IQ_MAX_AUX];
 };
 
+constexpr int IQ_RANK_CAP = 4096;  // most candidates of a pick evaluated between its phases
 struct PickLaunch {
   int64_t P = 0;           // positions
   int64_t npat = 0;        // enabled positions (finite D)
@@ -428,6 +433,10 @@ struct PickLaunch {
   double* rr = nullptr;       // their error radii
   uint8_t* rl = nullptr;      // their levels
   int64_t dx = 0, dxy = 0;    // distance-map strides (x extent, x * y extents)
+  // level-1 distances of the candidates, IQ_RANK_CAP per CTA and source (1 + naux_max; nullable: the
+  // pick evaluates them itself); maxK: most offsets of a refined source
+  float* lvl1 = nullptr;
+  int maxK = 0;
   // outputs, one per CTA
   int64_t* rind = nullptr;
   int64_t* ncand = nullptr;  // nullable
@@ -452,7 +461,7 @@ int iq_launch_select_keys(iq_ctx* ctx, const float* maps, const unsigned* mm, in
 int iq_launch_select_bands(iq_ctx* ctx, const float* maps, const unsigned* mm,
                            const ExactSrc* srcs, int64_t nmaps, int64_t P, int64_t dx,
                            int64_t dxy, const int64_t* seq, int nq, PreBand* out, int32_t* pool,
-                           int64_t cap, int keys_exact = 0);
+                           int64_t cap, int keys_exact = 0, int32_t* memb = nullptr);
 
 // ---------------------------------------------------------------------------------------
 // Graph cut (iq_graphcut.cu) and paste (iq_paste.cu)

@@ -14,6 +14,13 @@
 // (value, index) keys into shared memory and a bitonic sort gives the exact key. Bins too
 // large to collect are narrowed by another histogram; a bin of one repeated value falls back
 // to a radix select over the indices. The primary and one auxiliary source share passes.
+// On continuous data the exact re-rank (below) is most of the pick. Picks of the 3-D conditioned
+// ensemble (100 x 100 x 50, tile 24 x 24 x 12, 3,456 picks of ~700 candidates and 2-3 sources),
+// 300 ms with a warp per evaluation: 177 with four evaluations sharing their terms, 165 with the
+// candidates' first evaluations spread over the chip (rank_eval_kernel), 139 with a work queue for
+// the later ones, 98 with blocked sums (a fifth of the radius, a fifth of the double-float
+// evaluations), 89 with the soft selections listed once per map. Unconditioned 3-D picks
+// (91 x 83 x 47): 16.5 -> 10.5 ms by deciding on the minimum's interval.
 // Candidate lists are compacted in ascending index order; dense ranks come from a
 // shared-memory bitonic sort (a stable LSD radix sort in global memory above 8192
 // candidates). All Float64 arithmetic uses explicit round-to-nearest intrinsics so that the
@@ -53,6 +60,10 @@ struct PickArgs {
   int* status;
   unsigned long long* ties;
   unsigned long long* stats;
+  int phase;          // 0: the whole pick; 1: up to the candidates; 2: weights and draw, with the
+                      // level-1 distances of the candidates made in between (rank_eval_kernel)
+  float* lvl1;        // [CTA][nsrc][IQ_RANK_CAP] (phases 1 and 2)
+  int nsrc;
 };
 
 // small shared state (static); the large regions are dynamic shared memory:
@@ -431,24 +442,55 @@ __device__ __noinline__ void hist_select(Smem& s, uint32_t* hist, unsigned long 
 
 constexpr double TIE_RTOL = 1e-6;                 // relative window of a reported near-tie
 
+// Positions of one compaction tile: warp w holds [t0 + 32 CITEMS w, + 32 CITEMS), lane l its every
+// 32nd position starting at l, so that a load of 32 lanes is one line (a thread with CITEMS
+// consecutive positions reads eight lines per load).
+__device__ __forceinline__ int64_t tile_pos(int64_t t0) {
+  return t0 + (int64_t)(threadIdx.x >> 5) * (32 * CITEMS) + (threadIdx.x & 31);
+}
+
+// Ordered append of the tile's positions whose bit i (position tile_pos + 32 i) is set; base
+// advances by the tile's count (the same in every thread).
+__device__ __forceinline__ void tile_append(Smem& s, uint32_t bits, int64_t t0, int32_t* out,
+                                            int64_t& base) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint32_t bal[CITEMS], cnt = 0;
+#pragma unroll
+  for (int i = 0; i < CITEMS; ++i) {
+    bal[i] = __ballot_sync(0xffffffffu, bits >> i & 1u);
+    cnt += __popc(bal[i]);
+  }
+  if (lane == 0) s.warp[wid] = cnt;
+  __syncthreads();
+  const uint32_t mine = s.warp[lane];  // NW == 32: lane w reads warp w's count
+  uint32_t inc = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += y;
+  }
+  const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
+  const uint32_t before = __shfl_sync(0xffffffffu, inc - mine, wid);
+  if (out && cnt) {
+    int64_t o = base + before;
+    const int64_t p0 = tile_pos(t0);
+#pragma unroll
+    for (int i = 0; i < CITEMS; ++i) {
+      if (bits >> i & 1u) out[o + __popc(bal[i] & lanemask_lt())] = (int32_t)(p0 + 32 * i);
+      o += __popc(bal[i]);
+    }
+  }
+  base += total;
+  __syncthreads();
+}
+
 // Ordered compaction of {p : pred(p)} into out (if non-null); returns the count.
 template <typename Pred>
 __device__ int64_t compact(Smem& s, const Pred& pred, int64_t P, int32_t* out) {
   int64_t base = 0;
   const int64_t tile = (int64_t)PT * CITEMS;
-  for (int64_t t0 = 0; t0 < P; t0 += tile) {
-    const int64_t p0 = t0 + (int64_t)threadIdx.x * CITEMS;
-    const uint32_t bits = pred.eval8(p0, P);
-    uint32_t total;
-    uint32_t off = block_excl_sum(s, (uint32_t)__popc(bits), total);
-    if (out) {
-      int64_t o = base + off;
-#pragma unroll
-      for (int i = 0; i < CITEMS; ++i)
-        if (bits >> i & 1u) out[o++] = (int32_t)(p0 + i);
-    }
-    base += total;
-  }
+  for (int64_t t0 = 0; t0 < P; t0 += tile)
+    tile_append(s, pred.eval8(tile_pos(t0), P), t0, out, base);
   return base;
 }
 
@@ -460,16 +502,16 @@ struct ThrPred {
   __device__ ThrPred(const float* d, double t, bool ties) : D(d), thr(f_dn(t)), tlo(1.f), thi(0.f) {
     if (ties && t > 0.0 && t < 1e300) tie_window_f(t, __dmul_rn(TIE_RTOL, t), tlo, thi);
   }
-  // bit i set when D[p0 + i] <= thr (positions past P excluded)
+  // bit i set when D[p0 + 32 * i] <= thr (positions past P excluded)
   __device__ uint32_t eval8(int64_t p0, int64_t P) const {
     float v[CITEMS];
 #pragma unroll
-    for (int i = 0; i < CITEMS; ++i) v[i] = p0 + i < P ? D[p0 + i] : __int_as_float(0x7F800000);
+    for (int i = 0; i < CITEMS; ++i) v[i] = p0 + 32 * i < P ? D[p0 + 32 * i] : __int_as_float(0x7F800000);
     uint32_t bits = 0;
 #pragma unroll
     for (int i = 0; i < CITEMS; ++i) {
-      if (p0 + i < P && v[i] <= thr) bits |= 1u << i;
-      if (p0 + i < P && v[i] >= tlo && v[i] <= thi) nt++;
+      if (p0 + 32 * i < P && v[i] <= thr) bits |= 1u << i;
+      if (p0 + 32 * i < P && v[i] >= tlo && v[i] <= thi) nt++;
     }
     return bits;
   }
@@ -502,6 +544,22 @@ __device__ __forceinline__ bool band_member(const Band& b, int64_t p, float d) {
   return false;  // not reached for a position inside the band
 }
 
+// the refined selection b of src
+struct BandPred {
+  const float* src;
+  const Band* b;
+  __device__ uint32_t eval8(int64_t p0, int64_t P) const {
+    float v[CITEMS];
+#pragma unroll
+    for (int i = 0; i < CITEMS; ++i) v[i] = p0 + 32 * i < P ? src[p0 + 32 * i] : __int_as_float(0x7F800000);
+    uint32_t bits = 0;
+#pragma unroll
+    for (int i = 0; i < CITEMS; ++i)
+      if (p0 + 32 * i < P && band_member(*b, p0 + 32 * i, v[i])) bits |= 1u << i;
+    return bits;
+  }
+};
+
 template <int NAUX>
 struct RelaxPred {
   const float* D; Key kD;
@@ -510,17 +568,17 @@ struct RelaxPred {
   const float* aux[NAUX > 0 ? NAUX : 1];
   Key ka[NAUX > 0 ? NAUX : 1];
   const Band* ba[NAUX > 0 ? NAUX : 1];
-  // bit i set when position p0 + i is in the top set of D and of every auxiliary source
+  // bit i set when position p0 + 32 * i is in the top set of D and of every auxiliary source
   __device__ uint32_t eval8(int64_t p0, int64_t P) const {
     uint32_t b[CITEMS];
 #pragma unroll
-    for (int i = 0; i < CITEMS; ++i) b[i] = p0 + i < P ? fbits(D[p0 + i]) : 0xFFFFFFFFu;
+    for (int i = 0; i < CITEMS; ++i) b[i] = p0 + 32 * i < P ? fbits(D[p0 + 32 * i]) : 0xFFFFFFFFu;
     uint32_t bits = 0;
 #pragma unroll
     for (int i = 0; i < CITEMS; ++i) {
-      if (p0 + i >= P) continue;
-      const bool in = bD ? band_member(*bD, p0 + i, __uint_as_float(b[i]))
-                         : key_le(b[i], (uint32_t)(p0 + i), kD);
+      if (p0 + 32 * i >= P) continue;
+      const bool in = bD ? band_member(*bD, p0 + 32 * i, __uint_as_float(b[i]))
+                         : key_le(b[i], (uint32_t)(p0 + 32 * i), kD);
       if (in) bits |= 1u << i;
     }
 #pragma unroll
@@ -528,18 +586,48 @@ struct RelaxPred {
       if (a >= naux || !bits) continue;
       uint32_t c[CITEMS];
 #pragma unroll
-      for (int i = 0; i < CITEMS; ++i) c[i] = (bits >> i & 1u) ? fbits(aux[a][p0 + i]) : 0u;
+      for (int i = 0; i < CITEMS; ++i) c[i] = (bits >> i & 1u) ? fbits(aux[a][p0 + 32 * i]) : 0u;
 #pragma unroll
       for (int i = 0; i < CITEMS; ++i) {
         if (!(bits >> i & 1u)) continue;
-        const bool in = ba[a] ? band_member(*ba[a], p0 + i, __uint_as_float(c[i]))
-                              : key_le(c[i], (uint32_t)(p0 + i), ka[a]);
+        const bool in = ba[a] ? band_member(*ba[a], p0 + 32 * i, __uint_as_float(c[i]))
+                              : key_le(c[i], (uint32_t)(p0 + 32 * i), ka[a]);
         if (!in) bits &= ~(1u << i);
       }
     }
     return bits;
   }
+  // whether position p is in the top set of D and of every auxiliary source but `skip`
+  __device__ bool one(int64_t p, int skip) const {
+    const float d = D[p];
+    if (!(bD ? band_member(*bD, p, d) : key_le(fbits(d), (uint32_t)p, kD))) return false;
+#pragma unroll
+    for (int a = 0; a < NAUX; ++a) {
+      if (a >= naux || a == skip) continue;
+      const float c = aux[a][p];
+      if (!(ba[a] ? band_member(*ba[a], p, c) : key_le(fbits(c), (uint32_t)p, ka[a]))) return false;
+    }
+    return true;
+  }
 };
+
+// Ordered compaction of the positions of list[0, m) (ascending) that pass `pr` without source `skip`
+// (the list is that source's set).
+template <int NAUX>
+__device__ int64_t compact_list(Smem& s, const RelaxPred<NAUX>& pr, int skip, const int32_t* list,
+                                int64_t m, int32_t* out) {
+  int64_t base = 0;
+  for (int64_t t0 = 0; t0 < m; t0 += PT) {
+    const int64_t i = t0 + threadIdx.x;
+    const int32_t p = i < m ? list[i] : 0;
+    const bool in = i < m && pr.one(p, skip);
+    uint32_t total;
+    const uint32_t off = block_excl_sum(s, in ? 1u : 0u, total);
+    if (in) out[base + off] = p;
+    base += total;
+  }
+  return base;
+}
 
 // Stable LSD radix sort of (keys, vals)[0..n) between the buffer pairs (global memory);
 // returns 0 if the result is in (ka, va), 1 if in (kb, vb).
@@ -686,8 +774,9 @@ __device__ __noinline__ unsigned long long dense_ranks(Smem& s, unsigned long lo
 // model), so those positions are re-evaluated directly, D[p] = sum_k (img[p + k] - tmpl_k)^2 --
 // a sum of non-negative terms without cancellation -- at increasing precision until every
 // decision is certain:
-//   level 1  FP32, 32 lanes each summing every 32nd offset, then a 5-step butterfly:
-//            relative error <= (ceil(K/32) + 8) 2^-24
+//   level 1  FP32, 32 lanes each summing every 32nd offset in blocks of REF_BLOCK, then the
+//            blocks, then a 5-step butterfly: with n = ceil(K/32) terms per lane, relative error
+//            <= (min(n, REF_BLOCK) + ceil(n / REF_BLOCK) + 9) 2^-24
 //   level 2  the same in double-float (pairs of FP32 numbers, error-free sums and products):
 //            relative error <= 4.1 (ceil(K/32) + 8) 2^-48
 //   level 3  the Float64 sequence of the oracle (oracle/direct.c): offsets in column-major
@@ -769,14 +858,18 @@ struct RefCache {
   bool on;
 };
 
-__device__ RefCache ref_cache_load(const Ref& f) {
+__device__ __forceinline__ bool ref_cacheable(const Ref& f) {
+  return f.K <= REF_CACHE && f.isxy * 1024 < ((int64_t)1 << 31);
+}
+
+__device__ RefCache ref_cache_load(const Ref& f, int cap = REF_CACHE) {
   extern __shared__ __align__(16) unsigned char dyn[];
   int32_t* off = reinterpret_cast<int32_t*>(dyn);
-  float* tv = reinterpret_cast<float*>(dyn + 4 * REF_CACHE);
-  const bool on = f.K <= REF_CACHE && f.isxy * 1024 < ((int64_t)1 << 31);
+  float* tv = reinterpret_cast<float*>(dyn + 4 * cap);
+  const bool on = ref_cacheable(f);
   __syncthreads();  // earlier users of the region are done
   if (on) {
-    for (int j = threadIdx.x; j < f.K; j += PT) {
+    for (int j = threadIdx.x; j < f.K; j += blockDim.x) {
       const uint32_t k = __ldg(f.kl + j);
       const int kx = kx_of(k), ky = ky_of(k), kz = kz_of(k);
       off[j] = (int32_t)(kx + f.isx * ky + f.isxy * kz);
@@ -797,6 +890,18 @@ __device__ __forceinline__ void ref_term_c(const Ref& f, const RefCache& c, int6
   }
 }
 
+// Level-1 sums add blocks of REF_BLOCK terms per lane, then the blocks, then the lanes: a term passes
+// through at most REF_BLOCK + blocks + 5 roundings of the sums and 3 of its own, a fifth of those of a
+// plain sum of K / 32 terms at K = 7,000 (and as few as a fifth of the level-2 evaluations follow).
+constexpr int REF_BLOCK = 16;
+
+// radius of a level-1 value
+__device__ __forceinline__ double ref_radius1(const Ref& f, double v) {
+  const int nl = (f.K + 31) / 32, nr = min(nl, REF_BLOCK) + (nl + REF_BLOCK - 1) / REF_BLOCK;
+  const double tail = (double)(f.K + 2) * RU64 * 1.02;   // level 3 vs the exact sum
+  return v * ((double)(nr + 9) * RU32 * 1.02 + tail) + (double)(f.K + 8) * TINY32 * 4.0;
+}
+
 // Warp-collective: value and radius of D[p] at `level` (every lane gets the same result). The
 // image is L2-resident and the loop is bound by the latency of its loads, so each lane issues
 // four of them before it uses the first (sixteen measured slower on config 2: more registers,
@@ -809,29 +914,32 @@ __device__ __noinline__ void ref_eval(const Ref& f, const RefCache& c, int64_t p
   const double tail = (double)(f.K + 2) * RU64 * 1.02;   // level 3 vs the exact sum
   if (level <= 1) {
     float acc = 0.f;
-    int j = lane;
-    for (; j + 3 * 32 < f.K; j += 4 * 32) {
-      float ta[4], tb[4];
+    for (int j0 = lane; j0 < f.K; j0 += 32 * REF_BLOCK) {
+      float s = 0.f;  // one block
+      for (int u0 = 0; u0 < REF_BLOCK; u0 += 4) {
+        float ta[4], tb[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) ref_term_c(f, c, base, j + 32 * u, ta[u], tb[u]);
+        for (int u = 0; u < 4; ++u) {
+          ta[u] = 0.f; tb[u] = 0.f;
+          if (j0 + 32 * (u0 + u) < f.K) ref_term_c(f, c, base, j0 + 32 * (u0 + u), ta[u], tb[u]);
+        }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float d = __fsub_rn(ta[u], tb[u]);
-        acc = __fmaf_rn(d, d, acc);
+        for (int u = 0; u < 4; ++u) {
+          const float d = __fsub_rn(ta[u], tb[u]);
+          s = __fmaf_rn(d, d, s);
+        }
       }
-    }
-    for (; j < f.K; j += 32) {
-      float a, b;
-      ref_term_c(f, c, base, j, a, b);
-      const float d = __fsub_rn(a, b);
-      acc = __fmaf_rn(d, d, acc);
+      acc = __fadd_rn(acc, s);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
     v = (double)acc;
-    r = v * ((double)(nl + 8) * RU32 * 1.02 + tail) + (double)(f.K + 8) * TINY32 * 4.0;
+    r = ref_radius1(f, v);
   } else if (level == 2) {
-    float h = 0.f, l = 0.f;
+    // two sums per lane (even and odd terms), added at the end: the double-float additions are a
+    // dependent chain of ten operations a term, and a sum of half the terms plus one addition stays
+    // within the radius
+    float h = 0.f, l = 0.f, h1 = 0.f, l1 = 0.f;
     int j = lane;
     for (; j < f.K; j += 128) {
       float ta[4], tb[4];
@@ -841,17 +949,18 @@ __device__ __noinline__ void ref_eval(const Ref& f, const RefCache& c, int64_t p
         if (j + 32 * u < f.K) ref_term_c(f, c, base, j + 32 * u, ta[u], tb[u]);
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (j + 32 * u >= f.K) break;
+      for (int u = 0; u < 4; ++u) {  // (a term past the end is 0 - 0: it adds nothing)
         const float a = ta[u], b = tb[u];
         float dh, dl;
         two_sum(a, -b, dh, dl);                               // a - b = dh + dl exactly
         const float p2 = __fmul_rn(dh, dh);
         const float pe = __fmaf_rn(dh, dh, -p2);              // dh^2 = p2 + pe exactly
         const float q = __fmaf_rn(__fadd_rn(dh, dh), dl, pe);  // + 2 dh dl (dl^2 dropped)
-        df_add(h, l, p2, q);
+        if (u & 1) df_add(h1, l1, p2, q);
+        else df_add(h, l, p2, q);
       }
     }
+    df_add(h, l, h1, l1);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float h2 = __shfl_xor_sync(0xffffffffu, h, o);
@@ -901,10 +1010,87 @@ struct RefArr {
   unsigned* ev;   // shared-memory counts of evaluations per level [4] (nullable)
 };
 
-// Level 1 for entries [0, n) of pos (warp per entry).
+// Level 1 of up to REF_BATCH entries by one warp: ref_eval's level-1 sums (the same terms in the same
+// order per lane), the offsets and template values read once for all of them and 2 x REF_BATCH image
+// loads in flight per lane. The loop is bound by the latency of those loads (L2) and by shared-memory
+// reads, two per term when entries are summed one at a time.
+constexpr int REF_BATCH = 4;
+
+template <int REF_BATCH>
+__device__ __forceinline__ void ref_eval1_batch(const Ref& f, const RefCache& c, const int32_t* pos,
+                                                int m, float (&acc)[REF_BATCH]) {
+  const int lane = threadIdx.x & 31;
+  const float* b[REF_BATCH];
+#pragma unroll
+  for (int e = 0; e < REF_BATCH; ++e) {
+    b[e] = f.img + ref_base(f, pos[e < m ? e : 0] & 0x7FFFFFFF);
+    acc[e] = 0.f;
+  }
+  int j = lane;
+  while (j < f.K) {
+    float s[REF_BATCH];  // one block of REF_BLOCK terms
+#pragma unroll
+    for (int e = 0; e < REF_BATCH; ++e) s[e] = 0.f;
+#pragma unroll 2
+    for (int q = 0; q < REF_BLOCK && j + 32 < f.K; q += 2, j += 64) {
+      const int o0 = c.off[j], o1 = c.off[j + 32];
+      const float t0 = c.tv[j], t1 = c.tv[j + 32];
+      float x0[REF_BATCH], x1[REF_BATCH];
+#pragma unroll
+      for (int e = 0; e < REF_BATCH; ++e) {
+        x0[e] = __ldg(b[e] + o0);
+        x1[e] = __ldg(b[e] + o1);
+      }
+#pragma unroll
+      for (int e = 0; e < REF_BATCH; ++e) {
+        const float d0 = __fsub_rn(x0[e], t0), d1 = __fsub_rn(x1[e], t1);
+        s[e] = __fmaf_rn(d0, d0, s[e]);
+        s[e] = __fmaf_rn(d1, d1, s[e]);
+      }
+    }
+    if (j < f.K && j + 32 >= f.K) {  // the lane's last term
+      const int o0 = c.off[j];
+      const float t0 = c.tv[j];
+#pragma unroll
+      for (int e = 0; e < REF_BATCH; ++e) {
+        const float d0 = __fsub_rn(__ldg(b[e] + o0), t0);
+        s[e] = __fmaf_rn(d0, d0, s[e]);
+      }
+      j += 32;
+    }
+#pragma unroll
+    for (int e = 0; e < REF_BATCH; ++e) acc[e] = __fadd_rn(acc[e], s[e]);
+  }
+#pragma unroll
+  for (int e = 0; e < REF_BATCH; ++e)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      acc[e] = __fadd_rn(acc[e], __shfl_xor_sync(0xffffffffu, acc[e], o));
+}
+
+// Level 1 for entries [0, n) of pos (a warp per REF_BATCH entries).
 __device__ __noinline__ void ref_init(const Ref& f, const int32_t* pos, int64_t n, RefArr a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const RefCache c = ref_cache_load(f);
+  if (c.on) {
+    // few entries: spread them over the warps before batching them
+    const int bat = n >= (int64_t)NW * REF_BATCH ? REF_BATCH : (int)((n + NW - 1) / NW);
+    for (int64_t i = (int64_t)warp * bat; i < n; i += (int64_t)NW * bat) {
+      const int m = (int)min((int64_t)bat, n - i);
+      float acc[REF_BATCH];
+      ref_eval1_batch(f, c, pos + i, m, acc);
+      if (lane < m) {
+        float x = acc[0];
+#pragma unroll
+        for (int e = 1; e < REF_BATCH; ++e) x = lane == e ? acc[e] : x;
+        const double v = (double)x;
+        a.v[i + lane] = v; a.r[i + lane] = ref_radius1(f, v); a.l[i + lane] = 1;
+        if (a.ev) atomicAdd(a.ev + 1, 1u);
+      }
+    }
+    __syncthreads();
+    return;
+  }
   for (int64_t i = warp; i < n; i += NW) {
     double v, r;
     ref_eval(f, c, pos[i] & 0x7FFFFFFF, 1, v, r);
@@ -918,17 +1104,31 @@ __device__ __noinline__ void ref_init(const Ref& f, const int32_t* pos, int64_t 
 
 // Raise every marked entry by one level, or to level 3 when `to3`.
 __device__ __noinline__ void ref_raise(const Ref& f, const int32_t* pos, int64_t n, RefArr a, bool to3) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const RefCache c = ref_cache_load(f);
-  for (int64_t i = warp; i < n; i += NW) {
-    const uint8_t l = a.l[i];
-    if (!(l & 0x80)) continue;
-    const int nl = to3 ? 3 : min((l & 0x7F) + 1, 3);
-    double v, r;
-    ref_eval(f, c, pos[i] & 0x7FFFFFFF, nl, v, r);
-    if (lane == 0) {
-      a.v[i] = v; a.r[i] = r; a.l[i] = (uint8_t)nl;
-      if (a.ev) atomicAdd(a.ev + nl, 1u);
+  // Warps take eight entries at a time from a queue: the marked ones (a few percent, each worth
+  // thousands of terms) spread evenly whatever their places.
+  __shared__ unsigned queue;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) queue = 0;
+  const RefCache c = ref_cache_load(f);  // (barriers)
+  for (;;) {
+    unsigned q = 0;
+    if (lane == 0) q = atomicAdd(&queue, 8u);
+    const int64_t i0 = __shfl_sync(0xffffffffu, q, 0);
+    if (i0 >= n) break;
+    const uint8_t lv = lane < 8 && i0 + lane < n ? a.l[i0 + lane] : 0;
+    unsigned todo = __ballot_sync(0xffffffffu, lv & 0x80);
+    while (todo) {
+      const int e = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int l = __shfl_sync(0xffffffffu, (int)lv, e);
+      const int64_t i = i0 + e;
+      const int nl = to3 ? 3 : min((l & 0x7F) + 1, 3);
+      double v, r;
+      ref_eval(f, c, pos[i] & 0x7FFFFFFF, nl, v, r);
+      if (lane == 0) {
+        a.v[i] = v; a.r[i] = r; a.l[i] = (uint8_t)nl;
+        if (a.ev) atomicAdd(a.ev + nl, 1u);
+      }
     }
   }
   __syncthreads();
@@ -1120,29 +1320,24 @@ __device__ __noinline__ int64_t band_collect(Smem& s, const float* __restrict__ 
   const int64_t tile = (int64_t)PT * CITEMS;
   const float lof = f_up(lo), hif = f_dn(hi);
   for (int64_t t0 = 0; t0 < P; t0 += tile) {
-    const int64_t p0 = t0 + (int64_t)threadIdx.x * CITEMS;
+    const int64_t p0 = tile_pos(t0);
+    float v[CITEMS];
+#pragma unroll
+    for (int i = 0; i < CITEMS; ++i) v[i] = p0 + 32 * i < P ? src[p0 + 32 * i] : __int_as_float(0x7F800000);
     uint32_t bits = 0;
 #pragma unroll
-    for (int i = 0; i < CITEMS; ++i) {
-      if (p0 + i >= P) continue;
-      const float d = src[p0 + i];
-      if (d < lof) nb++;
-      else if (d <= hif) bits |= 1u << i;
+    for (int i = 0; i < CITEMS; ++i) {  // (Inf past the end: neither)
+      if (v[i] < lof) nb++;
+      else if (v[i] <= hif && p0 + 32 * i < P) bits |= 1u << i;
     }
-    uint32_t total;
-    const uint32_t off = block_excl_sum(s, (uint32_t)__popc(bits), total);
-    int64_t o = base + off;
-#pragma unroll
-    for (int i = 0; i < CITEMS; ++i)
-      if (bits >> i & 1u) out[o++] = (int32_t)(p0 + i);
-    base += total;
+    tile_append(s, bits, t0, out, base);
   }
   below = (int64_t)block_sum_u64(s, nb);
   return base;
 }
 
 // The exact top-k set of a refined map, given the k-th (value, index) key of its FP32 values:
-// fills `b` (list at `list`) and returns the near-ties at the boundary, or -1 when the bound
+// fills `b` (in shared memory; list at `list`) and returns the near-ties at the boundary, or -1 when the bound
 // failed (the FP32 k-th value lies outside the band: then the key is kept as it is).
 __device__ __noinline__ long long band_topk(Smem& s, unsigned long long* sbuf, const Ref& f,
                                const float* __restrict__ src, int64_t P, int64_t k, Key kv,
@@ -1150,32 +1345,41 @@ __device__ __noinline__ long long band_topk(Smem& s, unsigned long long* sbuf, c
                                uint32_t* v1, Band& b) {
   const double v = (double)__uint_as_float(kv.v);
   if (!(v < 1e300)) return -1;  // Inf boundary: the key is exact
-  // E0 valid up to Dc = v + 4E, E = E0 plus half the near-tie window
-  double E0 = tier0_bound(f, v * 1.001), E = 0.0;
-  for (int it = 0; it < 200; ++it) {
-    E = E0 + 0.51 * TIE_RTOL * (v + E0);
-    const double need = tier0_bound(f, v + 4.0 * E);
-    if (need <= E0) break;
-    E0 = fmax(need, 1.5 * E0);
+  // E0 valid up to Dc = v + 4E, E = E0 plus half the near-tie window. (One thread: the square roots
+  // of 1,024 would take the Float64 pipe 30 k cycles an iteration.)
+  __shared__ double bnd;
+  if (threadIdx.x == 0) {
+    double E0 = tier0_bound(f, v * 1.001), E = 0.0;
+    for (int it = 0; it < 200; ++it) {
+      E = E0 + 0.51 * TIE_RTOL * (v + E0);
+      const double need = tier0_bound(f, v + 4.0 * E);
+      if (need <= E0) break;
+      E0 = fmax(need, 1.5 * E0);
+    }
+    b.lo = v - 2.0 * E;
+    b.hi = v + 2.0 * E;
+    b.lof = f_up(b.lo);
+    b.hif = f_dn(b.hi);
+    b.list = list;
+    bnd = E;
   }
-  b.lo = v - 2.0 * E;
-  b.hi = v + 2.0 * E;
-  b.lof = f_up(b.lo);
-  b.hif = f_dn(b.hi);
-  b.list = list;
+  __syncthreads();
+  const double blo = v - 2.0 * bnd, bhi = v + 2.0 * bnd;
   int64_t below = 0;
-  b.n = band_collect(s, src, P, b.lo, b.hi, list, below);
+  const int64_t bn = band_collect(s, src, P, blo, bhi, list, below);
   const int64_t kk = k - below;
-  if (kk < 1 || kk > b.n) { b.n = 0; return -1; }
-  ref_init(f, list, b.n, a);
-  uint32_t* ord = const_cast<uint32_t*>(ref_sort(s, sbuf, b.n, a, k0, v0, k1, v1));
+  if (threadIdx.x == 0) b.n = kk < 1 || kk > bn ? 0 : bn;
+  __syncthreads();
+  if (kk < 1 || kk > bn) return -1;
+  ref_init(f, list, bn, a);
+  uint32_t* ord = const_cast<uint32_t*>(ref_sort(s, sbuf, bn, a, k0, v0, k1, v1));
   // The set is the first kk entries of the order once every entry on the left lies below every
   // entry on the right: raise only the entries that may cross the split, else (equal values
   // across it) put the whole band in exact (value, position) order.
   bool split = false;
   for (int round = 0; round < 4; ++round) {
     double mh = -1e308, ml = 1e308;
-    for (int64_t t = threadIdx.x; t < b.n; t += PT) {
+    for (int64_t t = threadIdx.x; t < bn; t += PT) {
       const uint32_t i = ord[t];
       if (t < kk) mh = fmax(mh, a.v[i] + a.r[i]);
       else ml = fmin(ml, a.v[i] - a.r[i]);
@@ -1184,16 +1388,16 @@ __device__ __noinline__ long long band_topk(Smem& s, unsigned long long* sbuf, c
     ml = block_min_f64(s, ml);
     if (mh < ml) { split = true; break; }
     int any = 0;
-    for (int64_t t = threadIdx.x; t < b.n; t += PT) {
+    for (int64_t t = threadIdx.x; t < bn; t += PT) {
       const uint32_t i = ord[t];
       const bool cross = t < kk ? a.v[i] + a.r[i] >= ml : a.v[i] - a.r[i] <= mh;
       if (cross && !ref_exact(a, i)) { ref_mark(a, i); any = 1; }
     }
     if (!__syncthreads_or(any)) break;
-    ref_raise(f, list, b.n, a, round >= 1);
-    ord = const_cast<uint32_t*>(ref_sort(s, sbuf, b.n, a, k0, v0, k1, v1));
+    ref_raise(f, list, bn, a, round >= 1);
+    ord = const_cast<uint32_t*>(ref_sort(s, sbuf, bn, a, k0, v0, k1, v1));
   }
-  if (!split) ref_resolve(s, f, list, b.n, ord, a);
+  if (!split) ref_resolve(s, f, list, bn, ord, a);
   for (int64_t t = threadIdx.x; t < kk; t += PT) list[ord[t]] |= (int32_t)0x80000000;
   __syncthreads();
   // the boundary: the largest (value, position) of the set
@@ -1237,11 +1441,11 @@ __device__ __noinline__ long long band_topk(Smem& s, unsigned long long* sbuf, c
       if (a.v[i] + a.r[i] >= mlo && !ref_exact(a, i)) ref_mark(a, i);
     }
     __syncthreads();
-    ref_raise(f, list, b.n, a, round >= 1);
+    ref_raise(f, list, bn, a, round >= 1);
   }
   if (bi < 0) bi = ord[kk - 1];  // not reached: level-3 values decide within 3 rounds
   __syncthreads();
-  return (long long)ref_count_ties(s, f, list, b.n, a, bi, true, 0.0);
+  return (long long)ref_count_ties(s, f, list, bn, a, bi, true, 0.0);
 }
 
 // Near-ties of an exact map against t (Float64 test of the oracle), counted over all positions.
@@ -1261,12 +1465,23 @@ __device__ __noinline__ unsigned long long count_near(Smem& s, const float* __re
 
 // Dense ranks (1-based) of a refined source over the candidates cand[0, n), written to rank[i];
 // returns the sum of (n - rank + 1). Ties of the Float64 distance share a rank.
-// `have`: the intervals of the candidates are in `a` already (the refined threshold pick).
+// `have`: the intervals of the candidates are in `a` already (the refined threshold pick); `lvl1`:
+// their level-1 values (nullable: evaluated here).
 __device__ __noinline__ unsigned long long dense_ranks_refined(Smem& s, unsigned long long* sbuf, const Ref& f,
                                                   const int32_t* cand, int64_t n, RefArr a,
-                                                  bool have, uint32_t* k0, uint32_t* v0,
-                                                  uint32_t* k1, uint32_t* v1, uint32_t* rank) {
-  if (!have) ref_init(f, cand, n, a);
+                                                  bool have, const float* lvl1, uint32_t* k0,
+                                                  uint32_t* v0, uint32_t* k1, uint32_t* v1,
+                                                  uint32_t* rank) {
+  if (!have && lvl1) {
+    for (int64_t i = threadIdx.x; i < n; i += PT) {
+      const double v = (double)lvl1[i];
+      a.v[i] = v; a.r[i] = ref_radius1(f, v); a.l[i] = 1;
+    }
+    if (a.ev && threadIdx.x == 0) atomicAdd(a.ev + 1, (unsigned)n);
+    __syncthreads();
+  } else if (!have) {
+    ref_init(f, cand, n, a);
+  }
   uint32_t* ord = const_cast<uint32_t*>(ref_sort(s, sbuf, n, a, k0, v0, k1, v1));
   ref_resolve(s, f, cand, n, ord, a);
   uint32_t carry = 0;
@@ -1328,16 +1543,58 @@ __device__ __noinline__ int64_t thr_refined(Smem& s, const Ref& f, const float* 
                                double m32, double tol, int32_t* cand, RefArr a,
                                unsigned long long& ties) {
   // every candidate, the minimum and every near-tie have D32 <= cut
-  double E0 = tier0_bound(f, (1.0 + tol) * m32 * 1.01), cut = 0.0;
-  for (int it = 0; it < 200; ++it) {
-    cut = (1.0 + tol) * (m32 + E0) * (1.0 + 1.01 * TIE_RTOL) + E0;
-    const double need = tier0_bound(f, cut + 2.0 * E0);
-    if (need <= E0) break;
-    E0 = fmax(need, 1.5 * E0);
+  __shared__ double scut;
+  if (threadIdx.x == 0) {
+    double E0 = tier0_bound(f, (1.0 + tol) * m32 * 1.01), c = 0.0;
+    for (int it = 0; it < 200; ++it) {
+      c = (1.0 + tol) * (m32 + E0) * (1.0 + 1.01 * TIE_RTOL) + E0;
+      const double need = tier0_bound(f, c + 2.0 * E0);
+      if (need <= E0) break;
+      E0 = fmax(need, 1.5 * E0);
+    }
+    scut = c;
   }
+  __syncthreads();
+  const double cut = scut;
   int64_t below = 0;
   const int64_t n0 = band_collect(s, D, P, -1.0, cut, cand, below);
   ref_init(f, cand, n0, a);
+  // First with the minimum's interval instead of its value: entries that may hold the minimum are
+  // raised to level 2 (an interval of 1e-13), and the threshold is an interval. Where that decides
+  // every membership and near-tie the exact minimum is not needed; its level-3 sum is a chain of K
+  // Float64 additions, 0.2 M cycles at K = 4,300 with one warp at work.
+  for (int round = 0; round < 3; ++round) {
+    double up = 1e308;
+    for (int64_t i = threadIdx.x; i < n0; i += PT) up = fmin(up, a.v[i] + a.r[i]);
+    const double mh = block_min_f64(s, up);
+    int any = 0;
+    for (int64_t i = threadIdx.x; i < n0; i += PT)
+      if (a.v[i] - a.r[i] <= mh && (a.l[i] & 0x7F) < 2) { ref_mark(a, (uint32_t)i); any = 1; }
+    if (__syncthreads_or(any)) {
+      ref_raise(f, cand, n0, a, false);
+      continue;
+    }
+    double dn = 1e308;
+    for (int64_t i = threadIdx.x; i < n0; i += PT) dn = fmin(dn, a.v[i] - a.r[i]);
+    const double ml = block_min_f64(s, dn);
+    // (1 + tol) * min, with slack for its two roundings and those made here
+    const double tv = (1.0 + tol) * 0.5 * (ml + mh);
+    const double tr = (1.0 + tol) * 0.5 * (mh - ml) * (1.0 + 1e-9) + tv * 16.0 * RU64;
+    if (!(ml > 0.0) || !(tv - tr > 0.0) || !(tv < 1e300)) break;
+    unsigned long long cnt = 0;
+    int und = 0;
+    for (int64_t i = threadIdx.x; i < n0; i += PT) {
+      const double v = a.v[i], r = a.r[i];
+      const int t = ref_tie(a, (uint32_t)i, tv, tr, false);
+      if (t > 0) cnt++;
+      const bool in = v + r <= tv - tr, out = v - r > tv + tr;
+      if (t < 0 || !(in || out)) und = 1;
+      a.link[i] = in ? 1 : 0;
+    }
+    if (__syncthreads_or(und)) break;
+    ties += block_sum_u64(s, cnt);
+    return ref_filter(s, cand, n0, a);
+  }
   // the exact minimum: raise every entry whose interval reaches below the smallest upper bound
   double mhi = 0.0;
   for (int round = 0; round < 8; ++round) {
@@ -1379,7 +1636,8 @@ __device__ __noinline__ int64_t thr_refined(Smem& s, const Ref& f, const float* 
 // map's error bound at 0; otherwise every mask value is compared with its window.
 __device__ __noinline__ bool all_zero_refined(const Ref& f, const float* __restrict__ D, int64_t P,
                                  unsigned mxbits) {
-  if ((double)__uint_as_float(mxbits) > tier0_bound(f, 0.0)) return false;
+  if (__syncthreads_or(threadIdx.x == 0 && (double)__uint_as_float(mxbits) > tier0_bound(f, 0.0)))
+    return false;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t step = (int64_t)NW * 8;
   for (int64_t p0 = 0; p0 < P; p0 += step) {
@@ -1458,7 +1716,11 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
   const long long t0 = prof ? clock64() : 0;
   int64_t n;
   bool have0 = false;  // D's candidate intervals are in ra (refined threshold pick)
-  if (naux == 0) {
+  if (a.phase == 2) {
+    n = a.ncand[b];
+    if (n <= 1) return;  // drawn, or failed, in phase 1
+    have0 = naux == 0 && can_ref && ref_on(tk.x0) && __uint_as_float(mm[0]) < __int_as_float(0x7F800000);
+  } else if (naux == 0) {
     const float mn = __uint_as_float(mm[0]);
     if (can_ref && ref_on(tk.x0) && mn < __int_as_float(0x7F800000)) {
       const Ref f0 = make_ref(tk.x0, r, a.dx, a.dxy);
@@ -1472,7 +1734,11 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
     }
   } else {
     if (a.npat <= 0) {
-      if (threadIdx.x == 0) { iq_dev_fail(a.status, IQ_ERR_NOPATTERN); a.rind[b] = -1; }
+      if (threadIdx.x == 0) {
+        iq_dev_fail(a.status, IQ_ERR_NOPATTERN);
+        a.rind[b] = -1;
+        if (a.phase == 1) a.ncand[b] = 0;
+      }
       return;
     }
     const bool ref0 = can_ref && ref_on(tk.x0);
@@ -1591,8 +1857,22 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
           }
         }
       }
-      // the compaction counts: an empty intersection moves on to the next softdbsize
-      n = compact(s, pr, P, cand);
+      // The compaction counts: an empty intersection moves on to the next softdbsize. Where a shared
+      // source's set is listed (1% of the positions in the first round), only those are tested.
+      int lead = -1;
+      int64_t nlead = 0;
+#pragma unroll
+      for (int j = 0; j < NAUX; ++j) {
+        if (j >= naux || !tk.memb || tiesA[j] < 0 || !tk.aux_pb[j] || q >= tk.nkeys || allzero) continue;
+        const PreBand& pb = tk.aux_pb[j][q];
+        if (pb.ok == 1 && pb.nm >= 0 && (lead < 0 || pb.nm < nlead)) { lead = j; nlead = pb.nm; }
+      }
+      if (lead >= 0) {
+        const int32_t* ml = tk.memb + tk.aux_pb[lead][q].off / tk.pb_cap * IQ_MEMB_CAP;
+        n = compact_list<NAUX>(s, pr, lead, ml, nlead, cand);
+      } else {
+        n = compact(s, pr, P, cand);
+      }
     }
     if (a.stats && threadIdx.x == 0) atomicAdd(a.stats + ST_PICK_ITERS, (unsigned long long)q);
     // near-ties at D's boundary and at each auxiliary boundary of the final round; exact maps
@@ -1617,15 +1897,21 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
       }
     }
   }
-  if (a.ties && threadIdx.x == 0 && ties) atomicAdd(a.ties, ties);
-  if (n <= 0) {
-    if (threadIdx.x == 0) { iq_dev_fail(a.status, IQ_ERR_NOPATTERN); a.rind[b] = -1; }
-    return;
-  }
-  if (a.ncand && threadIdx.x == 0) a.ncand[b] = n;
-  if (a.stats && threadIdx.x == 0) {
-    atomicAdd(a.stats + ST_PICK_CAND, (unsigned long long)n);
-    atomicAdd(a.stats + ST_PICK_CTAS, 1ull);
+  if (a.phase != 2) {
+    if (a.ties && threadIdx.x == 0 && ties) atomicAdd(a.ties, ties);
+    if (n <= 0) {
+      if (threadIdx.x == 0) {
+        iq_dev_fail(a.status, IQ_ERR_NOPATTERN);
+        a.rind[b] = -1;
+        if (a.phase == 1) a.ncand[b] = 0;
+      }
+      return;
+    }
+    if (a.ncand && threadIdx.x == 0) a.ncand[b] = n;
+    if (a.stats && threadIdx.x == 0) {
+      atomicAdd(a.stats + ST_PICK_CAND, (unsigned long long)n);
+      atomicAdd(a.stats + ST_PICK_CTAS, 1ull);
+    }
   }
   const long long t1 = prof ? clock64() : 0;
   if (prof) atomicAdd(a.stats + ST_PICK_TSEL, (unsigned long long)(t1 - t0));
@@ -1633,6 +1919,13 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
   // ---- tau model weights ----
   if (n == 1) {
     if (threadIdx.x == 0) { w[0] = 1.0; a.rind[b] = cand[0]; }
+    return;
+  }
+  if (a.phase == 1) {
+    if (prof)
+      atomicAdd(a.stats + ST_PICK_TBAND, (unsigned long long)tband);
+    if (a.stats && threadIdx.x == 0)
+      for (int l = 1; l < 4; ++l) atomicAdd(a.stats + ST_PICK_EV1 + l - 1, (unsigned long long)evc[l]);
     return;
   }
   const double dn = (double)n;
@@ -1647,7 +1940,9 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
     unsigned long long S;
     if (can_ref && ref_on(xs)) {
       const Ref f = make_ref(xs, r, a.dx, a.dxy);
-      S = dense_ranks_refined(s, sbuf, f, cand, n, ra, j == 0 && have0, k0, v0, k1, v1, rankbuf);
+      const float* l1 = a.phase == 2 && n <= IQ_RANK_CAP && ref_cacheable(f)
+                            ? a.lvl1 + ((int64_t)b * a.nsrc + j) * IQ_RANK_CAP : nullptr;
+      S = dense_ranks_refined(s, sbuf, f, cand, n, ra, j == 0 && have0, l1, k0, v0, k1, v1, rankbuf);
     } else {
       S = dense_ranks(s, sbuf, src, cand, n, k0, v0, k1, v1, rankbuf);
     }
@@ -1697,6 +1992,38 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
     a.rind[b] = cand[pick];
     if (prof) atomicAdd(a.stats + ST_PICK_TDRAW, (unsigned long long)(clock64() - t2));
   }
+}
+
+// Level-1 distances of every pick's candidates to every refined source of its task, between the
+// two phases of pick_kernel: a CTA evaluates EV_CH candidates of one (pick, source). A pick's ~700
+// candidates x 2-3 sources x ~5,500 terms dominated its single CTA (one of 16-80 in a launch, on as
+// many of the 152 SMs); here they spread over the chip, eight candidates per warp at a time.
+constexpr int EV_NT = 256;
+constexpr int EV_BATCH = 8;
+constexpr int EV_CH = EV_NT / 32 * EV_BATCH;
+
+__global__ void __launch_bounds__(EV_NT) rank_eval_kernel(const PickArgs a, int cap) {
+  const int b = blockIdx.x / a.nsrc, j = blockIdx.x - b * a.nsrc;
+  const PickTask& tk = a.tasks ? a.tasks[b / a.nreal] : a.t0;
+  const int r = b % a.nreal;
+  if (tk.pre || tk.naux == 0 || j > tk.naux) return;
+  const int64_t n = a.ncand[b], i0 = (int64_t)blockIdx.y * EV_CH;
+  if (n <= 1 || n > IQ_RANK_CAP || i0 >= n) return;
+  const ExactSrc& xs = j == 0 ? tk.x0 : tk.xa[j - 1];
+  if (!ref_on(xs)) return;
+  const Ref f = make_ref(xs, r, a.dx, a.dxy);
+  if (!ref_cacheable(f) || f.K > cap) return;
+  const RefCache c = ref_cache_load(f, cap);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t i = i0 + warp * EV_BATCH;
+  if (i >= n) return;
+  const int m = (int)min((int64_t)EV_BATCH, n - i);
+  float acc[EV_BATCH];
+  ref_eval1_batch<EV_BATCH>(f, c, a.cand + (int64_t)b * a.P + i, m, acc);
+  float x = acc[0];
+#pragma unroll
+  for (int e = 1; e < EV_BATCH; ++e) x = lane == e ? acc[e] : x;
+  if (lane < m) a.lvl1[((int64_t)b * a.nsrc + j) * IQ_RANK_CAP + i + lane] = x;
 }
 
 // One CTA per (map, sequence step): the key of the k-th smallest (value, index) of the map, as
@@ -1766,17 +2093,38 @@ int iq_launch_pick(iq_ctx* ctx, const PickLaunch& L) {
   a.stats = L.stats;
   const int naux = L.tasks ? L.naux_max : L.t0.naux;
   const int nblocks = L.ntask * L.nreal;
+  auto launch = [&]() {
+    switch (naux) {
+      case 0: return launch_pick_t<0>(a, nblocks, ctx->stream);
+      case 1: return launch_pick_t<1>(a, nblocks, ctx->stream);
+      case 2: return launch_pick_t<2>(a, nblocks, ctx->stream);
+      case 3: return launch_pick_t<3>(a, nblocks, ctx->stream);
+      case 4: return launch_pick_t<4>(a, nblocks, ctx->stream);
+      case 5: return launch_pick_t<5>(a, nblocks, ctx->stream);
+      case 6: return launch_pick_t<6>(a, nblocks, ctx->stream);
+      default: return launch_pick_t<7>(a, nblocks, ctx->stream);
+    }
+  };
+  // With auxiliary sources and maps that need the re-rank: selection, level-1 distances of the
+  // candidates, weights. (Without auxiliary sources the threshold pick evaluates its candidates
+  // itself, to find the threshold.)
+  const bool split = L.lvl1 && L.rv && L.ncand && naux > 0 && L.maxK > 0 && L.maxK <= REF_CACHE;
+  a.phase = split ? 1 : 0;
+  a.lvl1 = L.lvl1;
+  a.nsrc = naux + 1;
   iq_timer_start(ctx, "pick");
-  cudaError_t e;
-  switch (naux) {
-    case 0: e = launch_pick_t<0>(a, nblocks, ctx->stream); break;
-    case 1: e = launch_pick_t<1>(a, nblocks, ctx->stream); break;
-    case 2: e = launch_pick_t<2>(a, nblocks, ctx->stream); break;
-    case 3: e = launch_pick_t<3>(a, nblocks, ctx->stream); break;
-    case 4: e = launch_pick_t<4>(a, nblocks, ctx->stream); break;
-    case 5: e = launch_pick_t<5>(a, nblocks, ctx->stream); break;
-    case 6: e = launch_pick_t<6>(a, nblocks, ctx->stream); break;
-    default: e = launch_pick_t<7>(a, nblocks, ctx->stream); break;
+  cudaError_t e = launch();
+  if (split && e == cudaSuccess) {
+    const size_t sm = (size_t)8 * L.maxK;
+    e = cudaFuncSetAttribute(rank_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e == cudaSuccess) {
+      rank_eval_kernel<<<dim3((unsigned)(nblocks * a.nsrc), IQ_RANK_CAP / EV_CH), EV_NT, sm, ctx->stream>>>(
+          a, L.maxK);
+      e = cudaGetLastError();
+      a.phase = 2;
+      if (e == cudaSuccess) e = launch();
+      iq_count(ctx, 2);
+    }
   }
   iq_timer_stop(ctx, "pick", 4.0 * (double)L.P * (double)(1 + naux) * (double)nblocks);
   iq_count(ctx);
@@ -1815,6 +2163,7 @@ struct BandArgs {
   PreBand* out;
   int32_t* pool;
   int64_t cap;
+  int32_t* memb;      // the sets themselves, IQ_MEMB_CAP entries per selection (nullable)
   int keys_exact;     // exact maps get their key (ok = 2)
   // per-CTA scratch, P entries each
   double* rv;
@@ -1849,7 +2198,10 @@ __global__ void __launch_bounds__(PT) select_bands_kernel(const BandArgs a) {
   }
   int ok = 0;
   long long ties = 0;
-  Band band{};
+  int64_t nm = -1;
+  __shared__ Band band;
+  if (threadIdx.x == 0) band = Band{};
+  __syncthreads();
   if (k > 0 && k < P && ref_on(a.srcs[m])) {
     const Ref f = make_ref(a.srcs[m], 0, a.dx, a.dxy);
     RefArr ra;
@@ -1865,6 +2217,11 @@ __global__ void __launch_bounds__(PT) select_bands_kernel(const BandArgs a) {
       ok = 1;
       int32_t* dst = a.pool + (m * a.nq + q) * a.cap;
       for (int64_t i = threadIdx.x; i < band.n; i += PT) dst[i] = list[i];
+      // the whole set, while it fits: the picks then test its positions instead of scanning the map
+      if (a.memb && k <= IQ_MEMB_CAP) {
+        BandPred bp{src, &band};
+        nm = compact(s, bp, P, a.memb + (m * a.nq + q) * (int64_t)IQ_MEMB_CAP);
+      }
     }
   }
   if (!ref_on(a.srcs[m]) && a.keys_exact) ok = 2;  // an exact map: its key decides
@@ -1876,6 +2233,7 @@ __global__ void __launch_bounds__(PT) select_bands_kernel(const BandArgs a) {
     o->key = ((unsigned long long)key.v << 32) | key.i;
     o->ties = ok ? ties : 0;
     o->ok = ok;
+    o->nm = nm;
   }
 }
 
@@ -1884,7 +2242,7 @@ __global__ void __launch_bounds__(PT) select_bands_kernel(const BandArgs a) {
 int iq_launch_select_bands(iq_ctx* ctx, const float* maps, const unsigned* mm,
                            const ExactSrc* srcs, int64_t nmaps, int64_t P, int64_t dx,
                            int64_t dxy, const int64_t* seq, int nq, PreBand* out, int32_t* pool,
-                           int64_t cap, int keys_exact) {
+                           int64_t cap, int keys_exact, int32_t* memb) {
   if (nmaps <= 0 || nq <= 0) return IQ_OK;
   if (nq > IQ_PRE_KEYS) return iq_set_error(IQ_ERR_ARG, "too many precomputed selections");
   // per-CTA scratch for a batch of CTAs (38 bytes per position each)
@@ -1911,7 +2269,7 @@ int iq_launch_select_bands(iq_ctx* ctx, const float* maps, const unsigned* mm,
     a.maps = maps; a.mm = mm; a.srcs = srcs; a.m0 = m0; a.nmaps = std::min(mper, nmaps - m0);
     a.P = P; a.dx = dx; a.dxy = dxy; a.nq = nq;
     for (int q = 0; q < IQ_PRE_KEYS; ++q) a.seq[q] = q < nq ? seq[q] : 0;
-    a.out = out; a.pool = pool; a.cap = cap; a.keys_exact = keys_exact;
+    a.out = out; a.pool = pool; a.cap = cap; a.keys_exact = keys_exact; a.memb = memb;
     a.rv = rv; a.rr = rr; a.rl = rl; a.list = list; a.k0 = k0; a.v0 = v0; a.k1 = k1; a.v1 = v1;
     iq_timer_start(ctx, "pick");
     select_bands_kernel<<<(unsigned)(a.nmaps * nq), PT, DYN_BYTES, ctx->stream>>>(a);

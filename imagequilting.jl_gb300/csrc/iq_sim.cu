@@ -497,7 +497,10 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   for (int64_t t = 0; t < g.ntot && !need_ref; ++t)
     if (!tile_hard[t].empty())
       need_ref = iq_map_kappa(ctx->ti_stats, hard_stats, (int64_t)tile_hard[t].size(), 0) > 0.0;
-  const int64_t per_step = (int64_t)R * P * (4 + 4 + 16 + 16 + (need_ref ? 18 : 0)) + P * 4 +
+  // sources of a pick beyond its distance: soft variables, and the overlap of a data tile
+  const int naux_most = nsoft + (nh > 0 ? 1 : 0);
+  const int64_t lvl1_per = need_ref && naux_most > 0 ? (int64_t)R * (naux_most + 1) * IQ_RANK_CAP : 0;
+  const int64_t per_step = (int64_t)R * P * (4 + 4 + 16 + 16 + (need_ref ? 18 : 0)) + lvl1_per * 4 + P * 4 +
                            T * (rpad + 1) * 4 + (int64_t)R * 6 * (slabmax + cutscr_per) + 4096;
   size_t freeb = 0, totalb = 0;
   cudaMemGetInfo(&freeb, &totalb);
@@ -571,6 +574,8 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   double* d_rv = need_ref ? (double*)iq_scratch(ctx, S_PICK_RV, sizeof(double) * pk) : nullptr;
   double* d_rr = need_ref ? (double*)iq_scratch(ctx, S_PICK_RR, sizeof(double) * pk) : nullptr;
   uint8_t* d_rl = need_ref ? (uint8_t*)iq_scratch(ctx, S_PICK_RL, 2 * pk) : nullptr;
+  float* d_lvl1 = lvl1_per ? (float*)iq_scratch(ctx, S_LVL1, sizeof(float) * lvl1_per * cmax) : nullptr;
+  if (lvl1_per && !d_lvl1) return IQ_ERR_ALLOC;
   int64_t* d_rind = (int64_t*)iq_scratch(ctx, S_RIND, sizeof(int64_t) * R * cmax);
   int64_t* d_ncand = (int64_t*)iq_scratch(ctx, S_NCAND, sizeof(int64_t) * R * cmax);
   uint8_t* d_cutbuf = (uint8_t*)iq_scratch(ctx, S_CUTBUF, (size_t)R * cmax * 6 * slabmax);
@@ -953,6 +958,7 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   unsigned long long* d_softkeys = nullptr;
   PreBand* d_pb = nullptr;      // refined selections of the soft maps (maps with an error bound)
   int32_t* d_pbpool = nullptr;
+  int32_t* d_memb = nullptr;
   const int64_t pb_cap = 8192;  // listed band positions per selection
   if (nsoft > 0 && npat > 0 && nkeys > 0 && nslot > 0) {
     d_softkeys = (unsigned long long*)iq_scratch(ctx, S_SOFTKEYS,
@@ -986,11 +992,14 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
       ExactSrc* d_xs = (ExactSrc*)iq_scratch(ctx, S_PB_SRC, sizeof(ExactSrc) * xs.size());
       d_pb = (PreBand*)iq_scratch(ctx, S_PB_OUT, sizeof(PreBand) * nslot * nsoft * nkeys);
       d_pbpool = (int32_t*)iq_scratch(ctx, S_PB_POOL, sizeof(int32_t) * nslot * nsoft * nkeys * pb_cap);
-      if (!d_xs || !d_pb || !d_pbpool) return IQ_ERR_ALLOC;
+      // the selections' sets themselves, for the steps whose size IQ_MEMB_CAP holds
+      if (seqn[0] <= IQ_MEMB_CAP)
+        d_memb = (int32_t*)iq_scratch(ctx, S_PB_MEMB, sizeof(int32_t) * nslot * nsoft * nkeys * IQ_MEMB_CAP);
+      if (!d_xs || !d_pb || !d_pbpool || (seqn[0] <= IQ_MEMB_CAP && !d_memb)) return IQ_ERR_ALLOC;
       IQ_CUDA_OK(cudaMemcpyAsync(d_xs, xs.data(), sizeof(ExactSrc) * xs.size(),
                                  cudaMemcpyHostToDevice, st));
       RET_IF(iq_launch_select_bands(ctx, d_soft, d_softmm, d_xs, nslot * nsoft, P, distD.x,
-                                    distD.x * distD.y, seqn, nkeys, d_pb, d_pbpool, pb_cap));
+                                    distD.x * distD.y, seqn, nkeys, d_pb, d_pbpool, pb_cap, 0, d_memb));
       IQ_CUDA_OK(cudaStreamSynchronize(st));  // `xs` is a host vector
     }
   }
@@ -1140,6 +1149,8 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
             if (d_pb) {  // refined selections shared by all realizations
               q.aux_pb[na] = d_pb + slot * nkeys;
               q.pb_pool = d_pbpool;
+              q.pb_cap = pb_cap;
+              q.memb = d_memb;
               q.nkeys = nkeys;
             }
             // the auxiliary TI against the padded auxiliary grid at the tile, full tile
@@ -1312,6 +1323,9 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
         L.rv = d_rv ? d_rv + po : nullptr; L.rr = d_rr ? d_rr + po : nullptr;
         L.rl = d_rl ? d_rl + 2 * po : nullptr;
         L.dx = distD.x; L.dxy = distD.x * distD.y;
+        L.lvl1 = d_lvl1 ? d_lvl1 + grp_rind(grp) * (naux_most + 1) * IQ_RANK_CAP : nullptr;
+        L.maxK = (int)(nsoft > 0 ? T : maxK);  // (hard masks hold at most a tile's offsets too)
+        if (chard[c]) L.maxK = (int)T;
         L.ties = ctx->d_ties;
         L.rind = rind; L.ncand = d_ncand + grp_rind(grp); L.status = ctx->d_status;
         L.stats = ctx->prof ? ctx->d_stats : nullptr;
