@@ -13,7 +13,7 @@ import time
 # the library's defaults (include/iqgpu.h) and the candidate values tried for each knob
 DEFAULTS = {
     "graphcut.threads": 512,
-    "graphcut.gr_period": 32,
+    "graphcut.gr_period": 16,
     "sim.level_chunk": 64,
     "sim.streams": 1,
 }

@@ -666,6 +666,7 @@ extern "C" int iq_graphcut(iq_ctx* ctx, const float* A, const float* B, int32_t 
   L.nreal = 1; L.ntask = 1;
   L.A = dA; L.B = dA + n;
   L.out = dout; L.slabmax = n;
+  L.intmax = n / size[dim] * std::max<int64_t>(size[dim] - 2, 0);
   L.scratch = scr; L.scratch_per_cta = (int64_t)iq_cut_scratch_bytes(n);
   L.status = ctx->d_status;
   L.stats = ctx->prof ? ctx->d_stats : nullptr;

@@ -78,7 +78,7 @@ struct iq_ctx {
   int64_t prof_mma_launches = 0;
   double prof_tc_cols = 0;      // columns (templates, with padding) of those launches
   // tuning knobs (iq_set_option)
-  int cut_gr_period = 32;
+  int cut_gr_period = 16;
   int cut_threads = 512;
   int64_t level_chunk = 64;     // most tiles of one dependency level launched together
   int corr_variant = 1;         // launch shape of the 16-template correlation
@@ -495,12 +495,13 @@ struct CutLaunch {
   const float* A = nullptr; const float* B = nullptr;
   uint8_t* out = nullptr;      // (ntask * nreal) x 6 x slabmax bytes: keep-old flags
   int64_t slabmax = 0;
+  int64_t intmax = -1;         // most interior voxels of a slab (< 0: slabmax)
   void* scratch = nullptr;     // global scratch for slabs too large for shared memory
   int64_t scratch_per_cta = 0;
   int* status = nullptr;
   int round_cap = 1 << 18;
   unsigned long long* stats = nullptr;  // profiling counters (nullable)
-  int gr_period = 32;          // rounds between global relabels
+  int gr_period = 16;          // rounds between global relabels
   int threads = 512;           // threads per CTA
 };
 int iq_launch_cut(iq_ctx* ctx, const CutLaunch& L);

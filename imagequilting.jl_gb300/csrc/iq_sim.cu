@@ -486,12 +486,15 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   const int rpad = ((R + rt - 1) / rt) * rt;
   int64_t slabmax = 1;
   for (int d = 0; d < N; ++d) slabmax = std::max<int64_t>(slabmax, T / g.tile[d] * g.ovl[d]);
+  int64_t cutint = 0;  // most voxels of a slab between its source and sink slices
+  for (int d = 0; d < N; ++d)
+    cutint = std::max<int64_t>(cutint, T / g.tile[d] * std::max<int64_t>(g.ovl[d] - 2, 0));
   int64_t cutscr_per = 0;
   {
     int dev = 0, lim = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    lim -= 1024;  // the cut kernel's static shared memory
+    lim -= 6144;  // the cut kernel's static shared memory
     if ((int64_t)iq_cut_scratch_bytes(slabmax) > lim) cutscr_per = (int64_t)iq_cut_scratch_bytes(slabmax);
   }
   for (int64_t t = 0; t < g.ntot && !need_ref; ++t)
@@ -1338,7 +1341,7 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
           K.nreal = Rg; K.ntask = m; K.nslab_max = cslab[c]; K.tasks = d_st + k0;
           K.sim = sim; K.sim_dims = padD; K.sim_rstride = padvol;
           K.ti = ctx->d_ti; K.ti_dims = ctx->ti; K.dist_dims = distD; K.rind = rind;
-          K.out = cutbuf; K.slabmax = slabmax;
+          K.out = cutbuf; K.slabmax = slabmax; K.intmax = cutint;
           K.scratch = d_cutscr ? (char*)d_cutscr + grp_rind(grp) * 6 * cutscr_per : nullptr;
           K.scratch_per_cta = cutscr_per;
           K.status = ctx->d_status;
