@@ -128,7 +128,7 @@ enum IqSlot {
   S_PBH_OUT, S_PBH_POOL, S_PBH_SRC,
   S_LP_T, S_LP_NT, S_LP_TAU, S_LP_LIST, S_LP_CNT, S_LP_DL, S_LP_COLS, S_LP_TSRC, S_LP_TBOX,
   S_LP_RIND, S_LP_NCAND, S_LP_D, S_LP_BITS, S_LP_ITEMS, S_LP_X, S_LP_E, S_LP_GE, S_LP_FEAT, S_LP_BH1, S_LP_BGZ1, S_LP_BH2, S_LP_DENSE, S_LP_QUAD,
-  S_TZ_IMG, S_TZ_A2, S_TZ_PLAN, S_TZ_B, S_TZ_SIMG, S_TZ_SA2, S_PREDRAW, S_LP_W, S_LVL1, S_PB_MEMB,
+  S_TZ_IMG, S_TZ_A2, S_TZ_PLAN, S_TZ_B, S_TZ_SIMG, S_TZ_SA2, S_PREDRAW, S_LP_W, S_LVL1, S_PB_MEMB, S_LP_BITS2, S_LP_MIN,
   S_COUNT
 };
 
@@ -618,16 +618,16 @@ struct LpColumn {
   int32_t tdim[3];     // tile extents
   int32_t pad2_;
 };
-// The training image as the exact sums of the proposal read it. Plane form (codes 0..3, tiles
-// of x extent <= 32): 2-bit codes in tiles of 32 (x) by 16 (y) voxels, one 64-bit word per tile
-// row (bits 0-31: the low bit of each voxel's code, bits 32-63: the high bit), tiles ordered
-// (x, y, z) with one extra column of zero tiles past the last in x; a window row of 32 voxels
-// is then two words and a funnel shift. Byte form otherwise (quads).
+// The training image as the exact sums of the proposal read it. Plane form (codes 0..3, tiles of x
+// extent <= 32): bit planes of 32 voxels in x, entry (z * ntx + tx) * ny + y holding the low-bit words
+// of tiles tx and tx + 1 and their high-bit words (tiles past the image are zero), so that a window row
+// of 32 voxels is one 16-byte load and two funnel shifts, and the rows of one window are at fixed
+// offsets from its first. Byte form otherwise (quads).
 struct LpImg {
   const uint8_t* b8;               // bytes, 16 bytes of padding past the end
-  const unsigned long long* b2;    // plane form (nullptr: byte form)
+  const uint4* p2;                 // plane form (nullptr: byte form)
   int64_t isx, isxy;               // byte image strides
-  int64_t ntx, nty;                // plane tiles per row (x, including the zero column), per slice (y)
+  int32_t ntx, ny;                 // plane tiles per row, rows per slice
 };
 #ifdef __CUDACC__
 // Comparisons of FP32 map values with Float64 bounds, made in FP32 (the FP64 pipe of this part
@@ -694,8 +694,8 @@ __device__ __forceinline__ uint32_t iq_quad_ssd(const uint8_t* base, const uint4
                                                 const Bound& bound) {
   const int lane = threadIdx.x & 31;
   uint32_t acc = 0;
-  // Batches of 8 x 32 quads while all lanes have one, so that the trip count and the exit (the
-  // bound as lane 0 read it) are the warp's: the loop holds full-warp shuffles.
+  // Batches of 8 x 32 quads while all lanes have one, so that the trip count and the exit are
+  // the warp's: the loop holds full-warp reductions.
   int i = lane;
   for (; i - lane + 8 * 32 <= nq; i += 8 * 32) {
     uint32_t v[8];
@@ -707,28 +707,24 @@ __device__ __forceinline__ uint32_t iq_quad_ssd(const uint8_t* base, const uint4
       const uint32_t d = __vabsdiffu4(v[u], e.y) & e.z;
       acc = __dp4a(d, d, acc);
     }
-    uint32_t part = acc;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if ((float)part > __shfl_sync(0xffffffffu, bound(), 0)) return 0xFFFFFFFFu;
+    const uint32_t part = __reduce_add_sync(0xffffffffu, acc);
+    if (__any_sync(0xffffffffu, (float)part > bound())) return 0xFFFFFFFFu;
   }
   for (; i < nq; i += 32) {
     const uint4 e = q[i];
     const uint32_t d = __vabsdiffu4(iq_ld4(base + (int32_t)e.x), e.y) & e.z;
     acc = __dp4a(d, d, acc);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  return acc;
+  return __reduce_add_sync(0xffffffffu, acc);
 }
 
 // Plane form: stage a column's template rows (ty, tz) of the tile in shared memory as
-// (low-bit plane, high-bit plane, mask bits, ty | tz << 16): the rows outside the box's (y, z)
+// (low-bit plane, high-bit plane, mask bits, plane offset of the row): the rows outside the box's (y, z)
 // range (every x in the mask) first, then the rows through the box (x outside it only; left out
 // when the box spans every x), so that partial sums grow fast for the early exit. Returns the
 // number of rows staged, or -1 (for the whole block) when a template value in the mask is not
 // one of 0, 1, 2, 3.
-__device__ inline int iq_stage_rows(const LpColumn& col, uint4* rows) {
+__device__ inline int iq_stage_rows(const LpImg& im, const LpColumn& col, uint4* rows) {
   const int R = col.tdim[1] * col.tdim[2];
   const int* lh = col.lohi;
   const int iy0 = max(lh[1], 0), iy1 = max(min(lh[4], col.tdim[1]), iy0);
@@ -754,96 +750,127 @@ __device__ inline int iq_stage_rows(const LpColumn& col, uint4* rows) {
       p0 |= (c & 1u) << x;
       p1 |= (c >> 1) << x;
     }
-    rows[rin ? nouter + before : r - before] = make_uint4(p0, p1, m, (uint32_t)ty | ((uint32_t)tz << 16));
+    rows[rin ? nouter + before : r - before] = 
+        make_uint4(p0, p1, m, (uint32_t)tz * (uint32_t)im.ntx * (uint32_t)im.ny + (uint32_t)ty);
   }
   return __syncthreads_or(bad) ? -1 : (inner_empty ? nouter : R);
 }
 
-// Sum of (a - b)^2 over one row of 32 codes given as bit planes (a0, a1), (b0, b1) and mask m:
-// with u = a1 - b1, v = a0 - b0 in {-1, 0, 1}, (a - b)^2 = 4u^2 + 4uv + v^2, u^2 = a1 ^ b1,
-// v^2 = a0 ^ b0, and where both are nonzero uv = +1 exactly when a1 == a0 (then u and v have
-// the sign of a1 - b1 = a0 - b0), so sum 4uv = 4 popc(y) - 8 popc(y & (a1 ^ a0)) with
-// y = (a1 ^ b1) & (a0 ^ b0).
+// Sum of (a - b)^2 over one row of 32 codes given as bit planes (a0, a1), (b0, b1) and mask m. The
+// difference is odd where a0 != b0, 2 in magnitude where only the high bits differ, and 3 where both
+// differ and a1 == a0 (codes 0 and 3; 1 and 2 have a1 != a0): squares 1, 4 and 1 + 8, three counts
+// (POPC runs at a quarter of the integer rate and bounds the sums).
 __device__ __forceinline__ int iq_row_ssd(uint32_t a0, uint32_t a1, const uint4& t) {
-  const uint32_t m = t.z;
-  const uint32_t x1 = (a1 ^ t.y) & m, x0 = (a0 ^ t.x) & m;
-  const uint32_t y = x1 & x0;
-  return __popc(x0) + 4 * (__popc(x1) + __popc(y)) - 8 * __popc(y & (a1 ^ a0));
+  const uint32_t x1 = (a1 ^ t.y) & t.z, x0 = (a0 ^ t.x) & t.z;
+  const uint32_t d3 = x1 & x0 & ~(a1 ^ a0);
+  return __popc(x0) + 4 * __popc(x1 & ~x0) + 8 * __popc(d3);
 }
 
-// Warp-collective, plane form: sum over the R staged rows for the window at (x0, y0, z0), with
-// the early exit of iq_quad_ssd.
-// (The plane image has fewer than 2^31 words: 32-bit index arithmetic.)
+// Warp-collective, plane form: sum over the R staged rows for the window whose first row is entry
+// `base`, bit `s`, with the early exit of iq_quad_ssd.
 template <typename Bound>
-__device__ __forceinline__ uint32_t iq_plane_ssd(const LpImg& im, int64_t x0, int64_t y0,
-                                                 int64_t z0, const uint4* rows, int R,
-                                                 const Bound& bound) {
+__device__ __forceinline__ uint32_t iq_plane_ssd(const LpImg& im, uint32_t base, uint32_t s,
+                                                 const uint4* rows, int R, const Bound& bound) {
   const int lane = threadIdx.x & 31;
-  const uint32_t s = (uint32_t)(x0 & 31);
-  const uint32_t ntx16 = (uint32_t)im.ntx * 16u, zs = (uint32_t)im.nty * ntx16;
-  const uint32_t base = (uint32_t)z0 * zs + ((uint32_t)x0 >> 5) * 16u;
-  const uint32_t y0u = (uint32_t)y0;
+  const uint4* p = im.p2 + base;
   int acc = 0;
   // batches of 4 x 32 rows while all lanes have one (see iq_quad_ssd)
   int r = lane;
   for (; r - lane + 4 * 32 <= R; r += 4 * 32) {
-    unsigned long long wa[4], wb[4];
-    uint4 t[4];
+    uint4 w[4], t[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       t[u] = rows[r + 32 * u];
-      const uint32_t yy = y0u + (t[u].w & 0xFFFFu);
-      const uint32_t i0 = base + (t[u].w >> 16) * zs + (yy >> 4) * ntx16 + (yy & 15u);
-      wa[u] = __ldg(im.b2 + i0);
-      wb[u] = __ldg(im.b2 + i0 + 16);
+      w[u] = __ldg(p + t[u].w);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const uint32_t a0 = __funnelshift_r((uint32_t)wa[u], (uint32_t)wb[u], s);
-      const uint32_t a1 = __funnelshift_r((uint32_t)(wa[u] >> 32), (uint32_t)(wb[u] >> 32), s);
-      acc += iq_row_ssd(a0, a1, t[u]);
-    }
-    int part = acc;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if ((float)part > __shfl_sync(0xffffffffu, bound(), 0)) return 0xFFFFFFFFu;
+    for (int u = 0; u < 4; ++u)
+      acc += iq_row_ssd(__funnelshift_r(w[u].x, w[u].y, s), __funnelshift_r(w[u].z, w[u].w, s), t[u]);
+    const uint32_t part = __reduce_add_sync(0xffffffffu, (uint32_t)acc);
+    if (r - lane + 4 * 32 == R) return part;  // (the same bound would be applied to the total)
+    if (__any_sync(0xffffffffu, (float)part > bound())) return 0xFFFFFFFFu;
   }
   for (; r < R; r += 32) {
     const uint4 t = rows[r];
-    const uint32_t yy = y0u + (t.w & 0xFFFFu);
-    const uint32_t i0 = base + (t.w >> 16) * zs + (yy >> 4) * ntx16 + (yy & 15u);
-    const unsigned long long a = __ldg(im.b2 + i0), b = __ldg(im.b2 + i0 + 16);
-    acc += iq_row_ssd(__funnelshift_r((uint32_t)a, (uint32_t)b, s),
-                      __funnelshift_r((uint32_t)(a >> 32), (uint32_t)(b >> 32), s), t);
+    const uint4 w = __ldg(p + t.w);
+    acc += iq_row_ssd(__funnelshift_r(w.x, w.y, s), __funnelshift_r(w.z, w.w, s), t);
   }
+  return __reduce_add_sync(0xffffffffu, (uint32_t)acc);
+}
+
+// Two windows of one column at once: the staged rows are read once for both, and the early exit is
+// taken when both sums are past the bound (a total past it may then come back as it is).
+template <typename Bound>
+__device__ __forceinline__ void iq_plane_ssd2(const LpImg& im, uint2 oa, uint2 ob, const uint4* rows,
+                                              int R, const Bound& bound, uint32_t& sa, uint32_t& sb) {
+  const int lane = threadIdx.x & 31;
+  const uint4 *pa = im.p2 + oa.x, *pb = im.p2 + ob.x;
+  int ca = 0, cb = 0;
+  int r = lane;
+  for (; r - lane + 4 * 32 <= R; r += 4 * 32) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  return (uint32_t)acc;
+    for (int h = 0; h < 2; ++h) {
+      uint4 t[2], wa[2], wb[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        t[u] = rows[r + 32 * (2 * h + u)];
+        wa[u] = __ldg(pa + t[u].w);
+        wb[u] = __ldg(pb + t[u].w);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        ca += iq_row_ssd(__funnelshift_r(wa[u].x, wa[u].y, oa.y), __funnelshift_r(wa[u].z, wa[u].w, oa.y), t[u]);
+        cb += iq_row_ssd(__funnelshift_r(wb[u].x, wb[u].y, ob.y), __funnelshift_r(wb[u].z, wb[u].w, ob.y), t[u]);
+      }
+    }
+    sa = __reduce_add_sync(0xffffffffu, (uint32_t)ca);
+    sb = __reduce_add_sync(0xffffffffu, (uint32_t)cb);
+    if (r - lane + 4 * 32 == R) return;
+    if (__any_sync(0xffffffffu, (float)min(sa, sb) > bound())) {
+      sa = sb = 0xFFFFFFFFu;
+      return;
+    }
+  }
+  for (; r < R; r += 32) {
+    const uint4 t = rows[r];
+    const uint4 wa = __ldg(pa + t.w), wb = __ldg(pb + t.w);
+    ca += iq_row_ssd(__funnelshift_r(wa.x, wa.y, oa.y), __funnelshift_r(wa.z, wa.w, oa.y), t);
+    cb += iq_row_ssd(__funnelshift_r(wb.x, wb.y, ob.y), __funnelshift_r(wb.z, wb.w, ob.y), t);
+  }
+  sa = __reduce_add_sync(0xffffffffu, (uint32_t)ca);
+  sb = __reduce_add_sync(0xffffffffu, (uint32_t)cb);
 }
 
 // Stage a column for either form (rows or quads at `stage`): the number of staged items, or -1
 // when the column cannot be summed in that form.
 __device__ inline int iq_stage(const LpImg& im, const LpColumn& col, uint4* stage) {
-  if (im.b2) return iq_stage_rows(col, stage);
+  if (im.p2) return iq_stage_rows(im, col, stage);
   return iq_stage_quads(col, stage) ? col.nq : -1;
 }
 
-// Exact sum of the column at distance-map position (x, y, z), either form; n: staged items.
+// Where the window at distance-map position p (strides dx, dxy) begins in either form: its first
+// entry or byte, and the bit shift of the plane form. (32-bit: P and the images are below 2^31.)
+__device__ __forceinline__ uint2 iq_lp_origin(const LpImg& im, uint32_t p, uint32_t dx, uint32_t dxy) {
+  const uint32_t z = p / dxy, r = p - z * dxy, y = r / dx, x = r - y * dx;
+  if (im.p2) return make_uint2((z * (uint32_t)im.ntx + (x >> 5)) * (uint32_t)im.ny + y, x & 31u);
+  return make_uint2(x + (uint32_t)im.isx * y + (uint32_t)im.isxy * z, 0u);
+}
+
+// Exact sum of the column for the window of origin o, either form; n: staged items.
 template <typename Bound>
-__device__ __forceinline__ uint32_t iq_lp_ssd(const LpImg& im, const uint4* stage, int n,
-                                              int64_t x, int64_t y, int64_t z, const Bound& bound) {
-  if (im.b2) return iq_plane_ssd(im, x, y, z, stage, n, bound);
-  return iq_quad_ssd(im.b8 + x + im.isx * y + im.isxy * z, stage, n, bound);
+__device__ __forceinline__ uint32_t iq_lp_ssd(const LpImg& im, const uint4* stage, int n, uint2 o,
+                                              const Bound& bound) {
+  if (im.p2) return iq_plane_ssd(im, o.x, o.y, stage, n, bound);
+  return iq_quad_ssd(im.b8 + o.x, stage, n, bound);
 }
 #endif
 #define IQ_LP_SAMPLES 8192  // positions sampled per column for its shortlist threshold
 // dst[0, n) = the image as bytes (dst holds n + 16 bytes; the 16 past the end are zeroed);
 // *bad (device) = 1 when a value is not an integer in [0, 255].
 int iq_lp_to_u8(iq_ctx* ctx, const float* src, int64_t n, uint8_t* dst, int* bad);
-// The plane form of an image of codes 0..3 (LpImg; dst: d.z * nty * ntx * 16 words);
+// The plane form of an image of codes 0..3 (LpImg; dst: d.z * ntx * d.y entries);
 // *bad (device) = 1 when a value is not one of the four codes.
-int iq_lp_to_planes(iq_ctx* ctx, const float* src, Dim3 d, int64_t ntx, int64_t nty,
-                    unsigned long long* dst, int* bad);
+int iq_lp_to_planes(iq_ctx* ctx, const float* src, Dim3 d, int64_t ntx, uint4* dst, int* bad);
 // Rows i * ceil(P / IQ_LP_SAMPLES) of the window embeddings (the sampled positions).
 int iq_lp_sample_rows(iq_ctx* ctx, const __nv_bfloat16* W, const float* nW, int64_t P,
                       __nv_bfloat16* Ws, float* nWs);

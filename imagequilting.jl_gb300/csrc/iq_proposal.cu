@@ -53,11 +53,14 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b
 }
 
 // Scores of every position against every column with tensor-core MMAs (mma.sync m16n8k16, BF16
-// in, FP32 accumulation): s = |w|^2 + |e|^2 - 2 w.e; positions with s <= tau[col] are appended
-// to the column's list (cap entries; cnt keeps counting past it so that an overflow is seen).
-// The columns are staged in shared memory in chunks of LP_SCAN_COLS (rows padded to 36 words,
-// conflict-free fragment loads); a warp keeps the A fragments of its 16 positions in registers
-// and sweeps the chunk's columns, so the window embeddings are read once per chunk.
+// in, FP32 accumulation): s = |w|^2 + |e|^2 - 2 w.e. The columns are staged in shared memory in chunks
+// of LP_SCAN_COLS (rows padded to 36 words, conflict-free fragment loads); a warp keeps the A
+// fragments of its 16 positions in registers and sweeps the chunk's columns, so the window embeddings
+// are read once per chunk.
+// Scan: the positions with s <= tau[col] leave as bits, four ballots per 16 positions x 8 columns;
+// lp_list_kernel turns a column's bits into its list, ascending. (Appending each hit with a global
+// atomic took 0.35 ms of a launch's 0.39 on a 0.46 M-position image with 55 columns: 16,384 adds to
+// one address per column.)
 // DENSE: every score is written to dense[col * P + row] instead (the sampled rows).
 constexpr int LP_SCAN_COLS = 512;
 constexpr int LP_SCAN_LD = 36;  // words per staged column (32 + 4 of padding)
@@ -70,8 +73,7 @@ __global__ void __launch_bounds__(LP_SCAN_THREADS) lp_scan_kernel(const __nv_bfl
                                                       const __nv_bfloat16* __restrict__ T,
                                                       const float* __restrict__ nT,
                                                       const float* __restrict__ tau, int N,
-                                                      int32_t* list, int32_t* cnt, int cap,
-                                                      float* dense) {
+                                                      uint4* __restrict__ bits, float* dense) {
   extern __shared__ __align__(16) uint32_t sT[];
   float* sN = reinterpret_cast<float*>(sT + LP_SCAN_COLS * LP_SCAN_LD);
   float* sTau = sN + LP_SCAN_COLS;
@@ -113,6 +115,7 @@ __global__ void __launch_bounds__(LP_SCAN_THREADS) lp_scan_kernel(const __nv_bfl
           // word ks * 8 + tig holds dims ks * 16 + 2 tig, +1 (b0); +4 words: dims + 8 (b1)
           const uint32_t* src = sT + (cl < nc ? cl : 0) * LP_SCAN_LD + tig;
           float acc[4] = {0.f, 0.f, 0.f, 0.f};
+          unsigned hit[4];
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
             const uint32_t b0 = cl < nc ? src[ks * 8] : 0u, b1 = cl < nc ? src[ks * 8 + 4] : 0u;
@@ -120,22 +123,72 @@ __global__ void __launch_bounds__(LP_SCAN_THREADS) lp_scan_kernel(const __nv_bfl
           }
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const int h = e & 1;
-            const int cc = cb + nt * 8 + 2 * tig + h;  // column within the chunk
-            if (cc >= nc) continue;
+            const int cc = cb + nt * 8 + 2 * tig + (e & 1);  // column within the chunk
             const int64_t row = e < 2 ? r0 : r1;
-            if (row >= P) continue;
+            const bool in = cc < nc && row < P;
             if (DENSE) {
-              dense[(int64_t)(c0 + cc) * P + row] = (e < 2 ? w0 : w1) + sN[cc] - 2.f * acc[e];
-            } else if (fmaf(-2.f, acc[e], e < 2 ? w0 : w1) <= sTau[cc]) {
-              const int idx = atomicAdd(cnt + c0 + cc, 1);
-              if (idx < cap) list[(int64_t)(c0 + cc) * cap + idx] = (int32_t)row;
+              if (in) dense[(int64_t)(c0 + cc) * P + row] = (e < 2 ? w0 : w1) + sN[cc] - 2.f * acc[e];
+            } else {
+              hit[e] = __ballot_sync(0xffffffffu, in && fmaf(-2.f, acc[e], e < 2 ? w0 : w1) <= sTau[cc]);
             }
           }
+          // word e: bit 4 g + t is row g (e < 2) or g + 8, column 2 t + (e & 1) of the tile
+          if (!DENSE && lane == 0 && cb + nt * 8 < nc)
+            bits[(int64_t)((c0 + cb) / 8 + nt) * nblk + blk] = make_uint4(hit[0], hit[1], hit[2], hit[3]);
         }
       }
     }
   }
+}
+
+// One column's list from the scan's bits: the positions in ascending order (the first `cap`), and
+// their count. A thread takes four blocks of 16 positions at a time (four loads in flight).
+constexpr int LL_NT = 512, LL_BLK = 4;
+
+__global__ void __launch_bounds__(LL_NT) lp_list_kernel(const uint4* __restrict__ bits, int64_t nblk,
+                                                        int32_t* list, int32_t* cnt, int cap) {
+  __shared__ int wsum[LL_NT / 32];
+  const int col = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint4* src = bits + (int64_t)(col >> 3) * nblk;
+  const int t = (col & 7) >> 1, h = col & 1;
+  int32_t* out = list + (int64_t)col * cap;
+  int base = 0;
+  for (int64_t b0 = 0; b0 < nblk; b0 += LL_NT * LL_BLK) {
+    const int64_t b = b0 + (int64_t)threadIdx.x * LL_BLK;
+    unsigned rows[2 * LL_BLK];  // eight rows g each, at bits 4 g
+    int c = 0;
+#pragma unroll
+    for (int k = 0; k < LL_BLK; ++k) {
+      const uint4 w = b + k < nblk ? src[b + k] : make_uint4(0u, 0u, 0u, 0u);
+      rows[2 * k] = ((h ? w.y : w.x) >> t) & 0x11111111u;
+      rows[2 * k + 1] = ((h ? w.w : w.z) >> t) & 0x11111111u;
+    }
+#pragma unroll
+    for (int k = 0; k < 2 * LL_BLK; ++k) c += __popc(rows[k]);
+    int inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
+    }
+    if (lane == 31) wsum[warp] = inc;
+    __syncthreads();
+    const int ws = lane < LL_NT / 32 ? wsum[lane] : 0;
+    int wi = ws;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, wi, o);
+      if (lane >= o) wi += y;
+    }
+    int at = base + __shfl_sync(0xffffffffu, wi - ws, warp) + inc - c;
+#pragma unroll
+    for (int k = 0; k < 2 * LL_BLK; ++k)
+      for (unsigned m = rows[k]; m; m &= m - 1, ++at)
+        if (at < cap) out[at] = (int32_t)(b * 16 + 8 * k + ((__ffs(m) - 1) >> 2));
+    base += __shfl_sync(0xffffffffu, wi, 31);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) cnt[col] = base;
 }
 
 // Rows i * stride of the window embeddings (the positions the per-column thresholds sample).
@@ -150,41 +203,37 @@ __global__ void lp_sample_rows_kernel(const __nv_bfloat16* __restrict__ W, const
   if (d == 0) nWs[row] = p < P ? nW[p] : 3.0e38f;
 }
 
-// The m-th smallest of each column's S sampled scores (MSD radix select on order-preserving
-// keys, one CTA per column).
-__global__ void __launch_bounds__(256) lp_select_kernel(const float* __restrict__ dense, int S,
-                                                        int m, float* tau) {
-  __shared__ unsigned hist[256];
-  __shared__ unsigned sel, need;
-  const float* x = dense + (int64_t)blockIdx.x * S;
-  unsigned prefix = 0, pmask = 0;
-  if (threadIdx.x == 0) need = (unsigned)m;
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    hist[threadIdx.x] = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < S; i += blockDim.x) {
-      const unsigned b = __float_as_uint(x[i]);
-      const unsigned key = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-      if ((key & pmask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned run = 0, d = 0;
-      for (; d < 255; ++d) {
-        if (run + hist[d] >= need) break;
-        run += hist[d];
-      }
-      sel = d;
-      need -= run;
-    }
-    __syncthreads();
-    prefix |= sel << shift;
-    pmask |= 255u << shift;
+// The m-th smallest of each column's S = IQ_LP_SAMPLES sampled scores, one CTA per column: the scores
+// stay in registers as order-preserving keys, and the largest v with fewer than m keys below it is
+// found a bit at a time (32 counts over the CTA; a radix select's histogram had all keys in a few of
+// its bins).
+constexpr int SEL_NT = 256;
+
+__global__ void __launch_bounds__(SEL_NT) lp_select_kernel(const float* __restrict__ dense, int m,
+                                                           float* tau) {
+  __shared__ int wcnt[2][SEL_NT / 32];
+  const float* x = dense + (int64_t)blockIdx.x * IQ_LP_SAMPLES;
+  unsigned key[IQ_LP_SAMPLES / SEL_NT];
+#pragma unroll
+  for (int i = 0; i < IQ_LP_SAMPLES / SEL_NT; ++i) {
+    const unsigned b = __float_as_uint(x[i * SEL_NT + threadIdx.x]);
+    key[i] = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
   }
-  if (threadIdx.x == 0) {
-    const unsigned b = (prefix & 0x80000000u) ? (prefix & 0x7FFFFFFFu) : ~prefix;
-    tau[blockIdx.x] = __uint_as_float(b);
+  unsigned v = 0;
+  for (int bit = 31; bit >= 0; --bit) {
+    const unsigned t = v | (1u << bit);
+    int c = 0;
+#pragma unroll
+    for (int i = 0; i < IQ_LP_SAMPLES / SEL_NT; ++i) c += key[i] < t ? 1 : 0;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0) wcnt[bit & 1][threadIdx.x >> 5] = c;
+    __syncthreads();
+    c = 0;
+#pragma unroll
+    for (int w = 0; w < SEL_NT / 32; ++w) c += wcnt[bit & 1][w];
+    if (c < m) v = t;
   }
+  if (threadIdx.x == 0) tau[blockIdx.x] = __uint_as_float((v & 0x80000000u) ? (v & 0x7FFFFFFFu) : ~v);
 }
 
 __global__ void lp_template_features_kernel(LpGeo g, const float* grid, const int64_t* tsrc,
@@ -212,12 +261,17 @@ __global__ void __launch_bounds__(256) lp_full_kernel(const LpImg im, int64_t dx
   if (nst < 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned mn = 0x7F800000u;
-  for (int64_t p = (int64_t)blockIdx.x * 8 + warp; p < P; p += (int64_t)gridDim.x * 8) {
-    const int64_t z = p / dxy, r = p - z * dxy, y = r / dx, x = r - y * dx;
-    const uint32_t s = iq_lp_ssd(im, qd, nst, x, y, z, [] { return INFINITY; });
-    const float acc = (float)s;
-    if (lane == 0) D[p] = acc;
-    mn = min(mn, __float_as_uint(acc));
+  for (int64_t p0 = ((int64_t)blockIdx.x * 8 + warp) * 32; p0 < P; p0 += (int64_t)gridDim.x * 8 * 32) {
+    const uint2 o = iq_lp_origin(im, (uint32_t)min(p0 + lane, P - 1), (uint32_t)dx, (uint32_t)dxy);
+    const int m = (int)min((int64_t)32, P - p0);
+    float mine = 0.f;
+    for (int e = 0; e < m; ++e) {
+      const uint2 oe = make_uint2(__shfl_sync(0xffffffffu, o.x, e), __shfl_sync(0xffffffffu, o.y, e));
+      const float acc = (float)iq_lp_ssd(im, qd, nst, oe, [] { return INFINITY; });
+      if (lane == e) mine = acc;
+      mn = min(mn, __float_as_uint(acc));
+    }
+    if (lane < m) D[p0 + lane] = mine;
   }
   if (lane == 0) atomicMin(dmin, mn);
 }
@@ -270,39 +324,36 @@ __global__ void lp_to_u8_kernel(const float* __restrict__ src, int64_t n, uint8_
 
 namespace {
 // Plane form of an image of codes 0..3 (see LpImg); *bad = 1 for any other value.
-__global__ void lp_to_planes_kernel(const float* __restrict__ src, Dim3 d, int64_t ntx, int64_t nty,
-                                    unsigned long long* dst, int* bad) {
-  const int64_t nw = d.z * nty * ntx * 16;
+__global__ void lp_to_planes_kernel(const float* __restrict__ src, Dim3 d, int64_t ntx, uint4* dst,
+                                    int* bad) {
+  const int64_t nw = d.z * ntx * d.y;
   int b = 0;
   for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < nw;
        w += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t yr = w & 15, t = w >> 4;
-    const int64_t tx = t % ntx, ty = (t / ntx) % nty, z = t / (ntx * nty);
-    const int64_t y = ty * 16 + yr;
-    uint32_t p0 = 0, p1 = 0;
-    if (y < d.y) {
+    const int64_t y = w % d.y, t = w / d.y, tx = t % ntx, z = t / ntx;
+    uint32_t p0[2] = {0, 0}, p1[2] = {0, 0};
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
       for (int i = 0; i < 32; ++i) {
-        const int64_t x = tx * 32 + i;
+        const int64_t x = (tx + k) * 32 + i;
         if (x >= d.x) break;
         const float v = src[x + d.x * y + d.x * d.y * z];
         if (!(v == 0.f || v == 1.f || v == 2.f || v == 3.f)) b = 1;
         const uint32_t c = (uint32_t)v & 3u;
-        p0 |= (c & 1u) << i;
-        p1 |= (c >> 1) << i;
+        p0[k] |= (c & 1u) << i;
+        p1[k] |= (c >> 1) << i;
       }
-    }
-    dst[w] = (unsigned long long)p0 | ((unsigned long long)p1 << 32);
+    dst[w] = make_uint4(p0[0], p0[1], p1[0], p1[1]);
   }
   if (__syncthreads_or(b) && threadIdx.x == 0) atomicOr(bad, 1);
 }
 }  // namespace
 
-int iq_lp_to_planes(iq_ctx* ctx, const float* src, Dim3 d, int64_t ntx, int64_t nty,
-                    unsigned long long* dst, int* bad) {
+int iq_lp_to_planes(iq_ctx* ctx, const float* src, Dim3 d, int64_t ntx, uint4* dst, int* bad) {
   IQ_CUDA_OK(cudaMemsetAsync(bad, 0, sizeof(int), ctx->stream));
-  const int64_t nw = d.z * nty * ntx * 16;
+  const int64_t nw = d.z * ntx * d.y;
   lp_to_planes_kernel<<<(unsigned)std::min<int64_t>((nw + 255) / 256, 4096), 256, 0, ctx->stream>>>(
-      src, d, ntx, nty, dst, bad);
+      src, d, ntx, dst, bad);
   iq_count(ctx);
   IQ_CUDA_OK(cudaGetLastError());
   return IQ_OK;
@@ -334,6 +385,9 @@ int iq_lp_shortlist(iq_ctx* ctx, const __nv_bfloat16* W, const float* nW, int64_
                     const float* nT, int N, int64_t k, float* tau, float* dense, int32_t* list,
                     int32_t* cnt, int cap) {
   if (N <= 0) return IQ_OK;
+  const int64_t nblk = (P + 15) / 16;
+  uint4* bits = (uint4*)iq_scratch(ctx, S_LP_BITS2, sizeof(uint4) * (size_t)((N + 7) / 8) * nblk);
+  if (!bits) return IQ_ERR_ALLOC;
   const int S = IQ_LP_SAMPLES;
   const int64_t stride = (P + S - 1) / S;
   // the m-th smallest sampled score stands for about m * stride positions
@@ -348,16 +402,15 @@ int iq_lp_shortlist(iq_ctx* ctx, const __nv_bfloat16* W, const float* nW, int64_
   IQ_CUDA_OK(cudaFuncSetAttribute(lp_scan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   IQ_CUDA_OK(cudaFuncSetAttribute(lp_scan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   lp_scan_kernel<true><<<(unsigned)((S / 16 + 15) / 16), LP_SCAN_THREADS, sm, st>>>(
-      Ws, nWs, S, T, nT, nullptr, N, nullptr, nullptr, 0, dense);
-  lp_select_kernel<<<(unsigned)N, 256, 0, st>>>(dense, S, m, tau);
+      Ws, nWs, S, T, nT, nullptr, N, nullptr, dense);
+  lp_select_kernel<<<(unsigned)N, SEL_NT, 0, st>>>(dense, m, tau);
   IQ_CUDA_OK(cudaGetLastError());
-  IQ_CUDA_OK(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * N, st));
-  const int64_t nblk = (P + 15) / 16;
   const int64_t gx = std::max<int64_t>(1, std::min<int64_t>((nblk + 15) / 16, (int64_t)nsm * 2));
-  lp_scan_kernel<false><<<(unsigned)gx, LP_SCAN_THREADS, sm, st>>>(W, nW, P, T, nT, tau, N, list,
-                                                                   cnt, cap, nullptr);
+  lp_scan_kernel<false><<<(unsigned)gx, LP_SCAN_THREADS, sm, st>>>(W, nW, P, T, nT, tau, N, bits,
+                                                                   nullptr);
+  lp_list_kernel<<<(unsigned)N, LL_NT, 0, st>>>(bits, nblk, list, cnt, cap);
   iq_timer_stop(ctx, "lp.scan", 2.0 * (double)(P + S) * N * EMB);
-  iq_count(ctx, 3);
+  iq_count(ctx, 4);
   IQ_CUDA_OK(cudaGetLastError());
   return IQ_OK;
 }
@@ -376,14 +429,14 @@ int iq_lp_recall(iq_ctx* ctx, const LpImg& im, Dim3 dist, const LpColumn& col,
                  const int32_t* list, const int32_t* cnt, int cap, double tol, float* Dbuf,
                  unsigned* dmin, uint32_t* bits, unsigned long long* counters) {
   const int64_t P = dist.vol();
-  const size_t sm = (size_t)16 * (im.b2 ? (size_t)col.tdim[1] * col.tdim[2] : (size_t)col.nq) + 16;
+  const size_t sm = (size_t)16 * (im.p2 ? (size_t)col.tdim[1] * col.tdim[2] : (size_t)col.nq) + 16;
   if (sm > 227 * 1024) return iq_set_error(IQ_ERR_LIMIT, "recall check: mask too large");
   IQ_CUDA_OK(cudaFuncSetAttribute(lp_full_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const unsigned inf = 0x7F800000u;
   IQ_CUDA_OK(cudaMemcpyAsync(dmin, &inf, sizeof(unsigned), cudaMemcpyHostToDevice, ctx->stream));
   IQ_CUDA_OK(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * ((P + 31) / 32), ctx->stream));
   iq_timer_start(ctx, "lp.monitor");
-  lp_full_kernel<<<(unsigned)std::min<int64_t>((P + 7) / 8, 152 * 8), 256, sm, ctx->stream>>>(
+  lp_full_kernel<<<(unsigned)std::min<int64_t>((P + 255) / 256, 152 * 8), 256, sm, ctx->stream>>>(
       im, dist.x, dist.x * dist.y, P, col, Dbuf, dmin);
   lp_mark_kernel<<<64, 256, 0, ctx->stream>>>(list, cnt, cap, bits);
   lp_recall_kernel<<<(unsigned)std::min<int64_t>((P + 255) / 256, 1024), 256, 0, ctx->stream>>>(

@@ -48,9 +48,9 @@ struct IqLp {
   size_t ti8_bytes = 0;
   int64_t ti8_ti = -1;
   bool ti8_ok = false;
-  unsigned long long* ti2 = nullptr;  // plane form (codes 0..3)
+  uint4* ti2 = nullptr;  // plane form (codes 0..3)
   size_t ti2_words = 0;
-  int64_t ti2_ntx = 0, ti2_nty = 0;
+  int64_t ti2_ntx = 0;
   bool ti2_ok = false;
   int* d_bad = nullptr;
   std::vector<LpCache> cache;
@@ -208,25 +208,24 @@ int ensure_ti8(iq_ctx* ctx, IqLp* lp) {
   // plane form when the codes are 0..3
   lp->ti2_ok = false;
   if (lp->ti8_ok) {
-    const int64_t ntx = (ctx->ti.x + 31) / 32 + 1, nty = (ctx->ti.y + 15) / 16;
-    const size_t words = (size_t)(ctx->ti.z * nty * ntx * 16);
+    const int64_t ntx = (ctx->ti.x + 31) / 32;
+    const size_t words = (size_t)(ctx->ti.z * ntx * ctx->ti.y);
     if (lp->ti2_words < words) {
       cudaFree(lp->ti2);
       lp->ti2 = nullptr;
       lp->ti2_words = 0;
-      if (cudaMalloc(&lp->ti2, sizeof(unsigned long long) * words) != cudaSuccess) {
+      if (cudaMalloc(&lp->ti2, sizeof(uint4) * words) != cudaSuccess) {
         cudaGetLastError();
         return iq_set_error(IQ_ERR_ALLOC, "proposal: plane image allocation failed");
       }
       lp->ti2_words = words;
     }
-    rc = iq_lp_to_planes(ctx, ctx->d_ti, ctx->ti, ntx, nty, lp->ti2, lp->d_bad);
+    rc = iq_lp_to_planes(ctx, ctx->d_ti, ctx->ti, ntx, lp->ti2, lp->d_bad);
     if (rc) return rc;
     IQ_CUDA_OK(cudaMemcpyAsync(&bad, lp->d_bad, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     IQ_CUDA_OK(cudaStreamSynchronize(ctx->stream));
     lp->ti2_ok = bad == 0 && words < ((size_t)1 << 31);
     lp->ti2_ntx = ntx;
-    lp->ti2_nty = nty;
   }
   lp->ti8_ti = ctx->ti_version;
   return IQ_OK;
@@ -239,9 +238,9 @@ LpImg lp_image(iq_ctx* ctx, IqLp* lp, Dim3 tile) {
   im.isx = ctx->ti.x;
   im.isxy = ctx->ti.x * ctx->ti.y;
   if (lp->ti2_ok && tile.x <= 32) {
-    im.b2 = lp->ti2;
-    im.ntx = lp->ti2_ntx;
-    im.nty = lp->ti2_nty;
+    im.p2 = lp->ti2;
+    im.ntx = (int32_t)lp->ti2_ntx;
+    im.ny = (int32_t)ctx->ti.y;
   }
   return im;
 }

@@ -6,10 +6,13 @@
 // full scan's.
 //
 // Codes 0..3 with tiles of x extent <= 32: the training image as 2-bit planes and the template
-// as staged rows, one row of 32 codes per lane step (iq_plane_ssd in iq_internal.h). Other byte
+// as staged rows, one row of 32 codes per lane step (iq_plane_ssd in iq_internal.h): one 16-byte
+// load, two shifts, eight logic operations and three counts a row. Other byte
 // codes: the image as bytes and the mask as quads of four consecutive x offsets of one row; a
 // lane forms the four differences of a quad with one __vabsdiffu4 and adds their squares with
 // one __dp4a. A sum stops early once it exceeds (1 + tol) x the running minimum x (1 + 2e-6).
+#include <algorithm>
+
 #include "iq_internal.h"
 
 namespace {
@@ -24,7 +27,9 @@ struct LpPickArgs {
   const int32_t* list;         // shortlists [N][cap]
   const int32_t* cnt;
   int cap;
-  float* dl;                   // distances of the shortlist entries [N][cap]
+  float* dl;                   // distances of the shortlist entries [N][cap] (+Inf: abandoned)
+  unsigned* dmin;              // per column the running minimum (bits of a non-negative float; all
+                               // ones: the column cannot be summed in the image's form)
   double tol;
   uint64_t seed;
   int64_t* rind;               // per column: drawn position, -1 when the column must fall back
@@ -50,26 +55,29 @@ __device__ __forceinline__ void lp_bitonic(unsigned long long* buf, int n) {
     }
 }
 
-__global__ void __launch_bounds__(LP_PT) lp_pick_kernel(const LpPickArgs a) {
+// The exact sums of a slice of LS_SLICE shortlist entries of one column. A warp takes 32 entries
+// (their origins a lane each), two at a time over the staged rows. Slices of all columns fill the
+// chip (a column per CTA left half of the warps of ~150 SMs idle, and the slowest column decided);
+// the running minimum of a column is shared through global memory, read once per 32 entries.
+// What bounds the sums: L1 (16 bytes of image and template a row and lane) and POPC. Per call of
+// the 192 x 192 x 64 facies ensemble (6,144 columns of 16,384 positions, tile 32 x 32 x 16): 100 ms
+// a column per CTA with two 8-byte loads a row, four counts and shuffle sums; 76 with one 16-byte
+// load, three counts and hardware reductions; 40 here.
+constexpr int LS_NT = 256, LS_SLICE = 2048;
+
+__global__ void __launch_bounds__(LS_NT) lp_sum_kernel(const LpPickArgs a) {
   extern __shared__ __align__(16) unsigned char dyn[];
-  __shared__ float red[32];
-  __shared__ unsigned long long ured[32];
-  __shared__ int sflag;
-  __shared__ unsigned smin;  // running minimum of the finished sums (bits of a non-negative float)
-  const int c = blockIdx.x;
-  const LpColumn col = a.cols[c];
+  __shared__ unsigned smin;
+  const int c = blockIdx.y, beg = blockIdx.x * LS_SLICE;
+  const int cnt = a.cnt[c];
+  if (cnt > a.cap || beg >= cnt) return;  // (an overflowed shortlist falls back)
+  const int end = min(cnt, beg + LS_SLICE);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int n = min(a.cnt[c], a.cap);
-  if (a.cnt[c] > a.cap || n <= 0) {  // overflowed or empty shortlist: the column falls back
-    if (threadIdx.x == 0) { a.rind[c] = -1; a.ncand[c] = 0; }
-    return;
-  }
-  // the column's rows (plane form) or quads (byte form) in shared memory
   uint4* qd = reinterpret_cast<uint4*>(dyn);
   if (threadIdx.x == 0) smin = 0x7F7FFFFFu;
-  const int nst = iq_stage(a.im, col, qd);
-  if (nst < 0) {  // template values outside the form: the column falls back
-    if (threadIdx.x == 0) { a.rind[c] = -1; a.ncand[c] = 0; }
+  const int nst = iq_stage(a.im, a.cols[c], qd);
+  if (nst < 0) {
+    if (threadIdx.x == 0) a.dmin[c] = 0xFFFFFFFFu;
     return;
   }
   // An entry is abandoned once a partial sum exceeds (1 + tol) * running minimum * (1 + 2e-6):
@@ -78,21 +86,56 @@ __global__ void __launch_bounds__(LP_PT) lp_pick_kernel(const LpPickArgs a) {
   const float pf = (float)((1.0 + a.tol) * (1.0 + 2e-6));
   const int32_t* lst = a.list + (int64_t)c * a.cap;
   float* dl = a.dl + (int64_t)c * a.cap;
-  float mloc = 3.4e38f;
-  for (int i = warp; i < n; i += LP_PT / 32) {
-    const int64_t p = lst[i];
-    const int64_t z = p / a.dxy, r = p - z * a.dxy, y = r / a.dx, x = r - y * a.dx;
-    const uint32_t s = iq_lp_ssd(a.im, qd, nst, x, y, z, [&] {
-      return __uint_as_float(*(volatile unsigned*)&smin) * pf;
-    });
-    const bool pruned = s == 0xFFFFFFFFu;
-    const float acc = pruned ? INFINITY : (float)s;
-    if (lane == 0) {
-      dl[i] = acc;
-      if (!pruned) atomicMin(&smin, __float_as_uint(acc));
+  auto bound = [&] { return __uint_as_float(*(volatile unsigned*)&smin) * pf; };
+  for (int i0 = beg + warp * 32; i0 < end; i0 += LS_NT) {
+    const int m = min(32, end - i0);
+    const uint2 o = iq_lp_origin(a.im, (uint32_t)lst[min(i0 + lane, end - 1)], (uint32_t)a.dx, (uint32_t)a.dxy);
+    if (lane == 0) atomicMin(&smin, __ldcg(a.dmin + c));
+    float mine = INFINITY;
+    unsigned best = 0xFFFFFFFFu;
+    for (int e = 0; e < m; e += 2) {
+      const int f = min(e + 1, m - 1);
+      const uint2 oa = make_uint2(__shfl_sync(0xffffffffu, o.x, e), __shfl_sync(0xffffffffu, o.y, e));
+      uint32_t sa, sb;
+      if (a.im.p2) {
+        const uint2 ob = make_uint2(__shfl_sync(0xffffffffu, o.x, f), __shfl_sync(0xffffffffu, o.y, f));
+        iq_plane_ssd2(a.im, oa, ob, qd, nst, bound, sa, sb);
+      } else {
+        const uint2 ob = make_uint2(__shfl_sync(0xffffffffu, o.x, f), __shfl_sync(0xffffffffu, o.y, f));
+        sa = iq_lp_ssd(a.im, qd, nst, oa, bound);
+        sb = iq_lp_ssd(a.im, qd, nst, ob, bound);
+      }
+      if (sa != 0xFFFFFFFFu && lane == e) mine = (float)sa;
+      if (sb != 0xFFFFFFFFu && lane == f) mine = (float)sb;
+      const unsigned lo = min(sa, sb);
+      if (lo < best) {
+        best = lo;
+        if (lane == 0) atomicMin(&smin, __float_as_uint((float)lo));
+      }
     }
-    mloc = fminf(mloc, acc);
+    if (lane < m) dl[i0 + lane] = mine;
+    if (lane == 0 && best != 0xFFFFFFFFu) atomicMin(a.dmin + c, __float_as_uint((float)best));
   }
+}
+
+__global__ void __launch_bounds__(LP_PT) lp_pick_kernel(const LpPickArgs a) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ float red[32];
+  __shared__ unsigned long long ured[32];
+  __shared__ int sflag;
+  const int c = blockIdx.x;
+  const LpColumn col = a.cols[c];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = min(a.cnt[c], a.cap);
+  // an overflowed or empty shortlist, or template values outside the form: the column falls back
+  if (a.cnt[c] > a.cap || n <= 0 || a.dmin[c] == 0xFFFFFFFFu) {
+    if (threadIdx.x == 0) { a.rind[c] = -1; a.ncand[c] = 0; }
+    return;
+  }
+  const int32_t* lst = a.list + (int64_t)c * a.cap;
+  const float* dl = a.dl + (int64_t)c * a.cap;
+  float mloc = 3.4e38f;
+  for (int i = threadIdx.x; i < n; i += LP_PT) mloc = fminf(mloc, dl[i]);
   // minimum
   for (int o = 16; o > 0; o >>= 1) mloc = fminf(mloc, __shfl_xor_sync(0xffffffffu, mloc, o));
   if (lane == 0) red[warp] = mloc;
@@ -212,18 +255,28 @@ int iq_lp_pick(iq_ctx* ctx, const LpImg& im, Dim3 dist, const LpColumn* cols, in
   a.im = im; a.dx = dist.x; a.dxy = dist.x * dist.y;
   a.cols = cols; a.list = list; a.cnt = cnt; a.cap = cap; a.dl = dl; a.tol = tol; a.seed = seed;
   a.rind = rind; a.ncand = ncand; a.ties = ctx->d_ties;
-  // shared memory: the mask's rows or quads (16 bytes each; maxQ: the most of either), later
-  // the sort buffers, weights and sums
-  const size_t sm = std::max<size_t>((size_t)16 * maxQ,
-                                     (size_t)LP_SORT * (8 + 8 + 8 + 4) +
-                                         8 * ((LP_SORT + IQ_DRAW_CHUNK - 1) / IQ_DRAW_CHUNK)) + 64;
-  if (sm > 227 * 1024)
+  // shared memory of the sums: the mask's rows or quads (16 bytes each; maxQ: the most of either);
+  // of the pick: the sort buffers, weights and sums
+  const size_t sq = (size_t)16 * maxQ + 16;
+  const size_t sm = (size_t)LP_SORT * (8 + 8 + 8 + 4) +
+                    8 * ((LP_SORT + IQ_DRAW_CHUNK - 1) / IQ_DRAW_CHUNK) + 64;
+  if (sq > 226 * 1024)
     return iq_set_error(IQ_ERR_LIMIT, "proposal pick: a mask of %d quads is too large", maxQ);
+  a.dmin = (unsigned*)iq_scratch(ctx, S_LP_MIN, sizeof(unsigned) * N);
+  if (!a.dmin) return IQ_ERR_ALLOC;
+  IQ_CUDA_OK(cudaMemsetAsync(a.dmin, 0x7F, sizeof(unsigned) * N, ctx->stream));  // 3.4e38
+  IQ_CUDA_OK(cudaFuncSetAttribute(lp_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sq));
   IQ_CUDA_OK(cudaFuncSetAttribute(lp_pick_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   iq_timer_start(ctx, "lp.pick");
+  for (int c0 = 0; c0 < N; c0 += 65535) {  // (columns are the grid's y)
+    LpPickArgs b = a;
+    b.cols += c0; b.list += (int64_t)c0 * cap; b.cnt += c0; b.dl += (int64_t)c0 * cap; b.dmin += c0;
+    lp_sum_kernel<<<dim3((unsigned)((cap + LS_SLICE - 1) / LS_SLICE), (unsigned)std::min(N - c0, 65535)),
+                    LS_NT, sq, ctx->stream>>>(b);
+  }
   lp_pick_kernel<<<(unsigned)N, LP_PT, sm, ctx->stream>>>(a);
   iq_timer_stop(ctx, "lp.pick");
-  iq_count(ctx);
+  iq_count(ctx, 2);
   IQ_CUDA_OK(cudaGetLastError());
   return IQ_OK;
 }
