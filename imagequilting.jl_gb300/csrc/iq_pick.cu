@@ -1139,12 +1139,6 @@ __device__ __forceinline__ void ref_mark(RefArr& a, uint32_t i) {
   if ((a.l[i] & 0x7F) < 3) a.l[i] = (uint8_t)(a.l[i] | 0x80);  // racing writers store one value
 }
 
-// (value, position) order of entries i and j
-__device__ __forceinline__ bool ref_less(const RefArr& a, const int32_t* pos, uint32_t i, uint32_t j) {
-  const double vi = a.v[i], vj = a.v[j];
-  return vi < vj || (vi == vj && (pos[i] & 0x7FFFFFFF) < (pos[j] & 0x7FFFFFFF));
-}
-
 // Sort entries [0, n) by (level-1 value, ordinal) into ord[0, n) (ordinals; ordinal order is
 // position order): a bitonic sort in shared memory up to SORT_CAP, else the radix sort.
 __device__ const uint32_t* ref_sort(Smem& s, unsigned long long* sbuf, int64_t n, RefArr a,
@@ -1168,11 +1162,12 @@ __device__ const uint32_t* ref_sort(Smem& s, unsigned long long* sbuf, int64_t n
 }
 
 // Make the order ord[0, n) exact: while two neighbours' intervals overlap (and are not both
-// exact), raise both and re-sort the runs of raised neighbours by (value, position). At the
-// end every adjacent pair is disjoint or both exact, so the order is the order of the Float64
-// distances with ties broken by position.
-__device__ __noinline__ void ref_resolve(Smem& s, const Ref& f, const int32_t* pos, int64_t n, uint32_t* ord,
-                            RefArr a) {
+// exact), raise both and sort again by (value, position). At the end every adjacent pair is disjoint
+// or both exact, so the order is the order of the Float64 distances with ties broken by position.
+// Returns the order (ord, or above SORT_CAP entries one of v0, v1).
+__device__ __noinline__ uint32_t* ref_resolve(Smem& s, unsigned long long* sbuf, const Ref& f,
+                                              const int32_t* pos, int64_t n, uint32_t* ord, RefArr a,
+                                              uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1) {
   for (int round = 0; round < 64; ++round) {
     int any = 0;
     for (int64_t t = threadIdx.x; t < n; t += PT) a.link[t] = 0;
@@ -1207,23 +1202,24 @@ __device__ __noinline__ void ref_resolve(Smem& s, const Ref& f, const int32_t* p
       __syncthreads();
       continue;
     }
-    // runs of linked neighbours [t, e]: insertion sort by (value, position)
-    for (int64_t t = threadIdx.x; t + 1 < n; t += PT) {
-      if (!a.link[t] || (t > 0 && a.link[t - 1])) continue;
-      int64_t e = t + 1;
-      while (e + 1 < n && a.link[e]) ++e;
-      for (int64_t x = t + 1; x <= e; ++x) {
-        const uint32_t key = ord[x];
-        int64_t y = x - 1;
-        while (y >= t && ref_less(a, pos, key, ord[y])) {
-          ord[y + 1] = ord[y];
-          --y;
-        }
-        ord[y + 1] = key;
-      }
+    // the whole order again: stable radix sorts by the low, then the high word of the Float64 values
+    // from the entries' order (position order). A raised entry may move past neighbours that are exact
+    // already, so sorting the raised runs alone would leave exact pairs out of order.
+    for (int64_t i = threadIdx.x; i < n; i += PT) {
+      k0[i] = (uint32_t)__double_as_longlong(a.v[i]);
+      v0[i] = (uint32_t)i;
     }
     __syncthreads();
+    uint32_t* wcnt = reinterpret_cast<uint32_t*>(sbuf);
+    const bool w = radix_sort(s, wcnt, k0, v0, k1, v1, n) != 0;
+    uint32_t *ka = w ? k1 : k0, *va = w ? v1 : v0, *kb = w ? k0 : k1, *vb = w ? v0 : v1;
+    for (int64_t t = threadIdx.x; t < n; t += PT)
+      ka[t] = (uint32_t)((unsigned long long)__double_as_longlong(a.v[va[t]]) >> 32);
+    __syncthreads();
+    ord = radix_sort(s, wcnt, ka, va, kb, vb, n) ? vb : va;
+    __syncthreads();
   }
+  return ord;
 }
 
 // Near-tie test |D - t| <= 1e-6 t (evaluated as the oracle does, in Float64) of entry i against
@@ -1397,7 +1393,7 @@ __device__ __noinline__ long long band_topk(Smem& s, unsigned long long* sbuf, c
     ref_raise(f, list, bn, a, round >= 1);
     ord = const_cast<uint32_t*>(ref_sort(s, sbuf, bn, a, k0, v0, k1, v1));
   }
-  if (!split) ref_resolve(s, f, list, bn, ord, a);
+  if (!split) ord = ref_resolve(s, sbuf, f, list, bn, ord, a, k0, v0, k1, v1);
   for (int64_t t = threadIdx.x; t < kk; t += PT) list[ord[t]] |= (int32_t)0x80000000;
   __syncthreads();
   // the boundary: the largest (value, position) of the set
@@ -1483,7 +1479,7 @@ __device__ __noinline__ unsigned long long dense_ranks_refined(Smem& s, unsigned
     ref_init(f, cand, n, a);
   }
   uint32_t* ord = const_cast<uint32_t*>(ref_sort(s, sbuf, n, a, k0, v0, k1, v1));
-  ref_resolve(s, f, cand, n, ord, a);
+  ord = ref_resolve(s, sbuf, f, cand, n, ord, a, k0, v0, k1, v1);
   uint32_t carry = 0;
   unsigned long long acc = 0;
   for (int64_t t0 = 0; t0 < n; t0 += PT) {

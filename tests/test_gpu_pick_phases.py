@@ -3,6 +3,8 @@ pick decides on exact distances whatever route it takes; no tolerance):
 
 - relaxation selections listed whole (at most 8192 positions) or tested by a scan of the map;
 - candidates ranked from distances made between the pick's phases (at most 4096) or in the pick;
+- threshold maps of at least 65,536 positions collected by a pass of their own (up to 8192 kept), smaller
+  ones by the pick;
 - threshold picks decided by the minimum's interval, or, on images whose distances tie (values on a
   coarse grid that FP16 halves do not hold exactly), by its exact value.
 """
@@ -47,7 +49,10 @@ def test_relaxation_routes(iq, ctx, tol, hard, nsoft):
 @pytest.mark.parametrize("values", ["continuous", "coarse"])
 @pytest.mark.parametrize("shape,tile,out,tol", [((70, 66), (9, 8), (22, 20), 0.1),
                                                 ((70, 66), (9, 8), (22, 20), 1.0),
-                                                ((30, 28, 20), (6, 7, 5), (15, 14, 9), 0.4)])
+                                                ((30, 28, 20), (6, 7, 5), (15, 14, 9), 0.4),
+                                                # 82,636 positions: collected ahead of the pick
+                                                ((300, 290), (9, 8), (15, 14), 0.1),
+                                                ((300, 290), (9, 8), (15, 14), 1.0)])
 def test_threshold_routes(iq, ctx, values, shape, tile, out, tol):
     rng = np.random.default_rng(92)
     ti = rng.normal(size=shape) if values == "continuous" else rng.integers(1, 4, shape) / 3.0
