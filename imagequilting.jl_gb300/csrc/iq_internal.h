@@ -128,7 +128,7 @@ enum IqSlot {
   S_PBH_OUT, S_PBH_POOL, S_PBH_SRC,
   S_LP_T, S_LP_NT, S_LP_TAU, S_LP_LIST, S_LP_CNT, S_LP_DL, S_LP_COLS, S_LP_TSRC, S_LP_TBOX,
   S_LP_RIND, S_LP_NCAND, S_LP_D, S_LP_BITS, S_LP_ITEMS, S_LP_X, S_LP_E, S_LP_GE, S_LP_FEAT, S_LP_BH1, S_LP_BGZ1, S_LP_BH2, S_LP_DENSE, S_LP_QUAD,
-  S_TZ_IMG, S_TZ_A2, S_TZ_PLAN, S_TZ_B, S_TZ_SIMG, S_TZ_SA2, S_PREDRAW, S_LP_W, S_LVL1, S_PB_MEMB, S_LP_BITS2, S_LP_MIN,
+  S_TZ_IMG, S_TZ_A2, S_TZ_PLAN, S_TZ_B, S_TZ_SIMG, S_TZ_SA2, S_PREDRAW, S_LP_W, S_LVL1, S_PB_MEMB, S_LP_BITS2, S_LP_MIN, S_THR,
   S_COUNT
 };
 
@@ -407,6 +407,7 @@ struct PickTask {
   ExactSrc xa[IQ_MAX_AUX];
 };
 
+constexpr int64_t IQ_THR_MIN = 65536; // positions from which threshold picks are collected ahead
 constexpr int IQ_RANK_CAP = 4096;  // most candidates of a pick evaluated between its phases
 struct PickLaunch {
   int64_t P = 0;           // positions
@@ -437,6 +438,10 @@ struct PickLaunch {
   // pick evaluates them itself); maxK: most offsets of a refined source
   float* lvl1 = nullptr;
   int maxK = 0;
+  // threshold picks (tasks without auxiliary sources, any_thr): two counters per CTA for collecting
+  // their positions ahead of the pick (nullable)
+  int* thr = nullptr;
+  bool any_thr = false;
   // outputs, one per CTA
   int64_t* rind = nullptr;
   int64_t* ncand = nullptr;  // nullable

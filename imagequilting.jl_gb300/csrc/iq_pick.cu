@@ -26,6 +26,8 @@
 // candidates). All Float64 arithmetic uses explicit round-to-nearest intrinsics so that the
 // weights equal the oracle's bit for bit; the draw sums in the fixed order of
 // oracle/iqsim_oracle.sample_index.
+#include <algorithm>
+
 #include "iq_internal.h"
 
 namespace {
@@ -64,6 +66,8 @@ struct PickArgs {
                       // level-1 distances of the candidates made in between (rank_eval_kernel)
   float* lvl1;        // [CTA][nsrc][IQ_RANK_CAP] (phases 1 and 2)
   int nsrc;
+  int* thr_n;         // threshold picks: positions collected in cand per CTA (nullable: by the pick)
+  int* thr_ties;      // near-ties counted while collecting (exact maps)
 };
 
 // small shared state (static); the large regions are dynamic shared memory:
@@ -1535,25 +1539,30 @@ __device__ __noinline__ int64_t ref_filter(Smem& s, int32_t* pos, int64_t n, Ref
 // Threshold pick of a refined map (src/iqsim.jl:237): the candidates D <= (1 + tol) min D of the
 // Float64 distance, ascending in cand[0, n), with their intervals in `a`; `ties` receives the
 // positions within 1e-6 of the threshold. m32 is the smallest FP32 value (finite).
-__device__ __noinline__ int64_t thr_refined(Smem& s, const Ref& f, const float* __restrict__ D, int64_t P,
-                               double m32, double tol, int32_t* cand, RefArr a,
-                               unsigned long long& ties) {
+// `ncol`: the positions up to thr_cut are in cand[0, ncol) already (< 0: collected here).
+__device__ double thr_cut(const Ref& f, double m32, double tol) {
   // every candidate, the minimum and every near-tie have D32 <= cut
-  __shared__ double scut;
-  if (threadIdx.x == 0) {
-    double E0 = tier0_bound(f, (1.0 + tol) * m32 * 1.01), c = 0.0;
-    for (int it = 0; it < 200; ++it) {
-      c = (1.0 + tol) * (m32 + E0) * (1.0 + 1.01 * TIE_RTOL) + E0;
-      const double need = tier0_bound(f, c + 2.0 * E0);
-      if (need <= E0) break;
-      E0 = fmax(need, 1.5 * E0);
-    }
-    scut = c;
+  double E0 = tier0_bound(f, (1.0 + tol) * m32 * 1.01), c = 0.0;
+  for (int it = 0; it < 200; ++it) {
+    c = (1.0 + tol) * (m32 + E0) * (1.0 + 1.01 * TIE_RTOL) + E0;
+    const double need = tier0_bound(f, c + 2.0 * E0);
+    if (need <= E0) break;
+    E0 = fmax(need, 1.5 * E0);
   }
-  __syncthreads();
-  const double cut = scut;
-  int64_t below = 0;
-  const int64_t n0 = band_collect(s, D, P, -1.0, cut, cand, below);
+  return c;
+}
+
+__device__ __noinline__ int64_t thr_refined(Smem& s, const Ref& f, const float* __restrict__ D, int64_t P,
+                               double m32, double tol, int32_t* cand, int64_t ncol, RefArr a,
+                               unsigned long long& ties) {
+  int64_t n0 = ncol;
+  if (ncol < 0) {
+    __shared__ double scut;
+    if (threadIdx.x == 0) scut = thr_cut(f, m32, tol);
+    __syncthreads();
+    int64_t below = 0;
+    n0 = band_collect(s, D, P, -1.0, scut, cand, below);
+  }
   ref_init(f, cand, n0, a);
   // First with the minimum's interval instead of its value: entries that may hold the minimum are
   // raised to level 2 (an interval of 1e-13), and the threshold is an interval. Where that decides
@@ -1718,10 +1727,23 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
     have0 = naux == 0 && can_ref && ref_on(tk.x0) && __uint_as_float(mm[0]) < __int_as_float(0x7F800000);
   } else if (naux == 0) {
     const float mn = __uint_as_float(mm[0]);
+    // positions collected by thr_collect_kernel, in any order: sorted here
+    int64_t ncol = a.thr_n ? a.thr_n[b] : -1;
+    if (ncol > SORT_CAP) ncol = -1;
+    if (ncol >= 0) {
+      for (int i = threadIdx.x; i < ncol; i += PT) sbuf[i] = (unsigned long long)(uint32_t)cand[i];
+      __syncthreads();
+      bitonic_sort(sbuf, (int)ncol);
+      for (int i = threadIdx.x; i < ncol; i += PT) cand[i] = (int32_t)sbuf[i];
+      __syncthreads();
+    }
     if (can_ref && ref_on(tk.x0) && mn < __int_as_float(0x7F800000)) {
       const Ref f0 = make_ref(tk.x0, r, a.dx, a.dxy);
-      n = thr_refined(s, f0, D, P, (double)mn, a.tol, cand, ra, ties);
+      n = thr_refined(s, f0, D, P, (double)mn, a.tol, cand, ncol, ra, ties);
       have0 = true;
+    } else if (ncol >= 0) {
+      n = ncol;
+      ties += (unsigned long long)a.thr_ties[b];
     } else {
       const double thr = __dmul_rn(__dadd_rn(1.0, a.tol), (double)mn);
       ThrPred pr(D, thr, true);
@@ -1990,6 +2012,58 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
   }
 }
 
+// Positions of a threshold pick's map that can matter (D <= the threshold of an exact map; up to
+// thr_cut of one with an error bound), appended to cand in any order by CTAs that share the map, and
+// the near-ties of an exact map. A pick's one CTA took 1.1 ms for a map of 5.7 M positions (16-64 of
+// them on 152 SMs, one pass at 20 GB/s each); this pass reads the maps at the chip's bandwidth.
+constexpr int TC_NT = 256, TC_ITEMS = 8;
+
+__global__ void __launch_bounds__(TC_NT) thr_collect_kernel(const PickArgs a) {
+  const int b = blockIdx.x, r = b % a.nreal;
+  const PickTask& tk = a.tasks ? a.tasks[b / a.nreal] : a.t0;
+  if (tk.pre || tk.naux > 0) return;
+  const float* D = tk.D0 + r * tk.D0_rs;
+  const float mn = __uint_as_float((tk.mm0 + r * tk.mm0_rs)[0]);
+  __shared__ float s_hi, s_tlo, s_thi;
+  if (threadIdx.x == 0) {
+    s_tlo = 1.f;
+    s_thi = 0.f;
+    if (a.rv && ref_on(tk.x0) && mn < __int_as_float(0x7F800000)) {
+      s_hi = f_dn(thr_cut(make_ref(tk.x0, r, a.dx, a.dxy), (double)mn, a.tol));
+    } else {
+      const double t = __dmul_rn(__dadd_rn(1.0, a.tol), (double)mn);
+      s_hi = f_dn(t);
+      if (t > 0.0 && t < 1e300) tie_window_f(t, __dmul_rn(TIE_RTOL, t), s_tlo, s_thi);
+    }
+  }
+  __syncthreads();
+  const float hi = s_hi, tlo = s_tlo, thi = s_thi;
+  int32_t* cand = a.cand + (int64_t)b * a.P;
+  const int lane = threadIdx.x & 31;
+  int nt = 0;
+  const int64_t step = (int64_t)gridDim.y * TC_NT * TC_ITEMS;
+  for (int64_t t0 = (int64_t)blockIdx.y * TC_NT * TC_ITEMS; t0 < a.P; t0 += step) {
+    const int64_t p0 = t0 + (threadIdx.x >> 5) * (32 * TC_ITEMS) + lane;
+    float v[TC_ITEMS];
+    // (NaN past the end: compares false)
+#pragma unroll
+    for (int i = 0; i < TC_ITEMS; ++i) v[i] = p0 + 32 * i < a.P ? __ldg(D + p0 + 32 * i) : __int_as_float(0x7FC00000);
+#pragma unroll
+    for (int i = 0; i < TC_ITEMS; ++i) {
+      if (v[i] >= tlo && v[i] <= thi) nt++;
+      const bool in = v[i] <= hi;
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (!m) continue;
+      int at = 0;
+      if (lane == 0) at = atomicAdd(a.thr_n + b, __popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (in) cand[at + __popc(m & lanemask_lt())] = (int32_t)(p0 + 32 * i);
+    }
+  }
+  nt = __reduce_add_sync(0xffffffffu, nt);
+  if (lane == 0 && nt) atomicAdd(a.thr_ties + b, nt);
+}
+
 // Level-1 distances of every pick's candidates to every refined source of its task, between the
 // two phases of pick_kernel: a CTA evaluates EV_CH candidates of one (pick, source). A pick's ~700
 // candidates x 2-3 sources x ~5,500 terms dominated its single CTA (one of 16-80 in a launch, on as
@@ -2105,6 +2179,20 @@ int iq_launch_pick(iq_ctx* ctx, const PickLaunch& L) {
   // candidates, weights. (Without auxiliary sources the threshold pick evaluates its candidates
   // itself, to find the threshold.)
   const bool split = L.lvl1 && L.rv && L.ncand && naux > 0 && L.maxK > 0 && L.maxK <= REF_CACHE;
+  // maps large enough that one CTA's pass over them shows beside another launch
+  a.thr_n = a.thr_ties = nullptr;
+  if (L.thr && L.tasks && L.any_thr && L.P >= IQ_THR_MIN) {
+    a.thr_n = L.thr;
+    a.thr_ties = L.thr + nblocks;
+    IQ_CUDA_OK(cudaMemsetAsync(L.thr, 0, sizeof(int) * 2 * nblocks, ctx->stream));
+    const int64_t tiles = (L.P + TC_NT * TC_ITEMS - 1) / (TC_NT * TC_ITEMS);
+    const int64_t ny = std::max<int64_t>(1, std::min<int64_t>(tiles, 152 * 8 / std::min(nblocks, 152 * 8)));
+    iq_timer_start(ctx, "pick");
+    thr_collect_kernel<<<dim3((unsigned)nblocks, (unsigned)ny), TC_NT, 0, ctx->stream>>>(a);
+    iq_timer_stop(ctx, "pick", 0);
+    iq_count(ctx);
+    IQ_CUDA_OK(cudaGetLastError());
+  }
   a.phase = split ? 1 : 0;
   a.lvl1 = L.lvl1;
   a.nsrc = naux + 1;

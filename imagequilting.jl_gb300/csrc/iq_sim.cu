@@ -579,6 +579,8 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   uint8_t* d_rl = need_ref ? (uint8_t*)iq_scratch(ctx, S_PICK_RL, 2 * pk) : nullptr;
   float* d_lvl1 = lvl1_per ? (float*)iq_scratch(ctx, S_LVL1, sizeof(float) * lvl1_per * cmax) : nullptr;
   if (lvl1_per && !d_lvl1) return IQ_ERR_ALLOC;
+  int* d_thr = (int*)iq_scratch(ctx, S_THR, sizeof(int) * 2 * R * cmax);
+  if (!d_thr) return IQ_ERR_ALLOC;
   int64_t* d_rind = (int64_t*)iq_scratch(ctx, S_RIND, sizeof(int64_t) * R * cmax);
   int64_t* d_ncand = (int64_t*)iq_scratch(ctx, S_NCAND, sizeof(int64_t) * R * cmax);
   uint8_t* d_cutbuf = (uint8_t*)iq_scratch(ctx, S_CUTBUF, (size_t)R * cmax * 6 * slabmax);
@@ -1327,6 +1329,9 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
         L.rl = d_rl ? d_rl + 2 * po : nullptr;
         L.dx = distD.x; L.dxy = distD.x * distD.y;
         L.lvl1 = d_lvl1 ? d_lvl1 + grp_rind(grp) * (naux_most + 1) * IQ_RANK_CAP : nullptr;
+        L.thr = d_thr + grp_rind(grp) * 2;
+        for (int i = 0; i < m; ++i)
+          L.any_thr = L.any_thr || (nsoft == 0 && !steps[k0 + i].hardtile && !predrawn(steps[k0 + i]));
         L.maxK = (int)(nsoft > 0 ? T : maxK);  // (hard masks hold at most a tile's offsets too)
         if (chard[c]) L.maxK = (int)T;
         L.ties = ctx->d_ties;
