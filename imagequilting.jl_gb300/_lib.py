@@ -19,6 +19,7 @@ IQ_ERR_STATE = 6
 IQ_ERR_LIMIT = 7
 IQ_F32 = 0
 IQ_F64 = 1
+IQ_ROWMAJOR = 0x100
 PATHS = {"raster": 0, "dilation": 1, "random": 2}
 
 c_i64p = ctypes.POINTER(ctypes.c_int64)

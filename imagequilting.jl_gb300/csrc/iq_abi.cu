@@ -331,6 +331,8 @@ static int read_dims(int32_t ndim, const int64_t* size, Dim3& d) {
 extern "C" int iq_set_ti(iq_ctx* ctx, const void* ti, int32_t dtype, int32_t ndim,
                          const int64_t* size) {
   if (!ctx || !ti) return iq_set_error(IQ_ERR_ARG, "null argument");
+  const bool rowmajor = (dtype & IQ_ROWMAJOR) != 0;
+  dtype &= ~IQ_ROWMAJOR;
   if (dtype != IQ_F32 && dtype != IQ_F64) return iq_set_error(IQ_ERR_ARG, "dtype must be F32 or F64");
   Dim3 d;
   int rc = read_dims(ndim, size, d);
@@ -354,7 +356,13 @@ extern "C" int iq_set_ti(iq_ctx* ctx, const void* ti, int32_t dtype, int32_t ndi
   ctx->has_ti = false;
   uint8_t* nanm = (uint8_t*)iq_scratch(ctx, S_TMP0, (size_t)n);
   if (!nanm) return IQ_ERR_ALLOC;
-  if (dtype == IQ_F32) {
+  if (rowmajor && ndim > 1) {
+    const size_t eb = dtype == IQ_F32 ? sizeof(float) : sizeof(double);
+    void* tmp = iq_scratch(ctx, S_TMP1, eb * n);
+    if (!tmp) return IQ_ERR_ALLOC;
+    IQ_CUDA_OK(cudaMemcpyAsync(tmp, ti, eb * n, cudaMemcpyDefault, ctx->stream));
+    if ((rc = iq_launch_from_rowmajor(ctx, tmp, dtype == IQ_F64, d, ctx->d_ti))) return rc;
+  } else if (dtype == IQ_F32) {
     IQ_CUDA_OK(cudaMemcpyAsync(ctx->d_ti, ti, sizeof(float) * n, cudaMemcpyDefault, ctx->stream));
   } else {
     double* tmp = (double*)iq_scratch(ctx, S_TMP1, sizeof(double) * n);

@@ -85,7 +85,8 @@ struct iq_ctx {
   int corr_engine = 2;          // box-mask distances: 2 tensor cores FP16 halves when the data's
                                 // range allows (else TF32), 1 tensor cores TF32, 0 SIMT
   int64_t max_steps = -1;       // tiles simulated per realization (< 0: all)
-  int sim_streams = 1;          // realization groups of iq_simulate, each on its own stream
+  int sim_streams = 0;          // realization groups of iq_simulate, each on its own stream (0: by
+                                // whether the maps need the exact re-rank)
   cudaStream_t stream2 = nullptr;  // stream of the second realization group (made on first use)
   struct IqLp* lp = nullptr;       // learned proposal state (iq_proposal_host.cu)
   int lp_enable = 0;               // iq_simulate shortlists with the proposal where it applies
@@ -538,6 +539,8 @@ int iq_launch_pad_symmetric(iq_ctx* ctx, const float* src, Dim3 src_dims, float*
 int iq_launch_prepare(iq_ctx* ctx, float* data, int64_t n, uint8_t* nanmask,
                       unsigned long long* hash = nullptr);
 int iq_launch_to_f32(iq_ctx* ctx, const double* src, float* dst, int64_t n);
+// dst (column-major FP32) = src (row-major, FP32 or Float64) of extents d
+int iq_launch_from_rowmajor(iq_ctx* ctx, const void* src, bool f64, Dim3 d, float* dst);
 
 // ---------------------------------------------------------------------------------------
 // Learned proposal (iq_proposal.cu)

@@ -5,6 +5,8 @@
 //   crop            view(simgrid, CartesianIndices(simsize))      src/iqsim.jl:302-304
 //   soft padding    padarray(aux, Pad(:symmetric, 0, append))      src/utils.jl:74-79
 //   prepare         NaN -> 0                                       src/utils.jl:96-102
+#include <algorithm>
+
 #include "iq_internal.h"
 
 namespace {
@@ -130,6 +132,26 @@ __global__ void prepare_kernel(float* data, int64_t n, uint8_t* nanmask, unsigne
   }
 }
 
+// Row-major (x, y, z; z fastest) to column-major: 32 x 32 tiles of (x, (y, z)) through shared memory, so
+// that both sides are read and written in lines.
+template <typename T>
+__global__ void from_rowmajor_kernel(const T* __restrict__ src, Dim3 d, float* __restrict__ dst) {
+  __shared__ float t[32][33];
+  const int64_t rest = d.y * d.z, x0 = (int64_t)blockIdx.x * 32;
+  for (int64_t c0 = (int64_t)blockIdx.y * 32; c0 < rest; c0 += (int64_t)gridDim.y * 32) {
+    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
+      const int64_t x = x0 + i, c = c0 + threadIdx.x;
+      if (x < d.x && c < rest) t[i][threadIdx.x] = (float)src[x * rest + c];
+    }
+    __syncthreads();
+    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
+      const int64_t x = x0 + threadIdx.x, c = c0 + i;
+      if (x < d.x && c < rest) dst[x + d.x * (c / d.z + d.y * (c % d.z))] = t[threadIdx.x][i];
+    }
+    __syncthreads();
+  }
+}
+
 __global__ void to_f32_kernel(const double* src, float* dst, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
@@ -207,6 +229,16 @@ int iq_launch_pad_symmetric(iq_ctx* ctx, const float* src, Dim3 src_dims, float*
 int iq_launch_prepare(iq_ctx* ctx, float* data, int64_t n, uint8_t* nanmask,
                       unsigned long long* hash) {
   prepare_kernel<<<blocks_for(n), 256, 0, ctx->stream>>>(data, n, nanmask, hash);
+  iq_count(ctx);
+  IQ_CUDA_OK(cudaGetLastError());
+  return IQ_OK;
+}
+
+int iq_launch_from_rowmajor(iq_ctx* ctx, const void* src, bool f64, Dim3 d, float* dst) {
+  const dim3 grid((unsigned)((d.x + 31) / 32), (unsigned)std::min<int64_t>((d.y * d.z + 31) / 32, 65535)),
+      block(32, 8);
+  if (f64) from_rowmajor_kernel<<<grid, block, 0, ctx->stream>>>((const double*)src, d, dst);
+  else from_rowmajor_kernel<<<grid, block, 0, ctx->stream>>>((const float*)src, d, dst);
   iq_count(ctx);
   IQ_CUDA_OK(cudaGetLastError());
   return IQ_OK;

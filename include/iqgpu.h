@@ -36,6 +36,7 @@ extern "C" {
 
 #define IQ_F32 0
 #define IQ_F64 1
+#define IQ_ROWMAJOR 0x100 /* or'ed to the dtype of iq_set_ti: last dim fastest instead of dim 1 */
 
 #define IQ_PATH_RASTER 0
 #define IQ_PATH_DILATION 1
@@ -103,7 +104,8 @@ int iq_ties(iq_ctx* ctx, int64_t* out);
 /*
  * Upload the training image and keep it resident: prepare (src/utils.jl:96-102, NaN -> 0,
  * Float32 on the device like the reference's GPU path src/utils.jl:59), its NaN mask and the
- * Float64 integral image of its squares. dtype IQ_F32 or IQ_F64; NaN marks inactive voxels.
+ * Float64 integral image of its squares. dtype IQ_F32 or IQ_F64, or'ed with IQ_ROWMAJOR when the
+ * array is in C order (extents are given per dim either way); NaN marks inactive voxels.
  */
 int iq_set_ti(iq_ctx* ctx, const void* ti, int32_t dtype, int32_t ndim, const int64_t* size);
 
@@ -203,7 +205,8 @@ int64_t iq_ctx_launches(iq_ctx* ctx);
  *                         (tcgen05) with FP16 halves after a power-of-two scaling when every
  *                         nonzero magnitude lies within 2^17 of the largest, else TF32 halves;
  *                         1 tensor cores with TF32 halves; 0 the SIMT FP32 kernel
- *   "sim.streams"         1 (default) or 2: with 2, the tensor-core engine and nreal >= 2,
+ *   "sim.streams"         1 or 2 (default: 2 when the maps need the exact re-rank, else 1): with
+ *                         2, the tensor-core engine and nreal >= 2,
  *                         iq_simulate runs two groups of realizations on two streams so that
  *                         one group's pick and cut overlap the other's correlation (each
  *                         correlation launch then holds half the columns, which costs more
