@@ -255,10 +255,18 @@ __global__ void ii_scan_kernel(T* __restrict__ ii, int64_t sx, int64_t sy, int64
     if (axis == 0) base = l * sx;
     else if (axis == 1) base = (l % sx) + sx * sy * (l / sx);
     else base = l;
+    // 16 loads in flight ahead of their additions (one at a time, a line of 128 took 46 us); the sums
+    // stay in line order
     T run = 0;
-    for (int64_t i = 0; i < len; ++i) {
-      run += ii[base + i * step];
-      ii[base + i * step] = run;
+    for (int64_t i0 = 0; i0 < len; i0 += 16) {
+      T v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) v[u] = i0 + u < len ? ii[base + (i0 + u) * step] : (T)0;
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        run += v[u];
+        if (i0 + u < len) ii[base + (i0 + u) * step] = run;
+      }
     }
   }
 }

@@ -498,14 +498,21 @@ __device__ int64_t compact(Smem& s, const Pred& pred, int64_t P, int32_t* out) {
   return base;
 }
 
+// FP32 bounds of a threshold t of an exact map: b[0] its membership test, b[1], b[2] its near-ties. One
+// thread computes them (the Float64 steps of 1,024 would take 16 k cycles of the Float64 pipe).
+__device__ __forceinline__ void thr_bounds(double t, float* b) {
+  b[0] = f_dn(t);
+  b[1] = 1.f;
+  b[2] = 0.f;
+  if (t > 0.0 && t < 1e300) tie_window_f(t, __dmul_rn(TIE_RTOL, t), b[1], b[2]);
+}
+
 struct ThrPred {
   const float* D;
   float thr;                          // f_dn of the Float64 threshold
   float tlo, thi;                     // near-ties |D - thr| <= 1e-6 thr (Float64): tlo <= D <= thi
   mutable unsigned long long nt = 0;  // this thread's near-ties
-  __device__ ThrPred(const float* d, double t, bool ties) : D(d), thr(f_dn(t)), tlo(1.f), thi(0.f) {
-    if (ties && t > 0.0 && t < 1e300) tie_window_f(t, __dmul_rn(TIE_RTOL, t), tlo, thi);
-  }
+  __device__ ThrPred(const float* d, const float* b) : D(d), thr(b[0]), tlo(b[1]), thi(b[2]) {}
   // bit i set when D[p0 + 32 * i] <= thr (positions past P excluded)
   __device__ uint32_t eval8(int64_t p0, int64_t P) const {
     float v[CITEMS];
@@ -1452,9 +1459,12 @@ __device__ __noinline__ long long band_topk(Smem& s, unsigned long long* sbuf, c
 __device__ __noinline__ unsigned long long count_near(Smem& s, const float* __restrict__ src, int64_t P,
                                          double t) {
   unsigned long long c = 0;
+  __shared__ float nb[3];
+  __syncthreads();  // an earlier call's readers are done
+  if (threadIdx.x == 0) thr_bounds(t, nb);
+  __syncthreads();
   if (t > 0.0 && t < 1e300) {
-    float lo, hi;
-    tie_window_f(t, __dmul_rn(TIE_RTOL, t), lo, hi);
+    const float lo = nb[1], hi = nb[2];
     for (int64_t p = threadIdx.x; p < P; p += PT) {
       const float d = src[p];
       if (d >= lo && d <= hi && d < __int_as_float(0x7F800000)) c++;
@@ -1745,8 +1755,10 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
       n = ncol;
       ties += (unsigned long long)a.thr_ties[b];
     } else {
-      const double thr = __dmul_rn(__dadd_rn(1.0, a.tol), (double)mn);
-      ThrPred pr(D, thr, true);
+      __shared__ float tb[3];
+      if (threadIdx.x == 0) thr_bounds(__dmul_rn(__dadd_rn(1.0, a.tol), (double)mn), tb);
+      __syncthreads();
+      ThrPred pr(D, tb);
       n = compact(s, pr, P, cand);
       ties += block_sum_u64(s, pr.nt);
     }
@@ -1947,8 +1959,13 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
     return;
   }
   const double dn = (double)n;
-  const double inv_n = __ddiv_rn(1.0, dn);
-  const double x0 = __ddiv_rn(__dsub_rn(1.0, inv_n), inv_n);
+  __shared__ double sx0;
+  if (threadIdx.x == 0) {  // (one thread: two Float64 divisions)
+    const double inv_n = __ddiv_rn(1.0, dn);
+    sx0 = __ddiv_rn(__dsub_rn(1.0, inv_n), inv_n);
+  }
+  __syncthreads();
+  const double x0 = sx0;
   for (int64_t i = threadIdx.x; i < n; i += PT) prod[i] = 1.0;
 #pragma unroll 1
   for (int j = 0; j <= naux; ++j) {
@@ -1983,31 +2000,45 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
     for (int l = 1; l < 4; ++l) atomicAdd(a.stats + ST_PICK_EV1 + l - 1, (unsigned long long)evc[l]);
   }
   // ---- weighted draw ----
+  // Chunk sums left to right, then the chunk totals left to right. The running sums of every chunk stay
+  // in `prod`, so that the walk through the drawn chunk compares them at once instead of adding again;
+  // the last place of a chunk then takes the total up to it.
   const int64_t nch = (n + IQ_DRAW_CHUNK - 1) / IQ_DRAW_CHUNK;
-  double* csum = prod;  // reuse
   for (int64_t c = threadIdx.x; c < nch; c += PT) {
     double run = 0.0;
     const int64_t lo = c * IQ_DRAW_CHUNK, hi = min(n, lo + IQ_DRAW_CHUNK);
-    for (int64_t i = lo; i < hi; ++i) run = __dadd_rn(run, w[i]);
-    csum[c] = run;
+#pragma unroll 8
+    for (int64_t i = lo; i < hi; ++i) {
+      run = __dadd_rn(run, w[i]);
+      prod[i] = run;
+    }
   }
   __syncthreads();
+  __shared__ double sdt, sdb;
+  __shared__ int64_t sdc;
+  __shared__ int sdp;
   if (threadIdx.x == 0) {
+    auto last = [&](int64_t c) { return min(n, (c + 1) * IQ_DRAW_CHUNK) - 1; };
     double run = 0.0;
-    for (int64_t c = 0; c < nch; ++c) { run = __dadd_rn(run, csum[c]); csum[c] = run; }
+    for (int64_t c = 0; c < nch; ++c) { run = __dadd_rn(run, prod[last(c)]); prod[last(c)] = run; }
     const double u = iq_draw_uniform(a.seed, tk.tile, a.real0 + r);
     const double t = __dmul_rn(u, run);
     int64_t c = 0;
-    while (c < nch - 1 && csum[c] < t) ++c;
-    const double base = c == 0 ? 0.0 : csum[c - 1];
-    const int64_t lo = c * IQ_DRAW_CHUNK, hi = min(n, lo + IQ_DRAW_CHUNK);
-    double part = 0.0;
-    int64_t pick = hi - 1;
-    for (int64_t i = lo; i < hi; ++i) {
-      part = __dadd_rn(part, w[i]);
-      if (__dadd_rn(base, part) >= t) { pick = i; break; }
-    }
-    a.rind[b] = cand[pick];
+    while (c < nch - 1 && prod[last(c)] < t) ++c;
+    sdt = t;
+    sdb = c == 0 ? 0.0 : prod[last(c - 1)];
+    sdc = c;
+    sdp = IQ_DRAW_CHUNK;
+  }
+  __syncthreads();
+  // the first entry of the chunk whose running sum reaches t (the last one when none does)
+  const int64_t dlo = sdc * IQ_DRAW_CHUNK, dhi = min(n, dlo + IQ_DRAW_CHUNK);
+  const int64_t di = dlo + threadIdx.x;
+  if (threadIdx.x < IQ_DRAW_CHUNK && di + 1 < dhi && __dadd_rn(sdb, prod[di]) >= sdt)
+    atomicMin(&sdp, (int)threadIdx.x);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    a.rind[b] = cand[sdp < IQ_DRAW_CHUNK ? dlo + sdp : dhi - 1];
     if (prof) atomicAdd(a.stats + ST_PICK_TDRAW, (unsigned long long)(clock64() - t2));
   }
 }

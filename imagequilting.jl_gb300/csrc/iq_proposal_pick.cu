@@ -123,6 +123,8 @@ __global__ void __launch_bounds__(LP_PT) lp_pick_kernel(const LpPickArgs a) {
   __shared__ float red[32];
   __shared__ unsigned long long ured[32];
   __shared__ int sflag;
+  __shared__ float stie[3];
+  __shared__ double sx0;
   const int c = blockIdx.x;
   const LpColumn col = a.cols[c];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -145,16 +147,19 @@ __global__ void __launch_bounds__(LP_PT) lp_pick_kernel(const LpPickArgs a) {
     for (int i = 1; i < LP_PT / 32; ++i) mm = fminf(mm, red[i]);
     red[0] = mm;
     sflag = 0;
+    // (one thread: Float64 steps of 1,024 threads take the narrow pipe 16 k cycles)
+    const double thr = __dmul_rn(__dadd_rn(1.0, a.tol), (double)mm);
+    // the Float64 tests d <= thr and |d - thr| <= 1e-6 thr as FP32 comparisons
+    stie[0] = f_dn(thr);
+    stie[1] = 1.f;
+    stie[2] = 0.f;
+    if (thr > 0.0 && thr < 1e300) tie_window_f(thr, __dmul_rn(1e-6, thr), stie[1], stie[2]);
   }
   __syncthreads();
-  const double thr = __dmul_rn(__dadd_rn(1.0, a.tol), (double)red[0]);
   // candidates (position, value) and near-ties
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(dyn);
   unsigned long long nt = 0;
-  // the Float64 tests d <= thr and |d - thr| <= 1e-6 thr as FP32 comparisons
-  const float thr_f = f_dn(thr);
-  float tlo = 1.f, thi = 0.f;
-  if (thr > 0.0 && thr < 1e300) tie_window_f(thr, __dmul_rn(1e-6, thr), tlo, thi);
+  const float thr_f = stie[0], tlo = stie[1], thi = stie[2];
   for (int i = threadIdx.x; i < n; i += LP_PT) {
     const float d = dl[i];
     if (d >= tlo && d <= thi) nt++;
@@ -201,13 +206,14 @@ __global__ void __launch_bounds__(LP_PT) lp_pick_kernel(const LpPickArgs a) {
       S += (unsigned long long)(nc - r + 1);
     }
     ured[0] = S;
+    const double inv_n = __ddiv_rn(1.0, (double)nc);
+    sx0 = __ddiv_rn(__dsub_rn(1.0, inv_n), inv_n);
   }
   __syncthreads();
   // tau model with one source, the arithmetic of the full pick: P = (n - r + 1) / S,
   // X = (1 - P) / P, x = x0 * (1 * X / x0), p = 1 / (1 + x)
   const double dS = (double)ured[0];
-  const double inv_n = __ddiv_rn(1.0, (double)nc);
-  const double x0 = __ddiv_rn(__dsub_rn(1.0, inv_n), inv_n);
+  const double x0 = sx0;
   for (int i = threadIdx.x; i < nc; i += LP_PT) {
     const double Pi = __ddiv_rn((double)(nc - (int64_t)rank[i] + 1), dS);
     const double X = __ddiv_rn(__dsub_rn(1.0, Pi), Pi);
