@@ -513,6 +513,12 @@ extern "C" int iq_fastdistance(iq_ctx* ctx, const int64_t* tilesize, int32_t ntm
       if (!d_st || !d_cols || !d_B) return IQ_ERR_ALLOC;
       IQ_CUDA_OK(cudaMemcpyAsync(d_st, stw.data(), sizeof(uint32_t) * stw.size(), cudaMemcpyHostToDevice, ctx->stream));
       IQ_CUDA_OK(cudaMemcpyAsync(d_cols, cols.data(), sizeof(TcCol) * cols.size(), cudaMemcpyHostToDevice, ctx->stream));
+      void* img16 = nullptr;
+      if (ctx->corr_engine == 2 && ctx->ti_stats.fp16_range()) {
+        img16 = iq_scratch(ctx, S_TZ_IMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * 4);
+        if (!img16) return IQ_ERR_ALLOC;
+        if ((rc = iq_tz_image(ctx, ctx->d_ti, ctx->ti, ctx->ti_stats, true, img16))) return rc;
+      }
       size_t col0 = 0;
       for (int32_t c0 = 0; c0 < ntmpl; c0 += IQ_TC_MAXN) {
         const int nb = std::min<int32_t>(IQ_TC_MAXN, ntmpl - c0);
@@ -523,7 +529,7 @@ extern "C" int iq_fastdistance(iq_ctx* ctx, const int64_t* tilesize, int32_t ntm
         L.stage_word = d_st; L.stage_prefix = d_st + ns; L.nstage = (int)ns; L.nsteps = stg.nsteps;
         L.stage16 = d_st + 2 * ns; L.nstage16 = (int)n16; L.nsteps16 = stg.nsteps16;
         L.grid = d_tmpl; L.grid_dims = t; L.cols = d_cols + col0; L.N = (nb + 15) / 16 * 16;
-        L.B = d_B; L.img_stats = ctx->ti_stats; L.tmpl_stats = tstats;
+        L.B = d_B; L.img_stats = ctx->ti_stats; L.tmpl_stats = tstats; L.img16 = img16;
         L.flops = 2.0 * (double)P * (double)K * nb;
         if ((rc = iq_launch_corr_tc(ctx, L))) return rc;
         col0 += L.N;

@@ -14,7 +14,12 @@
 // 128 and stride (M) byte offset 256, and advancing K by 8 offsets moves the start address by
 // 256 bytes. The CTA's threads build the image from TI values they load one stage ahead
 // (L2-resident rows); positions whose x lies past the valid extent are computed and dropped
-// (a linear run wraps rows).
+// (a linear run wraps rows). The FP16 form (8 values to an image row) reads the image that
+// iq_tz_image split into FP16 halves once per call, its rows padded to 8 values: an image row is
+// then five aligned words of each half and a funnel shift, where splitting in place took eight
+// loads and 32 conversions for every row of every stage of every CTA (with the chunk offsets of a
+// K-step taken bit by bit instead of searched: 16 templates of 24x24x12 over 100x100x50, 1.06 ->
+// 0.81 ms a call; at 16 columns the images of the three stages, not the MMAs, bind).
 //
 // B operand. tc_pack_kernel packs the templates per stage into the core-matrix layout (the
 // TF32 high halves of all the stage's K-steps, then the low halves; per K-step: offset block
@@ -75,12 +80,16 @@ template <bool F16> constexpr int stage_units() { return F16 ? 2 * F_ROWU : 8 * 
 template <bool F16> constexpr int upt() {
   return (stage_units<F16>() + TC_PTHREADS - 1) / TC_PTHREADS;  // image rows per thread
 }
-template <bool F16> constexpr int vpu() { return F16 ? 8 : 4; }  // values per image row
+// words a thread holds per image row: TF32 -> its 4 values; FP16 -> the 5 words that hold its 8 high
+// halves at either parity, then the 5 of the low halves
+template <bool F16> constexpr int vpu() { return F16 ? 10 : 4; }
 
 struct TcArgs {
   const float* img;
+  const __half *hi, *lo;   // FP16 form: the image's halves (iq_tz_image)
   int64_t ix, iy, nimg;
-  int64_t dx, dy, dz, Lp;  // valid extents; Lp = (dy - 1) * ix + dx linear span of a plane
+  int64_t lx;              // row pitch of the linear positions: ix, or padded to 8 (FP16 form)
+  int64_t dx, dy, dz, Lp;  // valid extents; Lp = (dy - 1) * lx + dx linear span of a plane
   int bpp;                 // CTAs per z-plane
   int64_t tx, ty, tz;
   const double* ii;
@@ -95,7 +104,6 @@ struct TcArgs {
   const TcCol* cols;
   int N;
   int exact;
-  float scale_a;              // FP16 form: 2^-kA applied to the image values
   float ab2;                  // 2 * 2^(kA + kB): D = |A2 + B2 - ab2 * acc|
   uint32_t tmem_cols;
   int* status;
@@ -221,7 +229,7 @@ __device__ __forceinline__ uint32_t stage_pre(const TcArgs& a, const uint32_t* s
 
 __device__ __forceinline__ int64_t row_e0(const TcArgs& a, uint32_t w, int64_t p0) {
   const int ky = (int)(w & 1023u), kz = (int)((w >> 10) & 1023u), g = (int)((w >> 20) & 63u);
-  return p0 + (int64_t)TC_GROUP * g + a.ix * (ky + a.iy * (int64_t)kz);
+  return p0 + (int64_t)TC_GROUP * g + a.lx * (ky + a.iy * (int64_t)kz);
 }
 
 // K-steps of a stage: TF32 -> one per active 8-offset step; FP16 -> the active 8-offset
@@ -267,24 +275,35 @@ __device__ __forceinline__ int64_t unit_base(const StageInfo& s, int u) {
 
 template <bool F16>
 __device__ __forceinline__ void stage_load(const TcArgs& a, const StageInfo& s, int ptid,
-                                           float (&v)[upt<F16>()][vpu<F16>()]) {
+                                           uint32_t (&v)[upt<F16>()][vpu<F16>()]) {
 #pragma unroll
   for (int i = 0; i < upt<F16>(); ++i) {
     const int u = ptid + i * TC_PTHREADS;
     if (u < s.nunits) {
       const int64_t base = unit_base<F16>(s, u);
+      if (F16) {
+        // (a stage's first position is a multiple of 8, so an image row's parity is its number's)
+        const uint32_t* ph = reinterpret_cast<const uint32_t*>(a.hi + (base & ~(int64_t)1));
+        const uint32_t* pl = reinterpret_cast<const uint32_t*>(a.lo + (base & ~(int64_t)1));
 #pragma unroll
-      for (int c = 0; c < vpu<F16>(); ++c) v[i][c] = __ldg(a.img + min(base + c, a.nimg - 1));
+        for (int c = 0; c < 5; ++c) v[i][c] = __ldg(ph + c);
+        if (!a.exact) {
+#pragma unroll
+          for (int c = 0; c < 5; ++c) v[i][5 % vpu<F16>() + c] = __ldg(pl + c);
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[i][c] = __float_as_uint(__ldg(a.img + min(base + c, a.nimg - 1)));
+      }
     }
   }
 }
 
-// chunk idx of an FP16 stage: byte offset of its core-matrix column inside the A hi region
+// first chunk of `left` (not 0): byte offset of its core-matrix column inside the A hi region
 // (row entry a at 0, row entry b at F_IMG; chunk c is c blocks further)
-__device__ __forceinline__ uint32_t f16_chunk_off(uint32_t ma, uint32_t mb, int idx) {
-  const int na = __popc(ma);
-  return idx < na ? 128u * (uint32_t)nth_bit(ma, idx)
-                  : (uint32_t)F_IMG + 128u * (uint32_t)nth_bit(mb, idx - na);
+__device__ __forceinline__ uint32_t f16_chunk_off(uint32_t left) {
+  const uint32_t i = (uint32_t)__ffs((int)left) - 1u;
+  return 128u * i + (i < F_CH ? 0u : (uint32_t)(F_IMG - 128 * F_CH));
 }
 
 template <bool F16>
@@ -344,7 +363,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_tc_kernel(const TcArgs a) 
   const uint32_t tmem = s_tmem;
 
   const int64_t z = blockIdx.x / a.bpp;
-  const int64_t zbase = z * a.ix * a.iy;
+  const int64_t zbase = z * a.lx * a.iy;
   const int64_t p0 = zbase + (int64_t)(blockIdx.x % a.bpp) * (128 * TC_MB);
   const uint32_t sbase = smem_u32(smem);
   // D F32; A, B: TF32 (2) or F16 (0); N >> 3 at bit 17, M >> 4 at bit 24
@@ -384,25 +403,28 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_tc_kernel(const TcArgs a) 
         const uint64_t dB = dB0 + (uint64_t)(b * dbuf);
         uint32_t acc = e > 0 ? 1u : 0u;
         if (F16) {
-          const int total = __popc(ma) + __popc(mb2);
+          // active chunks of both row entries, lowest first: bit i < F_CH is row entry a's chunk i
+          uint32_t left = ma | (mb2 << F_CH);
+          const uint64_t dA = make_desc(sA, 0u, 128u);
 #pragma unroll
           for (int t = 0; t < TC_STEPS; ++t) {
             if (t < (int)nks) {
               const uint64_t bh = dB + (uint64_t)(t * dstep), bl = dB + (uint64_t)((nks + t) * dstep);
               // two 8-offset chunks X, Y: the descriptor's leading offset joins them (the
               // unused half of an odd last K-step reads the next block, its B half is zero)
-              const uint32_t ox = f16_chunk_off(ma, mb2, 2 * t);
-              const uint32_t lbo = 2 * t + 1 < total ? f16_chunk_off(ma, mb2, 2 * t + 1) - ox : 128u;
+              const uint32_t ox = f16_chunk_off(left);
+              left &= left - 1;
+              const uint32_t lbo = left ? f16_chunk_off(left) - ox : 128u;
+              left &= left - 1;
+              const uint64_t dX = dA + (ox >> 4) + ((uint64_t)(lbo >> 4) << 16);
 #pragma unroll
               for (int mb = 0; mb < TC_MB; ++mb) {
-                const uint32_t ao = ox + 128u * 16u * mb;
                 const uint32_t d = tmem + (uint32_t)(mb * N);
-                const uint64_t dah = make_desc(sA + ao, lbo, 128u);
+                const uint64_t dah = dX + 8u * 16u * mb;
                 mma_f16(d, dah, bh, idesc, acc);
                 if (!a.exact) {
-                  const uint64_t dal = make_desc(sA + 2 * F_IMG + ao, lbo, 128u);
                   mma_f16(d, dah, bl, idesc, 1u);
-                  mma_f16(d, dal, bh, idesc, 1u);
+                  mma_f16(d, dah + 2 * F_IMG / 16, bh, idesc, 1u);
                 }
               }
               acc = 1u;
@@ -455,7 +477,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_tc_kernel(const TcArgs a) 
   } else {
     // ---- A images (TI values loaded two stages ahead, in two register sets) ----
     const int ptid = tid - 32;
-    float va[UPT][VPU], vb[UPT][VPU];
+    uint32_t va[UPT][VPU], vb[UPT][VPU];
     StageInfo sa{}, sbi{};
     if (a.nstage > 0) {
       sa = stage_info<F16>(a, s_stage, 0, p0);
@@ -471,7 +493,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_tc_kernel(const TcArgs a) 
     // write stage e's images from v; false when the wait for the buffer gave up
     const bool copier = warp == 1 && lane == 0;  // issues the B copies
     int ncopied = 0;
-    auto build = [&](int e, const StageInfo& si, float (&v)[UPT][VPU]) -> bool {
+    auto build = [&](int e, const StageInfo& si, uint32_t (&v)[UPT][VPU]) -> bool {
       const int b = e % TC_NST;
       const uint32_t use = (uint32_t)(e / TC_NST);
       const bool ok = use == 0 || mbar_wait_t(bar_done + 8 * b, (use - 1) & 1u, prof, t_wait);
@@ -488,14 +510,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_tc_kernel(const TcArgs a) 
         const int u = ptid + i * TC_PTHREADS;
         if (u < si.nunits) {
           if (F16) {
+            const uint32_t sh = 16u * (uint32_t)(u & 1);
             uint32_t h[4], l[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-              uint16_t h0, l0, h1, l1;
-              f16_split(v[i][2 * c], a.scale_a, h0, l0);
-              f16_split(v[i][2 * c + 1], a.scale_a, h1, l1);
-              h[c] = (uint32_t)h0 | ((uint32_t)h1 << 16);
-              l[c] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+              h[c] = __funnelshift_r(v[i][c], v[i][c + 1], sh);
+              l[c] = __funnelshift_r(v[i][(5 + c) % VPU], v[i][(6 + c) % VPU], sh);
             }
             const bool second = u >= F_ROWU;
             const uint32_t off = (second ? (uint32_t)F_IMG : 0u) + 16u * (uint32_t)(second ? u - F_ROWU : u);
@@ -504,7 +524,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_tc_kernel(const TcArgs a) 
           } else {
             uint32_t h[4], l[4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) tf32_split(v[i][c], h[c], l[c]);
+            for (int c = 0; c < 4; ++c) tf32_split(__uint_as_float(v[i][c]), h[c], l[c]);
             st_shared_v4(sA + 16u * u, h[0], h[1], h[2], h[3]);
             if (!a.exact) st_shared_v4(sA + TC_NQ * 128u + 16u * u, l[0], l[1], l[2], l[3]);
           }
@@ -549,7 +569,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_tc_kernel(const TcArgs a) 
     for (int mb = 0; mb < TC_MB; ++mb) {
       const int m = 128 * mb + 32 * lq + lane;
       const int64_t rel = p0 + m - zbase;
-      const int64_t x = rel % a.ix, y = rel / a.ix;
+      const int64_t x = rel % a.lx, y = rel / a.lx;
       const bool valid = rel < a.Lp && x < a.dx;
       double full = 0.0;
       if (valid) full = iq_box_sum(a.ii, sx, sxy, x, y, z, a.tx, a.ty, a.tz);
@@ -567,7 +587,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) corr_tc_kernel(const TcArgs a) 
     for (int mb = 0; mb < TC_MB; ++mb) {
       const int m = 128 * mb + 32 * lq + lane;
       const int64_t rel = p0 + m - zbase;
-      const int64_t x = rel % a.ix, y = rel / a.ix;
+      const int64_t x = rel % a.lx, y = rel / a.lx;
       const bool valid = rel < a.Lp && x < a.dx;
       const int64_t pout = valid ? x + a.dx * (y + a.dy * z) : 0;
       const bool dis = valid && a.disabled != nullptr && a.disabled[pout];
@@ -887,9 +907,13 @@ int iq_launch_corr_tc(iq_ctx* ctx, const TcCorrLaunch& L) {
   a.img = L.img;
   a.ix = L.img_dims.x;
   a.iy = L.img_dims.y;
+  a.lx = f16 ? (a.ix + 7) / 8 * 8 : a.ix;
+  a.hi = (const __half*)L.img16;
+  a.lo = a.hi + (iq_tz_image_halves(L.img_dims) + 63) / 64 * 64;
+  if (f16 && !L.img16) return iq_set_error(IQ_ERR_ARG, "tensor-core correlation: no FP16 image");
   a.nimg = L.img_dims.vol();
   a.dx = od.x; a.dy = od.y; a.dz = od.z;
-  a.Lp = (od.y - 1) * a.ix + od.x;
+  a.Lp = (od.y - 1) * a.lx + od.x;
   const int64_t bpp = (a.Lp + 128 * TC_MB - 1) / (128 * TC_MB);
   a.bpp = (int)bpp;
   a.tx = L.tile.x; a.ty = L.tile.y; a.tz = L.tile.z;
@@ -913,7 +937,6 @@ int iq_launch_corr_tc(iq_ctx* ctx, const TcCorrLaunch& L) {
   a.cols = L.cols;
   a.N = L.N;
   a.exact = exact ? 1 : 0;
-  a.scale_a = std::ldexp(1.f, -ka);
   a.ab2 = std::ldexp(1.f, ka + kb + 1);
   uint32_t tc = 32;
   while (tc < (uint32_t)(TC_MB * L.N)) tc <<= 1;

@@ -278,6 +278,7 @@ struct TcCorrLaunch {
   const TcCol* cols = nullptr;          // device array of N columns
   int N = 0;                            // multiple of 16, at most 256
   void* B = nullptr;                    // packed templates, max(nsteps, nsteps16) * 64 * N bytes
+  const void* img16 = nullptr;          // FP16 form: the image's halves (iq_tz_image, split)
   IqValueStats img_stats, tmpl_stats;   // ranges of the image and of the templates
   double flops = 0;                     // algorithmic FLOPs (profiling)
 };

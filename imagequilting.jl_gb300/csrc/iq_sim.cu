@@ -768,6 +768,13 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
                                  cudaMemcpyHostToDevice, st));
     }
   }
+  // FP16 halves of the images for the form of iq_corr_tc.cu, where the Toeplitz form is left out
+  void *d_img16 = nullptr, *d_simg16 = nullptr;
+  if (tc && !tz && ovl_form == 1) {
+    d_img16 = iq_scratch(ctx, S_TZ_IMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * 4);
+    if (!d_img16) return IQ_ERR_ALLOC;
+    RET_IF(iq_tz_image(ctx, ctx->d_ti, ctx->ti, ctx->ti_stats, true, d_img16));
+  }
   // one tensor-core launch over the columns cols[0..N) with the masks of `cfgset`
   auto tc_launch = [&](const std::vector<int>& cfgset, const TcStageRef& sr, const float* img,
                        const double* ii, const float* grid, Dim3 gdims, const TcCol* cols, int N,
@@ -787,6 +794,7 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
     L.nsteps16 = sr.nsteps16;
     L.grid = grid; L.grid_dims = gdims; L.cols = cols; L.N = N; L.B = B;
     L.img_stats = img_stats; L.tmpl_stats = tmpl_stats; L.flops = flops;
+    L.img16 = img == ctx->d_ti ? d_img16 : d_simg16;
     return iq_launch_corr_tc(ctx, L);
   };
 
@@ -899,6 +907,11 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
         for (const TzPlan::Launch& l : sp.launches)
           RET_IF(sp.launch(ctx, l, img, distD, a2, d_aux[s], psz, B, auxti_stats, aux_stats));
       } else if (tc && T > 0) {
+        if (ctx->corr_engine == 2 && auxti_stats.fp16_range()) {
+          d_simg16 = iq_scratch(ctx, S_TZ_SIMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * 4);
+          if (!d_simg16) return IQ_ERR_ALLOC;
+          RET_IF(iq_tz_image(ctx, d_auxti[s], ctx->ti, auxti_stats, true, d_simg16));
+        }
         // per-tile soft distance maps on the tensor cores, up to 256 tiles per launch
         std::vector<TcCol> cols;
         std::vector<std::pair<size_t, int>> launches;  // (first column, N)
