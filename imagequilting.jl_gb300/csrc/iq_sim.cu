@@ -1,12 +1,13 @@
 // iq_simulate: the iqsim driver (src/iqsim.jl:50-315) on the GPU.
 //
 // All realizations of a call share the tile path (genpath runs once per call,
-// src/iqsim.jl:139), so every step processes one tile for the whole batch of realizations:
-//   gather templates -> batched overlap distance -> [hard distance] -> pick (one CTA per
-//   realization) -> graph cuts (one CTA per realization and slab) -> paste.
-// The hard and soft distance terms do not depend on the realization; the soft maps of all
-// tiles are computed up front in batches of 16 tiles and kept resident in HBM, the hard map
-// of a data tile is computed once per step. Nothing is copied back to the host until the
+// src/iqsim.jl:139), and the tiles of a dependency level touch disjoint regions, so a step
+// processes a chunk of a level for all realizations of a group:
+//   gather templates -> batched overlap distance -> pick (one CTA per tile and realization)
+//   -> graph cuts (one CTA per tile, realization and slab) -> paste.
+// The hard and soft distance terms do not depend on the realization: the maps of all data tiles
+// and of all soft tiles are computed up front and kept resident in HBM, as are the FP16 image and
+// the A2 maps of the tensor-core correlation. Nothing is copied back to the host until the
 // crop at the end.
 #include <math.h>
 #include <string.h>
