@@ -1173,29 +1173,38 @@ __device__ const uint32_t* ref_sort(Smem& s, unsigned long long* sbuf, int64_t n
 }
 
 // Make the order ord[0, n) exact: while two neighbours' intervals overlap (and are not both
-// exact), raise both and sort again by (value, position). At the end every adjacent pair is disjoint
-// or both exact, so the order is the order of the Float64 distances with ties broken by position.
+// exact), raise both; while any were raised, or two exact neighbours stand the wrong way round, sort
+// again by (Float64 value, position). The second case needs no raise: ref_sort orders by the values
+// rounded to FP32, so entries that come in exact (a cluster raised whole) may differ below that. At the
+// end every adjacent pair is disjoint, or both exact and in (value, position) order, so the order is
+// that of the Float64 distances with ties broken by position.
 // Returns the order (ord, or above SORT_CAP entries one of v0, v1).
 __device__ __noinline__ uint32_t* ref_resolve(Smem& s, unsigned long long* sbuf, const Ref& f,
                                               const int32_t* pos, int64_t n, uint32_t* ord, RefArr a,
                                               uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1) {
   for (int round = 0; round < 64; ++round) {
-    int any = 0;
+    int any = 0, swapped = 0;
     for (int64_t t = threadIdx.x; t < n; t += PT) a.link[t] = 0;
     __syncthreads();
     for (int64_t t = threadIdx.x; t + 1 < n; t += PT) {
       const uint32_t i = ord[t], j = ord[t + 1];
-      if (ref_exact(a, i) && ref_exact(a, j)) continue;
+      if (ref_exact(a, i) && ref_exact(a, j)) {
+        if (a.v[i] > a.v[j] || (a.v[i] == a.v[j] && i > j)) swapped = 1;
+        continue;
+      }
       if (a.v[i] + a.r[i] >= a.v[j] - a.r[j]) {
         a.link[t] = 1;
         any = 1;
       }
     }
-    if (!__syncthreads_or(any)) break;
-    for (int64_t t = threadIdx.x; t + 1 < n; t += PT)
-      if (a.link[t]) { ref_mark(a, ord[t]); ref_mark(a, ord[t + 1]); }
-    __syncthreads();
-    ref_raise(f, pos, n, a, round >= 3);
+    any = __syncthreads_or(any);
+    if (!__syncthreads_or(any | swapped)) break;
+    if (any) {
+      for (int64_t t = threadIdx.x; t + 1 < n; t += PT)
+        if (a.link[t]) { ref_mark(a, ord[t]); ref_mark(a, ord[t + 1]); }
+      __syncthreads();
+      ref_raise(f, pos, n, a, round >= 3);
+    }
     if (n <= SORT_CAP) {
       // the whole order by (Float64 value, entry) in shared memory (values are >= 0, so their
       // bits order like the values)
@@ -1214,8 +1223,8 @@ __device__ __noinline__ uint32_t* ref_resolve(Smem& s, unsigned long long* sbuf,
       continue;
     }
     // the whole order again: stable radix sorts by the low, then the high word of the Float64 values
-    // from the entries' order (position order). A raised entry may move past neighbours that are exact
-    // already, so sorting the raised runs alone would leave exact pairs out of order.
+    // from the entries' order (position order). (A raised entry may move past neighbours that are exact
+    // already: sorting the raised runs alone would not do.)
     for (int64_t i = threadIdx.x; i < n; i += PT) {
       k0[i] = (uint32_t)__double_as_longlong(a.v[i]);
       v0[i] = (uint32_t)i;
