@@ -477,7 +477,7 @@ extern "C" int iq_fastdistance(iq_ctx* ctx, const int64_t* tilesize, int32_t ntm
         std::vector<TcCol> cc;
         for (int32_t i = c0; i < std::min<int32_t>(ntmpl, c0 + 16 * IQ_TZ_COLS); ++i)
           cc.push_back(TcCol{(int64_t)i * T, d_out + (size_t)i * P, d_b2 + i, nullptr, 0, 0});
-        pl.add_launch(cc, 2.0 * (double)P * (double)K * (double)cc.size());
+        pl.add_launches(cc, 2.0 * (double)P * (double)K * (double)cc.size(), IQ_TZ_BYTES);
       }
       void* img = iq_scratch(ctx, S_TZ_IMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * 2);
       float* a2 = (float*)iq_scratch(ctx, S_TZ_A2, sizeof(float) * P);

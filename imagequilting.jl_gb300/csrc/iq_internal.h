@@ -288,6 +288,11 @@ int iq_value_stats(iq_ctx* ctx, const float* d, int64_t n, IqValueStats& out);
 
 // ---- tensor-core correlation, Toeplitz templates (iq_corr_tz.cu) ----
 constexpr int IQ_TZ_COLS = 32;   // columns (templates) per group: N = 8 x columns <= 256
+// Most bytes of packed templates in a launch (a group at least). A template takes 16 to 20 bytes a mask
+// offset, twice that when split: a chunk of 64 tiles and 64 realizations of 32 x 32 x 16 tiles (9,472
+// offsets) would be 0.8 GB, and with more realizations the largest buffer of a call. A launch of 512 MB
+// holds 2,800 such columns, 85 groups of them, each of which alone fills the chip.
+constexpr int64_t IQ_TZ_BYTES = (int64_t)512 << 20;
 constexpr int IQ_TZ_ROWS = 5;    // image rows staged together
 constexpr int IQ_TZ_STEPS = 5;   // K-steps (two 8-offset chunks each) staged together
 

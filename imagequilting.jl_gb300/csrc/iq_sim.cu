@@ -514,6 +514,7 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   const bool tz = ovl_form == 1 && T > 0 && iq_tz_fits(ctx->ti, tileD, distD) &&
                   (double)(ncfg + 1) * (double)P * 4.0 <= (double)freeb / 8.0;
   const bool tz_split = !(ctx->ti_stats.narrow && sim_stats.narrow);
+  const int64_t tz_cap = std::min<int64_t>(IQ_TZ_BYTES, (int64_t)(freeb / 16));
   // hard-data distance maps depend on the data only: one map per data tile, all held at once
   int64_t nhs = 0;
   for (const Step& s : steps) nhs += s.hardtile ? 1 : 0;
@@ -641,7 +642,8 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   struct TcRun {
     int64_t chunk; size_t col0; int N; std::vector<int> cfgset; TcStageRef st; double flops;
   };
-  TzPlan tzp;                 // launch of (chunk c, group g): c * ngrp + g
+  TzPlan tzp;
+  std::vector<int64_t> tzbeg(nchunk * ngrp + 1, 0);  // its launches of (chunk c, group g): c * ngrp + g
   tzp.img = ctx->ti; tzp.tile = tileD; tzp.split = tz_split;
   for (int c = 0; c <= ncfg; ++c) tzp.boxes.push_back(cfg_box(c));
   std::vector<TcRun> tcruns;
@@ -674,7 +676,8 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
                                d_mm + (size_t)o.second * R * 2 + 2 * r, o.first, 0});
             fl += 2.0 * (double)P * (double)cfgs[o.first].K;
           }
-        tzp.add_launch(cc, fl);
+        tzp.add_launches(cc, fl, tz_cap);
+        tzbeg[cg + 1] = (int64_t)tzp.launches.size();
         continue;
       }
       if (order.empty()) {
@@ -876,7 +879,7 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
               const int64_t slot = (int64_t)s * nslot + slot_of[tl[i]];
               cc.push_back(TcCol{starts[i], d_soft + slot * P, d_softb2 + slot, d_softmm + 2 * slot, 0, 0});
             }
-            sp.add_launch(cc, 2.0 * (double)P * (double)T * (double)cc.size());
+            sp.add_launches(cc, 2.0 * (double)P * (double)T * (double)cc.size(), tz_cap);
           }
           soft_kappa[s] = iq_map_kappa_tz(auxti_stats, aux_stats, T, sp.touched[0]);
         } else
@@ -1320,8 +1323,9 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
         G.ntask = m; G.tasks = d_gt + grp * nsteps + k0;
         RET_IF(iq_launch_gather(ctx, G));
         if (tz) {
-          RET_IF(tzp.launch(ctx, tzp.launches[c * ngrp + grp], d_tzimg, distD, d_tza2, d_sim, padD,
-                            (char*)d_tzB + grp * tzb_bytes, ctx->ti_stats, sim_stats));
+          for (int64_t l = tzbeg[c * ngrp + grp]; l < tzbeg[c * ngrp + grp + 1]; ++l)
+            RET_IF(tzp.launch(ctx, tzp.launches[l], d_tzimg, distD, d_tza2, d_sim, padD,
+                              (char*)d_tzB + grp * tzb_bytes, ctx->ti_stats, sim_stats));
         } else if (chunk_tc[c]) {
           for (int64_t l = tcbeg[c * ngrp + grp]; l < tcbeg[c * ngrp + grp + 1]; ++l) {
             const TcRun& u = tcruns[l];

@@ -50,39 +50,47 @@ struct TzPlan {
     lists[set] = r;
     return r;
   }
-  // One launch over `c` (columns grouped by mask): groups of balanced, even width. Split data
-  // take groups of at most 16 columns, so that the two accumulators of two 1024-position blocks
-  // fill TMEM (the templates of a K-step then serve 2048 positions).
-  void add_launch(const std::vector<TcCol>& c, double flops) {
-    Launch L{(int)groups.size(), 0, 0, (int)c.size(), 0, 0, flops, 0.0};
+  // Launches over `c` (columns grouped by mask): groups of balanced, even width, as many to a launch
+  // as `cap` bytes of packed templates hold (one at least; the launches follow one another in the same
+  // buffer). Split data take groups of at most 16 columns, so that the two accumulators of two
+  // 1024-position blocks fill TMEM (the templates of a K-step then serve 2048 positions).
+  void add_launches(const std::vector<TcCol>& c, double flops, int64_t cap) {
     const int64_t most = split ? IQ_TZ_COLS / 2 : IQ_TZ_COLS, n = (int64_t)c.size();
     const int64_t ng = (n + most - 1) / most;
     const int64_t per = ng > 0 ? ((n + ng - 1) / ng + 1) / 2 * 2 : 0;
+    Launch L{};
     for (int64_t q = 0; q < n; q += per) {
       const int64_t m = std::min(per, n - q);
-      TzGroup g{};
-      g.col0 = (int32_t)cols.size();
       std::vector<int> set;
-      for (int64_t i = q; i < q + m; ++i) {
-        cols.push_back(c[i]);
+      for (int64_t i = q; i < q + m; ++i)
         if (set.empty() || set.back() != c[i].box) set.push_back(c[i].box);
-      }
       std::sort(set.begin(), set.end());
       set.erase(std::unique(set.begin(), set.end()), set.end());
-      if (m & 1) cols.push_back(TcCol{-1, nullptr, nullptr, nullptr, 0, 0});
-      g.ncol = (int32_t)(cols.size() - g.col0);
-      g.N = 8 * g.ncol;
       const Ref r = list_of(set);
+      TzGroup g{};
+      g.ncol = (int32_t)(m + (m & 1));
+      g.N = 8 * g.ncol;
       g.stage0 = r.stage0; g.nstage = r.nstage; g.nstep = r.nstep; g.chunk0 = r.chunk0;
+      const int64_t bytes = ((int64_t)g.nstep * 32 * g.N * (split ? 2 : 1) + 255) / 256 * 256;
+      if (L.ngroup > 0 && L.bytes + bytes > cap) {
+        launches.push_back(L);
+        L = Launch{};
+      }
+      if (L.ngroup == 0) L.group0 = (int)groups.size();
+      g.col0 = (int32_t)cols.size();
+      cols.insert(cols.end(), c.begin() + q, c.begin() + q + m);
+      if (m & 1) cols.push_back(TcCol{-1, nullptr, nullptr, nullptr, 0, 0});
       g.boff = L.bytes;
-      L.bytes += ((int64_t)g.nstep * 32 * g.N * (split ? 2 : 1) + 255) / 256 * 256;
+      L.bytes += bytes;
       L.units = std::max<int64_t>(L.units, (int64_t)g.nstep * 2 * g.N);
       L.Nmax = std::max(L.Nmax, (int)g.N);
       L.mma += 2.0 * 128 * 16 * (double)g.nstep * g.N;
+      L.flops += flops * (double)m / (double)n;
+      L.ncols += (int)m;
       L.ngroup++;
       groups.push_back(g);
     }
-    launches.push_back(L);
+    if (L.ngroup > 0) launches.push_back(L);
   }
   int64_t max_bytes() const {
     int64_t b = 1;
