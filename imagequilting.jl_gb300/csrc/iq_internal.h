@@ -100,6 +100,12 @@ struct iq_ctx {
                                    // resident image's (keys the proposal's caches)
   unsigned long long ti_hash = 0;  // content key of the resident image (values and extents)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // bytes of the scratch slots, kept from call to call
+  size_t held() const {
+    size_t b = 0;
+    for (size_t x : buf_bytes) b += x;
+    return b;
+  }
 };
 enum IqStat { ST_CUT_ROUNDS = 0, ST_CUT_LEVELS, ST_CUT_CTAS, ST_PICK_ITERS, ST_PICK_CAND,
               ST_PICK_CTAS, ST_CUT_MAXROUNDS, ST_CUT_MAXLEVELS,

@@ -508,13 +508,6 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
                            T * (rpad + 1) * 4 + (int64_t)R * 6 * (slabmax + cutscr_per) + 4096;
   size_t freeb = 0, totalb = 0;
   cudaMemGetInfo(&freeb, &totalb);
-  // The Toeplitz form of the correlation (iq_corr_tz.cu) for data FP16 halves represent, unless
-  // its A2 maps (one per mask) would take more than an eighth of the free memory: then, and for
-  // data of wider range, the form of iq_corr_tc.cu.
-  const bool tz = ovl_form == 1 && T > 0 && iq_tz_fits(ctx->ti, tileD, distD) &&
-                  (double)(ncfg + 1) * (double)P * 4.0 <= (double)freeb / 8.0;
-  const bool tz_split = !(ctx->ti_stats.narrow && sim_stats.narrow);
-  const int64_t tz_cap = std::min<int64_t>(IQ_TZ_BYTES, (int64_t)(freeb / 16));
   // hard-data distance maps depend on the data only: one map per data tile, all held at once
   int64_t nhs = 0;
   for (const Step& s : steps) nhs += s.hardtile ? 1 : 0;
@@ -524,10 +517,11 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
                         (long long)nhs, (long long)hard_bytes);
   // soft-data maps: one map of P floats per (non-skipped tile, soft variable), all held for the
   // whole call (about 122 GB for a 5.7 M-position map over 5,324 tiles)
+  double soft_bytes = 0.0;
   if (nsoft > 0) {
     int64_t nlive = 0;
     for (int64_t t = 0; t < g.ntot; ++t) nlive += skipped[t] ? 0 : 1;
-    const double soft_bytes = (double)nlive * nsoft * (double)P * 4.0;
+    soft_bytes = (double)nlive * nsoft * (double)P * 4.0;
     if (soft_bytes + (double)hard_bytes > (double)freeb * 0.75)
       return iq_set_error(IQ_ERR_LIMIT,
                           "soft-data maps of %lld tiles x %d variables need %.0f bytes, more than "
@@ -561,8 +555,23 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   const int ngrp = (tc && T > 0 && R >= 2 && nstr >= 2) ? 2 : 1;
   const int gb[3] = {0, ngrp == 2 ? (R + 1) / 2 : R, R};
 
-  // ---- device buffers ----
   const bool debug = p->debug != 0 && (cuts || voxs);
+  // The Toeplitz form of the correlation (iq_corr_tz.cu) for data FP16 halves represent, unless its
+  // image and A2 maps (one per mask) would take more than an eighth of the memory, or with its packed
+  // templates more than the rest of the call leaves: then, and for data of wider range, the form of
+  // iq_corr_tc.cu. The scratch held from earlier calls counts as memory, so that a repeated call, whose
+  // buffers are that scratch, takes the same form again.
+  const double mem = (double)freeb + (double)ctx->held();
+  const bool tz_split = !(ctx->ti_stats.narrow && sim_stats.narrow);
+  const int64_t tz_cap = std::min<int64_t>(IQ_TZ_BYTES, (int64_t)(mem / 16.0));
+  const double tz_maps = (double)(iq_tz_image_halves(ctx->ti) + 64) * (tz_split ? 4.0 : 2.0) +
+                         (double)(ncfg + 1) * (double)P * 4.0;
+  const double rest = 4.0 * R * ((double)padvol * (debug ? 2 : 1) + (double)simvol) + soft_bytes +
+                      (double)hard_bytes + (double)cmax * (double)per_step;
+  const bool tz = ovl_form == 1 && T > 0 && iq_tz_fits(ctx->ti, tileD, distD) && tz_maps <= mem / 8.0 &&
+                  rest + tz_maps + (double)tz_cap * ngrp <= mem * 15.0 / 16.0;
+
+  // ---- device buffers ----
   float* d_sim = (float*)iq_scratch(ctx, S_SIM, sizeof(float) * padvol * R);
   float* d_cut = debug ? (float*)iq_scratch(ctx, S_CUT, sizeof(float) * padvol * R) : nullptr;
   float* d_D = (float*)iq_scratch(ctx, S_D, sizeof(float) * P * R * cmax);

@@ -51,3 +51,37 @@ def test_packed_templates_of_many_realizations(iq):
         got = _fresh(iq, *args, **kw)
     for x, y in zip(got, want):
         assert np.array_equal(x, y)
+
+
+def _image(values, shape):
+    rng = np.random.default_rng(302)
+    z = rng.normal(size=shape)
+    return ((z > 0).astype(np.float32) if values == "binary" else np.exp(z).astype(np.float32))
+
+
+# Nine tiles, the first drawn without a map: the Toeplitz form computes eight columns, the other form
+# launches of 16. Five A2 maps of 2,017 x 2,017 positions take 81 MB.
+ARGS = ((32, 32), (56, 56))
+KW = dict(overlap=(0.25, 0.25), rng=4)
+
+
+@pytest.mark.parametrize("values,mb,padded", [("binary", 800, False), ("binary", 500, True),
+                                              ("lognormal", 900, False), ("lognormal", 560, True)])
+def test_form_of_the_correlation(iq, values, mb, padded):
+    """The Toeplitz form while its maps fit an eighth of the memory, for a first and a repeated call
+    alike, and the FP16 form of wider data's kernel where they do not: the same realizations."""
+    ti = _image(values, (2048, 2048))
+    want = _fresh(iq, ti, *ARGS, **KW)
+    ctx = iq.Context(0)
+    try:
+        ctx.set_ti(ti)
+        with left(mb * MB):
+            for _ in range(2):
+                ctx.profile(True)
+                got = _call(iq, ctx, ti, *ARGS, **KW)
+                cols = ctx.profile_get("corr.columns")[2]
+                assert cols == (8 * 16 if padded else 8)
+                for x, y in zip(got, want):
+                    assert np.array_equal(x, y)
+    finally:
+        ctx.close()
