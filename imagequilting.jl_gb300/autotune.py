@@ -10,7 +10,7 @@ context.
 """
 import time
 
-# the library's defaults (include/iqgpu.h) and the candidate values tried for each knob
+# where the search starts and the candidate values tried for each knob
 DEFAULTS = {
     "graphcut.threads": 512,
     "graphcut.gr_period": 16,
@@ -23,6 +23,10 @@ CANDIDATES = {
     "sim.level_chunk": (16, 64, 256),
     "sim.streams": (1, 2),
 }
+
+# the library's own defaults (include/iqgpu.h): `autotune` starts there, and -1 (the library chooses
+# the streams of each call) is one of its candidates
+LIBRARY = dict(DEFAULTS, **{"sim.streams": -1})
 
 
 def coordinate_descent(measure, knobs=None, start=None, sweeps=1):
@@ -69,10 +73,16 @@ def autotune(ctx, trainimg, tilesize, simsize=None, *, knobs=None, sample_steps=
 
     Each setting is timed as the fastest of `repeats` calls (after one untimed call that
     warms the context's buffers), each simulating the first `sample_steps` tiles of every
-    realization. The best settings are applied to `ctx` and `sim.max_steps` is restored to
-    -1 (all tiles). Returns (settings, seconds per sampled call, history)."""
+    realization. The search starts at the library's defaults (at one stream where the given candidates
+    of `sim.streams` leave the automatic choice out). The best settings are applied to `ctx` and
+    `sim.max_steps` is restored to -1 (all tiles). Returns (settings, seconds per sampled call,
+    history)."""
     from .api import iqsim
 
+    knobs = dict(CANDIDATES, **{"sim.streams": (-1, 1, 2)}) if knobs is None else dict(knobs)
+    start = dict(LIBRARY)
+    if -1 not in knobs.get("sim.streams", (-1,)):
+        start["sim.streams"] = DEFAULTS["sim.streams"]
     kw = dict(iqsim_kwargs)
     kw["ctx"] = ctx
 
@@ -92,7 +102,7 @@ def autotune(ctx, trainimg, tilesize, simsize=None, *, knobs=None, sample_steps=
 
     ctx.set_option("sim.max_steps", int(sample_steps))
     try:
-        best, best_t, history = coordinate_descent(measure, knobs, sweeps=sweeps)
+        best, best_t, history = coordinate_descent(measure, knobs, start, sweeps=sweeps)
     finally:
         ctx.set_option("sim.max_steps", -1)
     apply(best)

@@ -270,7 +270,8 @@ extern "C" int iq_set_option(iq_ctx* ctx, const char* name, int64_t value) {
     return IQ_OK;
   }
   if (!strcmp(name, "sim.streams")) {
-    if (value < 1 || value > 2) return iq_set_error(IQ_ERR_ARG, "sim.streams must be 1 or 2");
+    if (value != -1 && value != 1 && value != 2)
+      return iq_set_error(IQ_ERR_ARG, "sim.streams must be 1, 2 or -1 (automatic)");
     ctx->sim_streams = (int)value;
     return IQ_OK;
   }

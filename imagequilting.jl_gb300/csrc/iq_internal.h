@@ -85,7 +85,7 @@ struct iq_ctx {
   int corr_engine = 2;          // box-mask distances: 2 tensor cores FP16 halves when the data's
                                 // range allows (else TF32), 1 tensor cores TF32, 0 SIMT
   int64_t max_steps = -1;       // tiles simulated per realization (< 0: all)
-  int sim_streams = 0;          // realization groups of iq_simulate, each on its own stream (0: by
+  int sim_streams = -1;         // realization groups of iq_simulate, each on its own stream (-1: by
                                 // whether the maps need the exact re-rank)
   cudaStream_t stream2 = nullptr;  // stream of the second realization group (made on first use)
   struct IqLp* lp = nullptr;       // learned proposal state (iq_proposal_host.cu)
