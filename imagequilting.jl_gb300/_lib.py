@@ -76,6 +76,10 @@ SIGNATURES = {
                                    ctypes.POINTER(HardData), ctypes.c_int32,
                                    ctypes.POINTER(SoftData), ctypes.c_void_p, ctypes.c_void_p,
                                    ctypes.c_void_p]),
+    "iq_simulate_each": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(SimParams),
+                                        ctypes.POINTER(HardData), ctypes.c_int32,
+                                        ctypes.POINTER(SoftData), ctypes.POINTER(ctypes.c_void_p),
+                                        ctypes.c_void_p, ctypes.c_void_p]),
     "iq_fastdistance": (ctypes.c_int, [ctypes.c_void_p, c_i64p, ctypes.c_int32, ctypes.c_void_p,
                                        ctypes.c_void_p, ctypes.c_void_p]),
     "iq_pick": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int32,

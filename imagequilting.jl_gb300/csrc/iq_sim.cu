@@ -175,10 +175,11 @@ struct MaskCfg {
 
 }  // namespace
 
-extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* hard,
-                           int32_t nsoft, const iq_soft_data* soft, float* reals, float* cuts,
-                           double* voxs) {
-  if (!ctx || !p || !reals) return iq_set_error(IQ_ERR_ARG, "null argument");
+// `reals`: one buffer for all realizations; or `each`: one per realization (the other is null).
+static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* hard, int32_t nsoft,
+                    const iq_soft_data* soft, float* reals, float* const* each, float* cuts,
+                    double* voxs) {
+  if (!ctx || !p || (!reals && !each)) return iq_set_error(IQ_ERR_ARG, "null argument");
   if (!ctx->has_ti) return iq_set_error(IQ_ERR_STATE, "no training image set");
   IQ_CUDA_OK(cudaSetDevice(ctx->device));
   const int N = p->ndim;
@@ -197,6 +198,8 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   if (!(p->tol > 0 && p->tol <= 1)) return iq_set_error(IQ_ERR_ARG, "tolerance must be in range (0,1]");
   if (p->path < 0 || p->path > 2) return iq_set_error(IQ_ERR_ARG, "invalid simulation path");
   if (p->nreal <= 0) return iq_set_error(IQ_ERR_ARG, "invalid number of realizations");
+  for (int r = 0; each && r < p->nreal; ++r)
+    if (!each[r]) return iq_set_error(IQ_ERR_ARG, "null realization buffer");
   if (p->real0 < 0 || p->real0 + p->nreal > ((int64_t)1 << 32))
     return iq_set_error(IQ_ERR_ARG, "realization range outside [0, 2^32)");
   if (nsoft < 0 || (nsoft > 0 && !soft)) return iq_set_error(IQ_ERR_ARG, "invalid soft data");
@@ -1419,7 +1422,9 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   float* d_out = (float*)iq_scratch(ctx, S_OUT, sizeof(float) * simvol * R);
   if (!d_out) return IQ_ERR_ALLOC;
   RET_IF(iq_launch_crop(ctx, R, d_sim, padD, padvol, simD, d_out));
-  IQ_CUDA_OK(cudaMemcpyAsync(reals, d_out, sizeof(float) * simvol * R, cudaMemcpyDefault, st));
+  if (reals) IQ_CUDA_OK(cudaMemcpyAsync(reals, d_out, sizeof(float) * simvol * R, cudaMemcpyDefault, st));
+  for (int r = 0; each && r < R; ++r)
+    IQ_CUDA_OK(cudaMemcpyAsync(each[r], d_out + r * simvol, sizeof(float) * simvol, cudaMemcpyDefault, st));
   if (debug && cuts) {
     IQ_CUDA_OK(cudaStreamSynchronize(st));
     RET_IF(iq_launch_crop(ctx, R, d_cut, padD, padvol, simD, d_out));
@@ -1439,4 +1444,16 @@ extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_da
   if (status == IQ_ERR_CUTCAP) return iq_set_error(status, "graph cut hit its round limit");
   if (status) return iq_set_error(status, "kernel status %d", status);
   return IQ_OK;
+}
+
+extern "C" int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* hard,
+                           int32_t nsoft, const iq_soft_data* soft, float* reals, float* cuts,
+                           double* voxs) {
+  return simulate(ctx, p, hard, nsoft, soft, reals, nullptr, cuts, voxs);
+}
+
+extern "C" int iq_simulate_each(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* hard,
+                                int32_t nsoft, const iq_soft_data* soft, float* const* reals,
+                                float* cuts, double* voxs) {
+  return simulate(ctx, p, hard, nsoft, soft, nullptr, reals, cuts, voxs);
 }

@@ -119,6 +119,10 @@ int iq_set_ti(iq_ctx* ctx, const void* ti, int32_t dtype, int32_t ndim, const in
 int iq_simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* hard, int32_t nsoft,
                 const iq_soft_data* soft, float* reals, float* cuts, double* voxs);
 
+/* The same with a buffer per realization: reals[r] holds prod(simsize) floats. */
+int iq_simulate_each(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* hard, int32_t nsoft,
+                     const iq_soft_data* soft, float* const* reals, float* cuts, double* voxs);
+
 /*
  * fastdistance (src/utils.jl:5-13) of `ntmpl` templates against the resident TI:
  *   out[t][p] = |sum_k w_k TI[p+k]^2 - 2 sum_k w_k tmpl_t[k] TI[p+k] + sum_k w_k tmpl_t[k]^2|
