@@ -458,8 +458,9 @@ extern "C" int iq_fastdistance(iq_ctx* ctx, const int64_t* tilesize, int32_t ntm
   G.ntmpl = ntmpl; G.rpad = rpad;
   G.t0 = GatherTask{d_kl, K, 0, nullptr, d_tv, d_b2, nullptr};
   if ((rc = iq_launch_gather(ctx, G))) return rc;
-  std::vector<TcCol> cols;
+  std::vector<TcCol> cols;   // (the copies of these read them until the synchronization below)
   std::vector<uint32_t> stw;
+  TzPlan pl;
   if (use_tc) {
     IqValueStats tstats;
     if ((rc = iq_value_stats(ctx, d_tmpl, T * ntmpl, tstats))) return rc;
@@ -471,7 +472,6 @@ extern "C" int iq_fastdistance(iq_ctx* ctx, const int64_t* tilesize, int32_t ntm
     if (ctx->corr_engine == 2 && ctx->ti_stats.fp16_range() && tstats.fp16_range() &&
         iq_map_kappa(ctx->ti_stats, tstats, K, 1) == 0.0 && ctx->ti_stats.narrow && tstats.narrow &&
         iq_tz_fits(ctx->ti, t, od)) {
-      TzPlan pl;
       pl.img = ctx->ti; pl.tile = t; pl.boxes.push_back(box0);
       // at most 16 groups per launch: their packed templates share one buffer
       for (int32_t c0 = 0; c0 < ntmpl; c0 += 16 * IQ_TZ_COLS) {

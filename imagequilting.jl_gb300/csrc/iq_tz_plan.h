@@ -27,6 +27,9 @@ struct TzPlan {
   std::map<std::vector<int>, Ref> lists;
   struct Launch { int group0, ngroup, Nmax, ncols; int64_t units, bytes; double flops, mma; };
   std::vector<Launch> launches;
+  // What upload() copies from: a copy of pageable memory may still be reading it when the call returns,
+  // so the plan outlives the stream's next synchronization.
+  std::vector<char> host;
   // device copies
   const TzGroup* d_groups = nullptr;
   const TzStage* d_stages = nullptr;
@@ -104,16 +107,16 @@ struct TzPlan {
     const void* src[5] = {groups.data(), stages.data(), chunks.data(), boxes.data(), cols.data()};
     size_t total = 0;
     for (size_t b : sz) total += pad(b);
-    std::vector<char> h(total + 1);
+    host.assign(total + 1, 0);
     char* d = (char*)iq_scratch(ctx, slot, total + 256);
     if (!d) return IQ_ERR_ALLOC;
     size_t at[5], off = 0;
     for (int i = 0; i < 5; ++i) {
       at[i] = off;
-      if (sz[i]) memcpy(h.data() + off, src[i], sz[i]);
+      if (sz[i]) memcpy(host.data() + off, src[i], sz[i]);
       off += pad(sz[i]);
     }
-    IQ_CUDA_OK(cudaMemcpyAsync(d, h.data(), total, cudaMemcpyHostToDevice, st));
+    IQ_CUDA_OK(cudaMemcpyAsync(d, host.data(), total, cudaMemcpyHostToDevice, st));
     d_groups = (const TzGroup*)(d + at[0]);
     d_stages = (const TzStage*)(d + at[1]);
     d_chunks = (const uint32_t*)(d + at[2]);
