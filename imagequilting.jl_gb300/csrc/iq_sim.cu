@@ -732,25 +732,30 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
     }
     tcbeg[cg + 1] = (int64_t)tcruns.size();
   }
-  // Toeplitz form: the FP16 image, the A2 maps of every mask and the plan, once per call
+  // Toeplitz form: the FP16 image, the A2 maps of every mask and the plan, once per call, before the
+  // first chunk that computes maps (a call that the learned proposal serves has none)
   void *d_tzimg = nullptr, *d_tzB = nullptr;
   float* d_tza2 = nullptr;
   size_t tzb_bytes = 0;
-  if (tz) {
-    for (int c = 0; c < ncfg; ++c)
-      if (cfg_kappa[c] > 0.0) {
-        tzp.touched.resize(tzp.boxes.size(), 0);
-        cfg_kappa[c] = iq_map_kappa_tz(ctx->ti_stats, sim_stats, cfgs[c].K, tzp.touched[c]);
-      }
+  bool tz_ready = false;
+  auto tz_setup = [&]() -> int {
     tzb_bytes = (size_t)tzp.max_bytes();
     d_tzimg = iq_scratch(ctx, S_TZ_IMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * (tz_split ? 4 : 2));
     d_tza2 = (float*)iq_scratch(ctx, S_TZ_A2, sizeof(float) * P * (ncfg + 1));
     d_tzB = iq_scratch(ctx, S_TZ_B, tzb_bytes * ngrp);
     if (!d_tzimg || !d_tza2 || !d_tzB) return IQ_ERR_ALLOC;
-    RET_IF(tzp.upload(ctx, S_TZ_PLAN, st));
+    RET_IF(tzp.upload(ctx, S_TZ_PLAN, ctx->stream));
     RET_IF(iq_tz_image(ctx, ctx->d_ti, ctx->ti, ctx->ti_stats, tz_split, d_tzimg));
     RET_IF(iq_tz_a2_maps(ctx, ctx->d_ti2ii, ctx->ti, distD, tileD, tzp.d_boxes, ncfg, d_dis, d_tza2));
-  }
+    tz_ready = true;
+    return IQ_OK;
+  };
+  if (tz)
+    for (int c = 0; c < ncfg; ++c)
+      if (cfg_kappa[c] > 0.0) {
+        tzp.touched.resize(tzp.boxes.size(), 0);
+        cfg_kappa[c] = iq_map_kappa_tz(ctx->ti_stats, sim_stats, cfgs[c].K, tzp.touched[c]);
+      }
   const TcStageRef soft_st = (tc && nsoft > 0 && T > 0) ? stages_for(std::vector<int>{ncfg})
                                                          : TcStageRef{0, 0, 0, 0, 0, 0};
   uint32_t* d_tcst = nullptr;  // stage words of every list, then their prefixes
@@ -902,9 +907,8 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
         // per-tile soft distance maps, Toeplitz form
         void* img = iq_scratch(ctx, S_TZ_SIMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * (sp.split ? 4 : 2));
         float* a2 = (float*)iq_scratch(ctx, S_TZ_SA2, sizeof(float) * P);
-        void* B = iq_scratch(ctx, S_TZ_B, std::max((size_t)sp.max_bytes(), tzb_bytes * ngrp));
+        void* B = iq_scratch(ctx, S_TZ_B, (size_t)sp.max_bytes());
         if (!img || !a2 || !B) return IQ_ERR_ALLOC;
-        d_tzB = B;  // the slot may have moved
         RET_IF(sp.upload(ctx, S_TCSOFT, st));
         RET_IF(iq_tz_image(ctx, d_auxti[s], ctx->ti, auxti_stats, sp.split, img));
         RET_IF(iq_tz_a2_maps(ctx, d_auxii[s], ctx->ti, distD, tileD, sp.d_boxes, 1, d_dis, a2));
@@ -1263,6 +1267,7 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
   for (const MaskCfg& mc : cfgs) maxK = std::max<int64_t>(maxK, mc.K);
   const bool lp_on = iq_lp_applies(ctx, tileD, maxK, nh > 0 || nsoft > 0);
   const bool lp_cap = ctx->lp_capture > 0 && ctx->lp != nullptr;
+  if (tz && !lp_on && !tzp.launches.empty()) RET_IF(tz_setup());
   std::vector<int32_t> lc_lohi(6 * std::max(ncfg, 1)), lc_cfgK(std::max(ncfg, 1));
   for (int cf = 0; cf < ncfg; ++cf) {
     for (int d = 0; d < 3; ++d) {
@@ -1335,6 +1340,10 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
         G.ntask = m; G.tasks = d_gt + grp * nsteps + k0;
         RET_IF(iq_launch_gather(ctx, G));
         if (tz) {
+          if (!tz_ready && tzbeg[c * ngrp + grp] < tzbeg[c * ngrp + grp + 1]) {
+            RET_IF(tz_setup());
+            IQ_CUDA_OK(cudaStreamSynchronize(ctx->stream));  // the other group's stream reads it too
+          }
           for (int64_t l = tzbeg[c * ngrp + grp]; l < tzbeg[c * ngrp + grp + 1]; ++l)
             RET_IF(tzp.launch(ctx, tzp.launches[l], d_tzimg, distD, d_tza2, d_sim, padD,
                               (char*)d_tzB + grp * tzb_bytes, ctx->ti_stats, sim_stats));
