@@ -334,7 +334,9 @@ def proposal_roofline(dom, prof, lp_kernels, W, peaks, peak_kind, st, args):
     cols = st["cols_shortlist"] if st else 0
     planes = bool(np.isin(W["ti"], (0, 1, 2, 3)).all()) and W["tilesize"][0] <= 32
     per = 0.25 if planes else 1.0
-    byts = cols * (st["mean_shortlist"] if st else 0) * K * per
+    # `st` counts one call, the kernel's time is the sum over the timed calls
+    calls = args.steps if args is not None else 1
+    byts = cols * (st["mean_shortlist"] if st else 0) * K * per * calls
     ach = byts / (ms / 1e3) / 1e9 if ms else None
     return {"bound": "hbm", "kernel": dom, "achieved": ach, "unit": "GB/s",
             "peak": peaks.get("hbm_gbs"), "peak_kind": "%s (copy)" % peak_kind,
