@@ -49,6 +49,13 @@ void* iq_scratch(iq_ctx* ctx, int slot, size_t bytes) {
   return p;
 }
 
+int iq_sm_count() {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n > 0 ? n : 1;
+}
+
 // ---- timers --------------------------------------------------------------------------
 void iq_timer_start(iq_ctx* ctx, const char* name) {
   if (!ctx->prof) return;

@@ -579,9 +579,9 @@ int iq_launch_corr_tz(iq_ctx* ctx, const TzLaunch& L) {
     return iq_set_error(IQ_ERR_ARG, "tensor-core correlation: bad launch");
   const Dim3 od = L.out_dims;
   const int64_t ixp = (L.img_dims.x + 7) / 8 * 8;
-  int dev = 0, nsm = 0, lim = 0;
+  int dev = 0, lim = 0;
+  const int nsm = iq_sm_count();
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   lim -= 4096;  // the kernel's static shared memory
   // Accumulators per CTA: more of them reuse a staged template chunk for more positions, fewer

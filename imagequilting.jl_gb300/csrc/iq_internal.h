@@ -141,6 +141,7 @@ enum IqSlot {
 
 // device scratch of at least `bytes` in slot `slot` (contents undefined); nullptr on failure
 void* iq_scratch(iq_ctx* ctx, int slot, size_t bytes);
+int iq_sm_count();  // SMs of the current device
 
 // ---------------------------------------------------------------------------------------
 // Timing helpers (no-ops unless ctx->prof)

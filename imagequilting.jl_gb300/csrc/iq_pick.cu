@@ -2226,7 +2226,8 @@ int iq_launch_pick(iq_ctx* ctx, const PickLaunch& L) {
     a.thr_ties = L.thr + nblocks;
     IQ_CUDA_OK(cudaMemsetAsync(L.thr, 0, sizeof(int) * 2 * nblocks, ctx->stream));
     const int64_t tiles = (L.P + TC_NT * TC_ITEMS - 1) / (TC_NT * TC_ITEMS);
-    const int64_t ny = std::max<int64_t>(1, std::min<int64_t>(tiles, 152 * 8 / std::min(nblocks, 152 * 8)));
+    const int most = 8 * iq_sm_count();
+    const int64_t ny = std::max<int64_t>(1, std::min<int64_t>(tiles, most / std::min(nblocks, most)));
     iq_timer_start(ctx, "pick");
     thr_collect_kernel<<<dim3((unsigned)nblocks, (unsigned)ny), TC_NT, 0, ctx->stream>>>(a);
     iq_timer_stop(ctx, "pick", 0);

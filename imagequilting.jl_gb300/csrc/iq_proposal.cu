@@ -432,8 +432,9 @@ int iq_lp_shortlist(iq_ctx* ctx, const __nv_bfloat16* W, const float* nW, int64_
   if (N <= 0) return IQ_OK;
   const int64_t nblk = (P + 15) / 16;
   // slices of the lists: four CTAs per SM, each at least one pass of its threads
+  const int nsm = iq_sm_count();
   const int64_t grps = (N + 7) / 8, npass = (nblk + LL_NT * LL_BLK - 1) / (LL_NT * LL_BLK);
-  const int64_t want = std::max<int64_t>(1, std::min<int64_t>(npass, 4 * 152 / grps));
+  const int64_t want = std::max<int64_t>(1, std::min<int64_t>(npass, 4 * nsm / grps));
   const int64_t per = (npass + want - 1) / want * (LL_NT * LL_BLK), slices = (nblk + per - 1) / per;
   uint4* bits = (uint4*)iq_scratch(ctx, S_LP_BITS2, sizeof(uint4) * (size_t)grps * nblk +
                                                         sizeof(int) * 8 * (size_t)(grps * slices));
@@ -444,9 +445,6 @@ int iq_lp_shortlist(iq_ctx* ctx, const __nv_bfloat16* W, const float* nW, int64_
   // the m-th smallest sampled score stands for about m * stride positions
   const int m = (int)std::max<int64_t>(4, std::min<int64_t>(S, (k + stride - 1) / stride));
   cudaStream_t st = ctx->stream;
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   iq_timer_start(ctx, "lp.scan");
   // per-column thresholds: the sampled rows' scores as one GEMM, then a select per column
   const size_t sm = sizeof(uint32_t) * LP_SCAN_COLS * LP_SCAN_LD + 2 * sizeof(float) * LP_SCAN_COLS;
@@ -490,7 +488,7 @@ int iq_lp_recall(iq_ctx* ctx, const LpImg& im, Dim3 dist, const LpColumn& col,
   IQ_CUDA_OK(cudaMemcpyAsync(dmin, &inf, sizeof(unsigned), cudaMemcpyHostToDevice, ctx->stream));
   IQ_CUDA_OK(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * ((P + 31) / 32), ctx->stream));
   iq_timer_start(ctx, "lp.monitor");
-  lp_full_kernel<<<(unsigned)std::min<int64_t>((P + 255) / 256, 152 * 8), 256, sm, ctx->stream>>>(
+  lp_full_kernel<<<(unsigned)std::min<int64_t>((P + 255) / 256, 8 * iq_sm_count()), 256, sm, ctx->stream>>>(
       im, dist.x, dist.x * dist.y, P, col, Dbuf, dmin);
   lp_mark_kernel<<<64, 256, 0, ctx->stream>>>(list, cnt, cap, bits);
   lp_recall_kernel<<<(unsigned)std::min<int64_t>((P + 255) / 256, 1024), 256, 0, ctx->stream>>>(

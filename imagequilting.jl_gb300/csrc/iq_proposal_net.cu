@@ -879,13 +879,6 @@ LpGeo iq_lp_geo(Dim3 tile) {
 
 namespace {
 
-int sm_count() {
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  return nsm;
-}
-
 // prepared parameters in scratch
 int net_prep(iq_ctx* ctx, const LpGeo& g, const float* w, int bf16, float** out) {
   float* nw = (float*)iq_scratch(ctx, S_LP_W, sizeof(float) * NW_END);
@@ -902,7 +895,7 @@ int net_l2(iq_ctx* ctx, const LpGeo& g, const NetSrc& s, const float* nw, int64_
   a.g = g; a.s = s; a.nw = nw; a.n = n; a.X = X; a.h2 = h2;
   IQ_CUDA_OK(cudaFuncSetAttribute(net_l2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L2_SMEM));
   const int ipb = 4 * (8 / (g.g2[1] * g.g2[2]));
-  net_l2_kernel<<<(unsigned)std::min<int64_t>((n + ipb - 1) / ipb, sm_count()), NT, L2_SMEM, ctx->stream>>>(a);
+  net_l2_kernel<<<(unsigned)std::min<int64_t>((n + ipb - 1) / ipb, iq_sm_count()), NT, L2_SMEM, ctx->stream>>>(a);
   iq_count(ctx);
   IQ_CUDA_OK(cudaGetLastError());
   return IQ_OK;
@@ -910,7 +903,7 @@ int net_l2(iq_ctx* ctx, const LpGeo& g, const NetSrc& s, const float* nw, int64_
 
 int net_l3(iq_ctx* ctx, const L3Args& a) {
   IQ_CUDA_OK(cudaFuncSetAttribute(net_l3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L3_SMEM));
-  net_l3_kernel<<<(unsigned)std::min<int64_t>((a.n + L3_IPB - 1) / L3_IPB, sm_count()), NT, L3_SMEM, ctx->stream>>>(a);
+  net_l3_kernel<<<(unsigned)std::min<int64_t>((a.n + L3_IPB - 1) / L3_IPB, iq_sm_count()), NT, L3_SMEM, ctx->stream>>>(a);
   iq_count(ctx);
   IQ_CUDA_OK(cudaGetLastError());
   return IQ_OK;
@@ -983,7 +976,7 @@ int iq_lp_encode_templates(iq_ctx* ctx, const LpGeo& g, const float* w, const fl
 
 int iq_lp_train_batch(iq_ctx* ctx, const LpGeo& g, const LpTrainBatch& B, double* loss_out) {
   const int64_t n = (int64_t)B.nA * (2 + B.nneg);
-  const int nsm = sm_count();
+  const int nsm = iq_sm_count();
   cudaStream_t st = ctx->stream;
   float* nw = nullptr;
   int rc = net_prep(ctx, g, B.w, 0, &nw);
