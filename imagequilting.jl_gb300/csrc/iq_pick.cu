@@ -1682,6 +1682,11 @@ __device__ __noinline__ bool all_zero_refined(const Ref& f, const float* __restr
   return true;
 }
 
+// Whether thr_collect_kernel has the positions of this task's picks.
+__device__ __forceinline__ bool thr_collected(const PickArgs& a, const PickTask& tk) {
+  return a.thr_n && !tk.pre && tk.naux == 0 && (a.P >= IQ_THR_EXACT || (a.rv && ref_on(tk.x0)));
+}
+
 // One CTA per (task, realization): CTA b picks for realization b % nreal of task b / nreal.
 // NAUX is the largest number of auxiliary sources of the launch's tasks.
 template <int NAUX>
@@ -1747,7 +1752,7 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
   } else if (naux == 0) {
     const float mn = __uint_as_float(mm[0]);
     // positions collected by thr_collect_kernel, in any order: sorted here
-    int64_t ncol = a.thr_n ? a.thr_n[b] : -1;
+    int64_t ncol = thr_collected(a, tk) ? a.thr_n[b] : -1;
     if (ncol > SORT_CAP) ncol = -1;
     if (ncol >= 0) {
       for (int i = threadIdx.x; i < ncol; i += PT) sbuf[i] = (unsigned long long)(uint32_t)cand[i];
@@ -2061,7 +2066,7 @@ constexpr int TC_NT = 256, TC_ITEMS = 8;
 __global__ void __launch_bounds__(TC_NT) thr_collect_kernel(const PickArgs a) {
   const int b = blockIdx.x, r = b % a.nreal;
   const PickTask& tk = a.tasks ? a.tasks[b / a.nreal] : a.t0;
-  if (tk.pre || tk.naux > 0) return;
+  if (!thr_collected(a, tk)) return;
   const float* D = tk.D0 + r * tk.D0_rs;
   const float mn = __uint_as_float((tk.mm0 + r * tk.mm0_rs)[0]);
   __shared__ float s_hi, s_tlo, s_thi;
@@ -2221,7 +2226,7 @@ int iq_launch_pick(iq_ctx* ctx, const PickLaunch& L) {
   const bool split = L.lvl1 && L.rv && L.ncand && naux > 0 && L.maxK > 0 && L.maxK <= REF_CACHE;
   // maps large enough that one CTA's pass over them shows beside another launch
   a.thr_n = a.thr_ties = nullptr;
-  if (L.thr && L.tasks && L.any_thr && L.P >= IQ_THR_MIN) {
+  if (L.thr && L.tasks && L.any_thr && L.P >= (L.rv ? IQ_THR_MIN : IQ_THR_EXACT)) {
     a.thr_n = L.thr;
     a.thr_ties = L.thr + nblocks;
     IQ_CUDA_OK(cudaMemsetAsync(L.thr, 0, sizeof(int) * 2 * nblocks, ctx->stream));
