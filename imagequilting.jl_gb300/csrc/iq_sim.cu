@@ -756,6 +756,8 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
         tzp.touched.resize(tzp.boxes.size(), 0);
         cfg_kappa[c] = iq_map_kappa_tz(ctx->ti_stats, sim_stats, cfgs[c].K, tzp.touched[c]);
       }
+  // (here already where the proposal is off: the device works while the host makes its lists)
+  if (tz && !ctx->lp_enable && !tzp.launches.empty()) RET_IF(tz_setup());
   const TcStageRef soft_st = (tc && nsoft > 0 && T > 0) ? stages_for(std::vector<int>{ncfg})
                                                          : TcStageRef{0, 0, 0, 0, 0, 0};
   uint32_t* d_tcst = nullptr;  // stage words of every list, then their prefixes
@@ -907,8 +909,9 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
         // per-tile soft distance maps, Toeplitz form
         void* img = iq_scratch(ctx, S_TZ_SIMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * (sp.split ? 4 : 2));
         float* a2 = (float*)iq_scratch(ctx, S_TZ_SA2, sizeof(float) * P);
-        void* B = iq_scratch(ctx, S_TZ_B, (size_t)sp.max_bytes());
+        void* B = iq_scratch(ctx, S_TZ_B, std::max((size_t)sp.max_bytes(), tzb_bytes * ngrp));
         if (!img || !a2 || !B) return IQ_ERR_ALLOC;
+        d_tzB = B;  // the slot may have moved
         RET_IF(sp.upload(ctx, S_TCSOFT, st));
         RET_IF(iq_tz_image(ctx, d_auxti[s], ctx->ti, auxti_stats, sp.split, img));
         RET_IF(iq_tz_a2_maps(ctx, d_auxii[s], ctx->ti, distD, tileD, sp.d_boxes, 1, d_dis, a2));
@@ -1267,7 +1270,7 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
   for (const MaskCfg& mc : cfgs) maxK = std::max<int64_t>(maxK, mc.K);
   const bool lp_on = iq_lp_applies(ctx, tileD, maxK, nh > 0 || nsoft > 0);
   const bool lp_cap = ctx->lp_capture > 0 && ctx->lp != nullptr;
-  if (tz && !lp_on && !tzp.launches.empty()) RET_IF(tz_setup());
+  if (tz && !tz_ready && !lp_on && !tzp.launches.empty()) RET_IF(tz_setup());
   std::vector<int32_t> lc_lohi(6 * std::max(ncfg, 1)), lc_cfgK(std::max(ncfg, 1));
   for (int cf = 0; cf < ncfg; ++cf) {
     for (int d = 0; d < 3; ++d) {
