@@ -1022,9 +1022,10 @@ struct RefArr {
 };
 
 // Level 1 of up to REF_BATCH entries by one warp: ref_eval's level-1 sums (the same terms in the same
-// order per lane), the offsets and template values read once for all of them and 2 x REF_BATCH image
-// loads in flight per lane. The loop is bound by the latency of those loads (L2) and by shared-memory
-// reads, two per term when entries are summed one at a time.
+// order per lane, but where 16 terms end one short of the lane's last it joins their block as the 17th:
+// one rounding more, which the radius covers), the offsets and template values read once for all of them
+// and 2 x REF_BATCH image loads in flight per lane. The loop is bound by the latency of those loads (L2)
+// and by shared-memory reads, two per term when entries are summed one at a time.
 constexpr int REF_BATCH = 4;
 
 template <int REF_BATCH>
