@@ -792,7 +792,7 @@ __device__ inline int iq_stage_rows(const LpImg& im, const LpColumn& col, uint4*
 // Sum of (a - b)^2 over one row of 32 codes given as bit planes (a0, a1), (b0, b1) and mask m. The
 // difference is odd where a0 != b0, 2 in magnitude where only the high bits differ, and 3 where both
 // differ and a1 == a0 (codes 0 and 3; 1 and 2 have a1 != a0): squares 1, 4 and 1 + 8, three counts
-// (POPC runs at a quarter of the integer rate and bounds the sums).
+// (POPC runs at a quarter of the integer rate).
 __device__ __forceinline__ int iq_row_ssd(uint32_t a0, uint32_t a1, const uint4& t) {
   const uint32_t x1 = (a1 ^ t.y) & t.z, x0 = (a0 ^ t.x) & t.z;
   const uint32_t d3 = x1 & x0 & ~(a1 ^ a0);

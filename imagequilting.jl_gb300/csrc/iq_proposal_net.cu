@@ -3,7 +3,8 @@
 // items with channel-contiguous activations ([cell][32], rows of 36 words in shared memory), the
 // transposed weights resident in shared memory.
 //
-// What bounds them: the FP32 pipe. Layer 2 is 0.75 of the 0.85 M multiply-adds of an item (8 x 8 x 4
+// What bounds them: shared-memory reads that two warps a scheduler do not cover (net_l2: the data pipe
+// 0.58, FMA pipe 0.35, issue 0.48 of the cycles). Layer 2 is 0.75 of the 0.85 M multiply-adds of an item (8 x 8 x 4
 // cells), layer 3 most of the rest. One CTA per item with one output per thread and two loads per
 // multiply-add took 0.54 us a window (10.6 ms for 20,000) and 2.25 + 7.7 + 14.5 ms for the forward,
 // backward and weight gradients of a training batch of 4,352 items, of about 0.25 ms each at the

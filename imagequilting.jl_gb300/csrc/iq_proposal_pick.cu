@@ -59,7 +59,8 @@ __device__ __forceinline__ void lp_bitonic(unsigned long long* buf, int n) {
 // (their origins a lane each), two at a time over the staged rows. Slices of all columns fill the
 // chip (a column per CTA left half of the warps of ~150 SMs idle, and the slowest column decided);
 // the running minimum of a column is shared through global memory, read once per 32 entries.
-// What bounds the sums: L1 (16 bytes of image and template a row and lane) and POPC. Per call of
+// What bounds the sums: L1 (16 bytes of image and of template a row and lane; 0.78 of its throughput,
+// the population counts' pipe at 0.28). Per call of
 // the 192 x 192 x 64 facies ensemble (6,144 columns of 16,384 positions, tile 32 x 32 x 16): 100 ms
 // a column per CTA with two 8-byte loads a row, four counts and shuffle sums; 76 with one 16-byte
 // load, three counts and hardware reductions; 40 here.
