@@ -522,7 +522,7 @@ extern "C" int iq_fastdistance(iq_ctx* ctx, const int64_t* tilesize, int32_t ntm
       IQ_CUDA_OK(cudaMemcpyAsync(d_st, stw.data(), sizeof(uint32_t) * stw.size(), cudaMemcpyHostToDevice, ctx->stream));
       IQ_CUDA_OK(cudaMemcpyAsync(d_cols, cols.data(), sizeof(TcCol) * cols.size(), cudaMemcpyHostToDevice, ctx->stream));
       void* img16 = nullptr;
-      if (ctx->corr_engine == 2 && ctx->ti_stats.fp16_range()) {
+      if (ctx->corr_engine == 2 && ctx->ti_stats.fp16_range() && tstats.fp16_range()) {
         img16 = iq_scratch(ctx, S_TZ_IMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * 4);
         if (!img16) return IQ_ERR_ALLOC;
         if ((rc = iq_tz_image(ctx, ctx->d_ti, ctx->ti, ctx->ti_stats, true, img16))) return rc;

@@ -930,7 +930,7 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
         for (const TzPlan::Launch& l : sp.launches)
           RET_IF(sp.launch(ctx, l, img, distD, a2, d_aux[s], psz, B, auxti_stats, aux_stats));
       } else if (tc && T > 0) {
-        if (ctx->corr_engine == 2 && auxti_stats.fp16_range()) {
+        if (ctx->corr_engine == 2 && auxti_stats.fp16_range() && aux_stats.fp16_range()) {
           d_simg16 = iq_scratch(ctx, S_TZ_SIMG, (size_t)(iq_tz_image_halves(ctx->ti) + 64) * 4);
           if (!d_simg16) return IQ_ERR_ALLOC;
           RET_IF(iq_tz_image(ctx, d_auxti[s], ctx->ti, auxti_stats, true, d_simg16));
