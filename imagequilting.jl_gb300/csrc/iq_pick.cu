@@ -1988,7 +1988,9 @@ __global__ void __launch_bounds__(PT) pick_kernel(const PickArgs a) {
     const ExactSrc& xs = j == 0 ? tk.x0 : tk.xa[j > 0 ? j - 1 : 0];
     __syncthreads();
     unsigned long long S;
-    if (can_ref && ref_on(xs)) {
+    // (a map of disabled windows only is Inf everywhere and has one rank)
+    const bool inf = j == 0 && !(__uint_as_float(mm[0]) < __int_as_float(0x7F800000));
+    if (can_ref && ref_on(xs) && !inf) {
       const Ref f = make_ref(xs, r, a.dx, a.dxy);
       const float* l1 = a.phase == 2 && n <= IQ_RANK_CAP && ref_cacheable(f)
                             ? a.lvl1 + ((int64_t)b * a.nsrc + j) * IQ_RANK_CAP : nullptr;
