@@ -405,8 +405,9 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
   // overlap, so each level runs as one batch with results identical to the path order.
   {
     int64_t rng3[3];
+    // (without spacing every tile along the dimension lies in the same place)
     for (int d = 0; d < 3; ++d)
-      rng3[d] = g.spacing[d] > 0 ? (g.tile[d] + g.spacing[d] - 1) / g.spacing[d] - 1 : 0;
+      rng3[d] = g.spacing[d] > 0 ? (g.tile[d] + g.spacing[d] - 1) / g.spacing[d] - 1 : g.ntiles[d] - 1;
     std::vector<int> tile_level(g.ntot, -1);
     for (Step& s : steps) {
       const int64_t t3[3] = {s.tile % g.ntiles[0], (s.tile / g.ntiles[0]) % g.ntiles[1],
