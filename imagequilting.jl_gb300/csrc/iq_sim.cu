@@ -285,11 +285,10 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
     int64_t c[3] = {hlin[i] % g.pad[0], (hlin[i] / g.pad[0]) % g.pad[1], hlin[i] / (g.pad[0] * g.pad[1])};
     int64_t lo[3], hi[3];
     for (int d = 0; d < 3; ++d) {
-      // tiles t with t*spacing <= c < t*spacing + tile
-      const int64_t sp = std::max<int64_t>(g.spacing[d], 1);
-      const int64_t num = c[d] - g.tile[d] + 1;
-      lo[d] = num <= 0 ? 0 : (num + sp - 1) / sp;
-      hi[d] = std::min<int64_t>(c[d] / sp, g.ntiles[d] - 1);
+      // tiles t with t*spacing <= c < t*spacing + tile (all of them without spacing)
+      const int64_t sp = g.spacing[d], num = c[d] - g.tile[d] + 1;
+      lo[d] = sp <= 0 || num <= 0 ? 0 : (num + sp - 1) / sp;
+      hi[d] = sp <= 0 ? g.ntiles[d] - 1 : std::min<int64_t>(c[d] / sp, g.ntiles[d] - 1);
     }
     const bool isn = std::isnan(hv[i]);
     for (int64_t tz = lo[2]; tz <= hi[2]; ++tz)
@@ -753,10 +752,8 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
   };
   if (tz)
     for (int c = 0; c < ncfg; ++c)
-      if (cfg_kappa[c] > 0.0) {
-        tzp.touched.resize(tzp.boxes.size(), 0);
-        cfg_kappa[c] = iq_map_kappa_tz(ctx->ti_stats, sim_stats, cfgs[c].K, tzp.touched[c]);
-      }
+      if (cfg_kappa[c] > 0.0)
+        cfg_kappa[c] = iq_map_kappa_tz(ctx->ti_stats, sim_stats, cfgs[c].K, tzp.steps_of(c));
   // (here already where the proposal is off: the device works while the host makes its lists)
   if (tz && !ctx->lp_enable && !tzp.launches.empty()) RET_IF(tz_setup());
   const TcStageRef soft_st = (tc && nsoft > 0 && T > 0) ? stages_for(std::vector<int>{ncfg})
@@ -901,7 +898,7 @@ static int simulate(iq_ctx* ctx, const iq_sim_params* p, const iq_hard_data* har
             }
             sp.add_launches(cc, 2.0 * (double)P * (double)T * (double)cc.size(), tz_cap);
           }
-          soft_kappa[s] = iq_map_kappa_tz(auxti_stats, aux_stats, T, sp.touched[0]);
+          soft_kappa[s] = iq_map_kappa_tz(auxti_stats, aux_stats, T, sp.steps_of(0));
         } else
         soft_kappa[s] = iq_map_kappa(auxti_stats, aux_stats, T, form);
         soft_eabs[s] = iq_map_eabs(auxti_stats, tivol);

@@ -95,6 +95,8 @@ struct TzPlan {
     }
     if (L.ngroup > 0) launches.push_back(L);
   }
+  // K-steps of mask b (0: no column has it)
+  int64_t steps_of(size_t b) const { return b < touched.size() ? touched[b] : 0; }
   int64_t max_bytes() const {
     int64_t b = 1;
     for (const Launch& l : launches) b = std::max(b, l.bytes);
