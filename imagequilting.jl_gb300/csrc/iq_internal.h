@@ -424,12 +424,13 @@ struct PickTask {
   ExactSrc xa[IQ_MAX_AUX];
 };
 
-// Positions from which threshold picks are collected ahead of the pick (thr_collect_kernel): maps that
-// need the exact re-rank from IQ_THR_MIN, exact ones, whose candidates must then be sorted, from
-// IQ_THR_EXACT. Picks of a 2-D image, 8 realizations, collected ahead and by the pick: lognormal,
-// 66,049 positions 3.57 and 4.20 ms, 263,169 3.8 and 6.9; 2 codes, 37,249 2.01 and 1.21 ms, 124,609 4.56
-// and 3.84, 263,169 6.16 and 6.14, 1,046,529 29.1 and 29.5 (one realization 10.4 and 12.6).
-constexpr int64_t IQ_THR_MIN = 65536, IQ_THR_EXACT = 262144;
+// Positions from which threshold picks are collected ahead of the pick (thr_collect_kernel). Picks of a
+// 2-D lognormal image, 8 realizations, collected ahead and by the pick: 66,049 positions 3.57 and 4.20 ms,
+// 263,169 3.8 and 6.9. The positions arrive in any order and are sorted, which exact maps with thousands
+// of candidates pay for: 2 codes, 37,249 positions (248 candidates) 2.01 and 1.21 ms, 124,609 (1,703)
+// 4.56 and 3.84, 263,169 (3,124) 6.16 and 6.14, 1,046,529 29.1 and 29.5. With few they gain at every size
+// above the line: a 3-D simulation of 6 codes, 158,118 positions, 8.0 and 8.6 ms in all.
+constexpr int64_t IQ_THR_MIN = 65536;
 // Most candidates of a pick evaluated between its phases (16 KB of scratch per pick and source; longer
 // lists are evaluated by the pick's own CTA). Picks with one soft variable, 4 realizations, at 1,024,
 // 4,096 and 16,384: 765 candidates on average 48.1, 34.3 and 30.9 ms; 2,777 115, 72 and 62; 5,087 194,

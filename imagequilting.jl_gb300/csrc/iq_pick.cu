@@ -1685,7 +1685,7 @@ __device__ __noinline__ bool all_zero_refined(const Ref& f, const float* __restr
 
 // Whether thr_collect_kernel has the positions of this task's picks.
 __device__ __forceinline__ bool thr_collected(const PickArgs& a, const PickTask& tk) {
-  return a.thr_n && !tk.pre && tk.naux == 0 && (a.P >= IQ_THR_EXACT || (a.rv && ref_on(tk.x0)));
+  return a.thr_n && !tk.pre && tk.naux == 0;
 }
 
 // One CTA per (task, realization): CTA b picks for realization b % nreal of task b / nreal.
@@ -2229,7 +2229,7 @@ int iq_launch_pick(iq_ctx* ctx, const PickLaunch& L) {
   const bool split = L.lvl1 && L.rv && L.ncand && naux > 0 && L.maxK > 0 && L.maxK <= REF_CACHE;
   // maps large enough that one CTA's pass over them shows beside another launch
   a.thr_n = a.thr_ties = nullptr;
-  if (L.thr && L.tasks && L.any_thr && L.P >= (L.rv ? IQ_THR_MIN : IQ_THR_EXACT)) {
+  if (L.thr && L.tasks && L.any_thr && L.P >= IQ_THR_MIN) {
     a.thr_n = L.thr;
     a.thr_ties = L.thr + nblocks;
     IQ_CUDA_OK(cudaMemsetAsync(L.thr, 0, sizeof(int) * 2 * nblocks, ctx->stream));

@@ -1,5 +1,5 @@
 """Threshold picks of exact maps on both sides of the size from which their positions are collected ahead
-of the pick (262,144), with candidate lists the collecting pass keeps whole and ones it overflows (8,192):
+of the pick (65,536), with candidate lists the collecting pass keeps whole and ones it overflows (8,192):
 realizations and near-tie counts equal the oracle's (integer images: no tolerance)."""
 import numpy as np
 import pytest
@@ -16,7 +16,7 @@ def ctx(iq):
     c.close()
 
 
-@pytest.mark.parametrize("shape", [(519, 519), (520, 520)])  # 261,632 and 262,656 positions
+@pytest.mark.parametrize("shape", [(263, 263), (264, 263)])  # 65,280 and 65,536 positions
 @pytest.mark.parametrize("codes,tol", [(2, 0.1), (6, 0.05), (2, 1.0)])
 def test_exact_maps(iq, ctx, shape, codes, tol):
     rng = np.random.default_rng(801)
